@@ -33,6 +33,11 @@ struct Epilogue {
 shrk_status exact_pair_sums(const double* d_tgt, int64_t nt, const double* d_src, int64_t ns,
                             double eta, int precision, const Epilogue& epi, cudaStream_t s);
 
+// All-points FP64 sums S(ev_t) with every unordered pair evaluated once
+// (pairsym.cu).
+shrk_status sym_sums(const double* d_ev, int64_t p, double eta, const Epilogue& epi,
+                     cudaStream_t s);
+
 // The same raw sums (no epilogue) with every temporary in caller-provided
 // device memory and no library state touched: `part` holds part_capacity
 // (re, im) split partials (>= nt), `bounds` ns/256 + 2 double2 (MIXED only),
@@ -188,6 +193,7 @@ double mixed_near_k();
 // Sets the bulk-copy wait budget of the exact pair kernels (cycles; negative
 // = the default) and returns the previous one.
 long long set_wait_cycles(long long cycles);
+long long wait_cycles();
 shrk_status measure_pipe_rates(double* fp32, double* fp64);
 shrk_status measure_rcp_bias(double* uniform_mean, double* log_mean);
 

@@ -176,6 +176,8 @@ long long set_wait_cycles(long long cycles) {
   return g_wait_cycles.exchange(cycles < 0 ? WAIT_CYCLES_DEFAULT : cycles);
 }
 
+long long wait_cycles() { return g_wait_cycles.load(); }
+
 SplitPlan plan_splits(int64_t nt, int64_t ns, int tile, int chunk, int ctas_per_sm) {
   SplitPlan pl;
   pl.n_tiles = (nt + tile - 1) / tile;
@@ -213,6 +215,9 @@ shrk_status exact_pair_sums(const double* d_tgt, int64_t nt, const double* d_src
     return SHRK_EINVAL;
   }
   const bool mixed = (precision == SHRK_PREC_MIXED);
+  // All points of one spectrum: one evaluation per unordered pair.
+  if (!mixed && d_tgt == d_src && nt == ns)
+    return sym_sums(d_src, ns, eta, epi, s);
   // Fewer targets than one full tile (a query grid), or a sum whose full-tile
   // plan has fewer items than the GPU holds CTAs (a small spectrum): the
   // 4-target tiles would leave most of each thread's work on padding or the
