@@ -7,13 +7,16 @@
 // on ev_k (the target derivative of autovec.rs:38-59).  Pairs are recomputed,
 // never stored.
 //
-// G is antisymmetric (G(j, k) = -G(k, j)), so the main kernel evaluates each
-// unordered pair once and adds it to both ends; the row-sum kernel (every
-// ordered pair, four source sums per target) remains for sizes whose column
-// slabs would not fit.
+// G is antisymmetric (G(j, k) = -G(k, j)), so each unordered pair is evaluated
+// once and added to both ends.  FP64: the triangle in equal runs, the column
+// sums carried round the warp (adjoint_f64_kernel; the split of pairsym.cuh).
+// MIXED: fixed (T, S) tiles with FP32 far blocks (adjoint_sym_kernel); its
+// row-sum form (every ordered pair, four source sums per target) remains for
+// sizes whose column slabs would not fit.
 #include "common.cuh"
 #include "internal.h"
 #include "pairs.cuh"
+#include "pairsym.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -53,11 +56,10 @@ struct AdjArgs {
   double* part;  // [n_splits][4][p]
 };
 
-template <bool MIXED>
 __global__ void __launch_bounds__(NT, 2) adjoint_kernel(const AdjArgs a) {
   __shared__ __align__(16) double sl[ACH], sw[ACH], sv[ACH];
-  __shared__ __align__(16) float fmu[MIXED ? ACH : 4], fml[MIXED ? ACH : 4];
-  __shared__ __align__(16) float fw[MIXED ? ACH : 4], fv[MIXED ? ACH : 4];
+  __shared__ __align__(16) float fmu[ACH], fml[ACH];
+  __shared__ __align__(16) float fw[ACH], fv[ACH];
   __shared__ double red[NT / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double eta = a.eta, eta2 = eta * eta, teta = 2.0 * eta;
@@ -83,8 +85,8 @@ __global__ void __launch_bounds__(NT, 2) adjoint_kernel(const AdjArgs a) {
       xh[r] = xl[r] = 0.0f;
     }
     const double c = x0;
-    double wlo = 0, whi = 0, thr = INFINITY;
-    if (MIXED) {
+    double wlo, whi, thr;
+    {
       double spread = 0.0, mn = x[0], mx = x[0];
 #pragma unroll
       for (int r = 0; r < R; ++r) {
@@ -113,23 +115,21 @@ __global__ void __launch_bounds__(NT, 2) adjoint_kernel(const AdjArgs a) {
         sl[i] = a.ev[cs + i];
         sw[i] = a.w[cs + i];
         sv[i] = a.v[cs + i];
-        if (MIXED) {
-          split_source(sl[i], c, fmu[i], fml[i]);
-          fw[i] = (float)sw[i];
-          fv[i] = (float)sv[i];
-        }
+        split_source(sl[i], c, fmu[i], fml[i]);
+        fw[i] = (float)sw[i];
+        fv[i] = (float)sv[i];
       }
       __syncthreads();
       for (int sub = 0; sub < len; sub += SUB) {
         const int slen = min(SUB, len - sub);
         bool far32 = false;
-        if (MIXED && slen == SUB) {
+        if (slen == SUB) {
           const double2 bd = a.bounds[(cs + sub) / SUB];
           const double gap = fmax(fmax(bd.x - whi, wlo - bd.y), 0.0);
           const double span = fmax(bd.y - wlo, whi - bd.x);
           far32 = gap >= thr && span <= 1e9;
         }
-        if (MIXED && far32) {
+        if (far32) {
           for (int j = sub; j < sub + SUB; j += FOLD) {
             float pp[R][4];
 #pragma unroll
@@ -254,11 +254,11 @@ __device__ __forceinline__ F warp_sum4(const F (&c)[4], int lane) {
   return v;
 }
 
-template <bool MIXED, int RS>
+template <int RS>
 __global__ void __launch_bounds__(NT, 2) adjoint_sym_kernel(const AdjSymArgs a) {
   constexpr int STT = NT * RS, SWT = 32 * RS;
   __shared__ __align__(16) double sl[SUB], sw[SUB], sv[SUB];
-  __shared__ __align__(16) float fsm[MIXED ? SUB : 1], fw[MIXED ? SUB : 1], fv[MIXED ? SUB : 1];
+  __shared__ __align__(16) float fsm[SUB], fw[SUB], fv[SUB];
   __shared__ double colw[NT / 32][SUB];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double eta = a.eta, eta2 = eta * eta, teta = 2.0 * eta, m2e2 = -2.0 * eta2;
@@ -279,17 +279,14 @@ __global__ void __launch_bounds__(NT, 2) adjoint_sym_kernel(const AdjSymArgs a) 
       vk[r] = valid[r] ? teta * a.v[idx] : 0.0;
       row[r] = 0.0;
     }
-    double wlo = 0.0, whi = 0.0;
-    if (MIXED) {
-      double mn = x[0], mx = x[0];
+    double wlo = x[0], whi = x[0];
 #pragma unroll
-      for (int r = 0; r < RS; ++r) {
-        mn = fmin(mn, x[r]);
-        mx = fmax(mx, x[r]);
-      }
-      wlo = warp_min(mn);
-      whi = warp_max(mx);
+    for (int r = 0; r < RS; ++r) {
+      wlo = fmin(wlo, x[r]);
+      whi = fmax(whi, x[r]);
     }
+    wlo = warp_min(wlo);
+    whi = warp_max(whi);
     const int64_t src0 = (int64_t)S * STT, src1 = min(a.p, src0 + STT);
     for (int64_t cs = src0; cs < src1; cs += SUB) {
       const int len = (int)min((int64_t)SUB, src1 - cs);
@@ -300,21 +297,19 @@ __global__ void __launch_bounds__(NT, 2) adjoint_sym_kernel(const AdjSymArgs a) 
         sl[i] = l;
         sw[i] = wj;
         sv[i] = vj;
-        if (MIXED) {
-          fsm[i] = (float)(l - cb);
-          fw[i] = (float)wj;
-          fv[i] = (float)vj;
-        }
+        fsm[i] = (float)(l - cb);
+        fw[i] = (float)wj;
+        fv[i] = (float)vj;
       }
       __syncthreads();
       bool far32 = false;
-      if (MIXED && len == SUB) {
+      if (len == SUB) {
         const double2 bd = a.bounds[cs / SUB];
         const double gap = fmax(fmax(bd.x - whi, wlo - bd.y), 0.0);
         const double span = fmax(bd.y - wlo, whi - bd.x);
         far32 = gap >= a.near_dist && span <= 1e9;
       }
-      if (MIXED && far32) {
+      if (far32) {
         float th[RS], tl[RS], wkf[RS], vkf[RS];
 #pragma unroll
         for (int r = 0; r < RS; ++r) {
@@ -410,20 +405,219 @@ __global__ void adjoint_slab_reduce_kernel(const double* __restrict__ part, int 
   grad[k] = s * inv_p;
 }
 
+// ------------------------------------------------------ FP64 adjoint ----
+// With r = 1/(d^2 + eta^2), d = ev_k - ev_j, v' = 2 eta v and dw = w_k - w_j:
+//   G(k, j) = r (dw - r (2 eta^2 dw + (v'_k + v'_j) d)),
+// 12 FP64 operations a pair with both accumulations (A and B formed apart:
+// 14).  The FP64 pipe bounds it; tiles, units, column rotation and chunked row
+// sums as in pairsym.cu, one column sum per source.  Measured (B200), against
+// (T, S) tiles with the column sums reduced across lanes: p = 20 000 184 us
+// (315), 2e5 16.5 ms (23.7), up to 4 000 20 us with its launches (36).
+struct AdjF64Args {
+  SymPlan pl;
+  const double* ev;
+  const double* w;
+  const double* v;
+  double eta;
+  double* rows;  // [grid + tiles][tt]
+  double* cols;  // [tiles][p]
+};
+
+template <int R>
+struct AdjTargets {
+  double x[R], w[R], v[R];
+};
+
+template <int R, bool MASK, bool COL>
+__device__ __forceinline__ void adj_step(const AdjTargets<R>& t, double l, double wj, double vj,
+                                         double eta2, double teta2, bool on, double (&row)[R],
+                                         double& col) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const double d = t.x[r] - l;
+    double rr = rcp_f64(fma(d, d, eta2));
+    const double dw = t.w[r] - wj;
+    const double y = fma(t.v[r] + vj, d, teta2 * dw);
+    const double g = fma(-rr, y, dw);
+    if (MASK && !on) rr = 0.0;
+    row[r] = fma(rr, g, row[r]);
+    if (COL) col = fma(rr, g, col);
+  }
+}
+
+template <int R>
+__global__ void __launch_bounds__(NT, 2) adjoint_f64_kernel(const AdjF64Args a) {
+  constexpr int NW = NT / 32;
+  __shared__ double2 slw[SYM_CH];  // (ev, w)
+  __shared__ double sv[SYM_CH];    // 2 eta v
+  __shared__ double colw[NW][SYM_CH];
+  const SymPlan& pl = a.pl;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const double eta2 = a.eta * a.eta, teta = 2.0 * a.eta, teta2 = 2.0 * eta2;
+  const int64_t base0 = pl.before(pl.t0);
+  int64_t u = pl.first_unit(blockIdx.x);
+  const int64_t u_end = pl.first_unit(blockIdx.x + 1);
+  int T = pl.tile_of(u);
+  for (; u < u_end; ++T) {
+    const int64_t ub = pl.before(T) - base0;
+    const int64_t seg_end = min(u_end, pl.before(T + 1) - base0);
+    const int64_t tile0 = (int64_t)T * pl.tt, wbase = tile0 + (int64_t)warp * (32 * R);
+    const int64_t diag_end = min(pl.p, tile0 + pl.tt);
+    const int64_t s0 = tile0 + (u - ub) * SYM_UB;
+    const int64_t s1 = min(pl.p, tile0 + (seg_end - ub) * SYM_UB);
+    AdjTargets<R> t;
+    double tot[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int64_t idx = min(wbase + r * 32 + lane, pl.p - 1);
+      t.x[r] = a.ev[idx];
+      t.w[r] = a.w[idx];
+      t.v[r] = teta * a.v[idx];
+      tot[r] = 0.0;
+    }
+    int len = 0;
+    for (int64_t cs = s0; cs < s1; cs += len) {
+      const bool diag = cs < diag_end;
+      len = (int)min((int64_t)SYM_CH, (diag ? min(s1, diag_end) : s1) - cs);
+      __syncthreads();  // the previous chunk's readers are done
+      {
+        const int64_t i = cs + min(tid, len - 1);
+        slw[tid] = make_double2(a.ev[i], a.w[i]);
+        sv[tid] = teta * a.v[i];
+      }
+      __syncthreads();
+      double row[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) row[r] = 0.0;
+      if (diag) {  // the tile against itself: full square, rows only
+#pragma unroll 2
+        for (int j = 0; j < len; ++j) {
+          const double2 s = slw[j];
+          double none;
+          adj_step<R, false, false>(t, s.x, s.y, sv[j], eta2, teta2, true, row, none);
+        }
+      } else {
+        int b = 0;
+        for (; b + 64 <= len; b += 64) {
+          double c0 = 0.0, c1 = 0.0;
+#pragma unroll 2
+          for (int g = 0; g < 32; g += 8) {
+            const int at = lane ^ g, turn = (g & 8) ? 31 : 15;  // (g + 7) ^ (g + 8)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const int j = b + (at ^ k);
+              const double2 s = slw[j], q = slw[j + 32];
+              adj_step<R, false, true>(t, s.x, s.y, sv[j], eta2, teta2, true, row, c0);
+              adj_step<R, false, true>(t, q.x, q.y, sv[j + 32], eta2, teta2, true, row, c1);
+              const int m = k < 7 ? k ^ (k + 1) : turn;
+              c0 = __shfl_xor_sync(0xffffffffu, c0, m);
+              c1 = __shfl_xor_sync(0xffffffffu, c1, m);
+            }
+          }
+          colw[warp][b + lane] = c0;
+          colw[warp][b + 32 + lane] = c1;
+        }
+        for (; b < len; b += 32) {  // the spectrum's end: sources past it masked
+          double c0 = 0.0;
+#pragma unroll 1
+          for (int k = 0; k < 32; ++k) {
+            const int j = b + (lane ^ k);
+            const double2 s = slw[j];
+            adj_step<R, true, true>(t, s.x, s.y, sv[j], eta2, teta2, j < len, row, c0);
+            c0 = __shfl_xor_sync(0xffffffffu, c0, (k ^ (k + 1)) & 31);
+          }
+          colw[warp][b + lane] = c0;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) tot[r] += row[r];
+      if (diag) continue;
+      __syncthreads();
+      if (tid < len) {
+        double c = 0.0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) c += colw[w][tid];
+        a.cols[(int64_t)(T - pl.t0) * pl.p + cs + tid] = -c;
+      }
+    }
+    double* row = a.rows + (int64_t)(blockIdx.x + T - pl.t0) * pl.tt;
+#pragma unroll
+    for (int r = 0; r < R; ++r) row[warp * (32 * R) + r * 32 + lane] = tot[r];
+    u = seg_end;
+  }
+}
+
+__global__ void __launch_bounds__(NT) adjoint_f64_reduce_kernel(SymPlan pl, const double* rows,
+                                                                const double* cols, double* acc,
+                                                                bool first, bool last,
+                                                                double inv_p, double* grad) {
+  const int64_t t0 = (int64_t)blockIdx.x * 32, t = t0 + (threadIdx.x & 31);
+  const double g = sym_collect<double>(pl, rows, cols, first ? nullptr : acc, t0);
+  if (threadIdx.x >= 32 || t >= pl.p) return;
+  if (last) grad[t] = g * inv_p;
+  else acc[t] = g;
+}
+
+template <int R>
+shrk_status launch_adjoint_f64(const AdjF64Args& a, cudaStream_t s) {
+  adjoint_f64_kernel<R><<<a.pl.grid, NT, 0, s>>>(a);
+  SHRK_CUDA(cudaGetLastError());
+  return SHRK_OK;
+}
+
+shrk_status adjoint_f64(const double* d_ev, int64_t p, double eta, const double* d_gre,
+                        const double* d_gim, double* d_grad, cudaStream_t s) {
+  // Targets per thread, measured (us for R = 1 / 2 / 4): p = 7001 38 / 33 / 41,
+  // 14000 116 / 99 / 105, 20000 214 / 189 / 184, 60000 1815 / 1560 / 1519; up to
+  // 5000 all three within 2 us (launches).
+  const int R = p >= 16384 ? 4 : p >= 3072 ? 2 : 1;
+  const int tt = NT * R;
+  const int n_tiles = (int)((p + tt - 1) / tt);
+  const int ctas = sm_count() * 2;
+  // tiles of a phase: as many column slabs as 256 MB hold
+  const int64_t per = std::max<int64_t>(1, ((int64_t)256 << 20) / ((int64_t)sizeof(double) * p));
+  const int phase = (int)std::min<int64_t>(n_tiles, per);
+  const size_t row_n = (size_t)(ctas + phase) * tt, acc_n = phase < n_tiles ? (size_t)p : 0;
+  void* buf = nullptr;
+  SHRK_TRY(scratch_get(2, sizeof(double) * (row_n + acc_n + (size_t)phase * (size_t)p), &buf));
+  double* rows = (double*)buf;
+  double* acc = rows + row_n;
+  AdjF64Args a;
+  a.ev = d_ev;
+  a.w = d_gre;
+  a.v = d_gim;
+  a.eta = eta;
+  a.rows = rows;
+  a.cols = acc + acc_n;
+  for (int t0 = 0; t0 < n_tiles; t0 += phase) {
+    a.pl = sym_plan(p, tt, t0, std::min(n_tiles, t0 + phase), ctas);
+    {
+      LaunchScope ls("adjoint_f64", s);
+      if (R == 4) SHRK_TRY(launch_adjoint_f64<4>(a, s));
+      else if (R == 2) SHRK_TRY(launch_adjoint_f64<2>(a, s));
+      else SHRK_TRY(launch_adjoint_f64<1>(a, s));
+    }
+    LaunchScope ls("adjoint_reduce", s);
+    adjoint_f64_reduce_kernel<<<(unsigned)((p + 31) / 32), NT, 0, s>>>(
+        a.pl, rows, a.cols, acc, t0 == 0, a.pl.t1 == n_tiles, 1.0 / (double)p, d_grad);
+    SHRK_CUDA(cudaGetLastError());
+  }
+  return SHRK_OK;
+}
+
 }  // namespace
 
 namespace {
 
-// Row-sum path (every ordered pair).
+// Row-sum path (every ordered pair), MIXED.
 shrk_status adjoint_rows(const double* d_ev, int64_t p, double eta, const double* d_gre,
-                         const double* d_gim, int precision, double* d_grad, cudaStream_t s) {
-  const bool mixed = (precision == SHRK_PREC_MIXED);
+                         const double* d_gim, double* d_grad, cudaStream_t s) {
   const SplitPlan pl = plan_splits(p, p, TT, ACH, 2);
   void* part = nullptr;
   SHRK_TRY(scratch_get(2, sizeof(double) * 4 * (size_t)pl.n_splits * (size_t)p, &part));
   double2* bounds = nullptr;
   const int64_t nblocks = (p + SUB - 1) / SUB;
-  if (mixed) {
+  {
     void* b = nullptr;
     SHRK_TRY(scratch_get(1, sizeof(double2) * (size_t)(nblocks + 1), &b));
     bounds = (double2*)b;
@@ -435,7 +629,7 @@ shrk_status adjoint_rows(const double* d_ev, int64_t p, double eta, const double
   a.v = d_gim;
   a.p = p;
   a.bounds = bounds;
-  a.gminmax = bounds ? bounds + nblocks : nullptr;
+  a.gminmax = bounds + nblocks;
   a.eta = eta;
   a.near_dist = std::max(mixed_near_k() * eta, 1e-9);
   a.n_tiles = pl.n_tiles;
@@ -443,9 +637,8 @@ shrk_status adjoint_rows(const double* d_ev, int64_t p, double eta, const double
   a.split_len = pl.split_len;
   a.part = (double*)part;
   {
-    LaunchScope ls(mixed ? "adjoint_mixed" : "adjoint_f64", s);
-    if (mixed) adjoint_kernel<true><<<pl.grid, NT, 0, s>>>(a);
-    else adjoint_kernel<false><<<pl.grid, NT, 0, s>>>(a);
+    LaunchScope ls("adjoint_mixed", s);
+    adjoint_kernel<<<pl.grid, NT, 0, s>>>(a);
     SHRK_CUDA(cudaGetLastError());
   }
   {
@@ -459,10 +652,9 @@ shrk_status adjoint_rows(const double* d_ev, int64_t p, double eta, const double
 
 
 template <int RS>
-shrk_status launch_sym(const AdjSymArgs& a, bool mixed, int grid, cudaStream_t s) {
-  LaunchScope ls(mixed ? "adjoint_mixed" : "adjoint_f64", s);
-  if (mixed) adjoint_sym_kernel<true, RS><<<grid, NT, 0, s>>>(a);
-  else adjoint_sym_kernel<false, RS><<<grid, NT, 0, s>>>(a);
+shrk_status launch_sym(const AdjSymArgs& a, int grid, cudaStream_t s) {
+  LaunchScope ls("adjoint_mixed", s);
+  adjoint_sym_kernel<RS><<<grid, NT, 0, s>>>(a);
   SHRK_CUDA(cudaGetLastError());
   return SHRK_OK;
 }
@@ -472,7 +664,7 @@ shrk_status launch_sym(const AdjSymArgs& a, bool mixed, int grid, cudaStream_t s
 shrk_status adjoint(const double* d_ev, int64_t p, double eta, const double* d_gre,
                     const double* d_gim, int precision, double* d_grad, cudaStream_t s) {
   if (p <= 0) return SHRK_OK;
-  const bool mixed = (precision == SHRK_PREC_MIXED);
+  if (precision != SHRK_PREC_MIXED) return adjoint_f64(d_ev, p, eta, d_gre, d_gim, d_grad, s);
   // Targets per thread: the widest tile that still gives the grid a few
   // waves of (T, S) items.
   const int64_t ctas = (int64_t)sm_count() * 2;
@@ -485,17 +677,14 @@ shrk_status adjoint(const double* d_ev, int64_t p, double eta, const double* d_g
   }
   const size_t slab_bytes = sizeof(double) * (size_t)n_t * (size_t)p;
   if (slab_bytes > (size_t(2) << 30))
-    return adjoint_rows(d_ev, p, eta, d_gre, d_gim, precision, d_grad, s);
+    return adjoint_rows(d_ev, p, eta, d_gre, d_gim, d_grad, s);
   void* part = nullptr;
   SHRK_TRY(scratch_get(2, slab_bytes, &part));
-  double2* bounds = nullptr;
-  if (mixed) {
-    const int64_t nblocks = (p + SUB - 1) / SUB;
-    void* b = nullptr;
-    SHRK_TRY(scratch_get(1, sizeof(double2) * (size_t)(nblocks + 1), &b));
-    bounds = (double2*)b;
-    SHRK_TRY(source_bounds(d_ev, p, nblocks, bounds, s));
-  }
+  const int64_t nblocks = (p + SUB - 1) / SUB;
+  void* b = nullptr;
+  SHRK_TRY(scratch_get(1, sizeof(double2) * (size_t)(nblocks + 1), &b));
+  double2* bounds = (double2*)b;
+  SHRK_TRY(source_bounds(d_ev, p, nblocks, bounds, s));
   AdjSymArgs a;
   a.ev = d_ev;
   a.w = d_gre;
@@ -508,9 +697,9 @@ shrk_status adjoint(const double* d_ev, int64_t p, double eta, const double* d_g
   a.n_items = n_t * (n_t + 1) / 2;
   a.part = (double*)part;
   const int grid = (int)std::min<int64_t>(a.n_items, ctas);
-  if (RS == 4) SHRK_TRY(launch_sym<4>(a, mixed, grid, s));
-  else if (RS == 2) SHRK_TRY(launch_sym<2>(a, mixed, grid, s));
-  else SHRK_TRY(launch_sym<1>(a, mixed, grid, s));
+  if (RS == 4) SHRK_TRY(launch_sym<4>(a, grid, s));
+  else if (RS == 2) SHRK_TRY(launch_sym<2>(a, grid, s));
+  else SHRK_TRY(launch_sym<1>(a, grid, s));
   LaunchScope ls("adjoint_reduce", s);
   adjoint_slab_reduce_kernel<<<(unsigned)((p + 255) / 256), 256, 0, s>>>(
       (const double*)part, (int)n_t, p, 1.0 / (double)p, d_grad);

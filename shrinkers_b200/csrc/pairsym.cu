@@ -256,59 +256,13 @@ struct SymReduceArgs {
   Epilogue epi;
 };
 
-// Sums of 32 targets a CTA: warp w takes every eighth partial (the columns of
-// the tiles before theirs, then their rows in CTA order), the eight sums are
-// added in order to the earlier phases', and the last phase applies the
-// epilogue.  A thread per target walked all partials alone: 11 us at p = 4096
-// where the sums themselves take 12.
+// The phase's sums of 32 targets a CTA; the last phase applies the epilogue.
 __global__ void __launch_bounds__(NT) sym_reduce_kernel(const SymReduceArgs a) {
-  __shared__ double2 part[NW][32];
-  __shared__ int cs[2];
-  const SymPlan& pl = a.pl;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t t0 = (int64_t)blockIdx.x * 32;
-  const int64_t t = min(t0 + lane, pl.p - 1);
-  const int tile = (int)(t0 / pl.tt);  // tiles are multiples of 256 targets
-  const bool own = tile >= pl.t0 && tile < pl.t1;
-  if (threadIdx.x < 2 && own) {
-    const int64_t base0 = pl.before(pl.t0);
-    cs[threadIdx.x] = pl.cta_of(pl.before(tile + threadIdx.x) - base0 - threadIdx.x);
-  }
-  const int nc = min(tile, pl.t1) - pl.t0;
-  double re = 0.0, iv = 0.0;
-  const double2* col = a.cols + t;
-#pragma unroll 4
-  for (int k = warp; k < nc; k += NW) {
-    const double2 q = col[(int64_t)k * pl.p];
-    re += q.x;
-    iv += q.y;
-  }
-  __syncthreads();
-  if (own) {
-    const int c0 = cs[0], c1 = cs[1];
-    const double2* row = a.rows + (int64_t)(tile - pl.t0) * pl.tt + (t - (int64_t)tile * pl.tt);
-#pragma unroll 4
-    for (int c = c0 + warp; c <= c1; c += NW) {
-      const double2 q = row[(int64_t)c * pl.tt];
-      re += q.x;
-      iv += q.y;
-    }
-  }
-  part[warp][lane] = make_double2(re, iv);
-  __syncthreads();
-  if (warp != 0 || t0 + lane >= pl.p) return;
-  if (!a.first) {
-    const double2 q = a.acc[t];
-    re += q.x;
-    iv += q.y;
-  }
-#pragma unroll
-  for (int w = 1; w < NW; ++w) {
-    re += part[w][lane].x;
-    iv += part[w][lane].y;
-  }
-  if (a.last) epi_store(a.epi, t, a.ev[t], re, a.eta * iv);
-  else a.acc[t] = make_double2(re, iv);
+  const int64_t t0 = (int64_t)blockIdx.x * 32, t = t0 + (threadIdx.x & 31);
+  const double2 q = sym_collect(a.pl, a.rows, a.cols, a.first ? nullptr : a.acc, t0);
+  if (threadIdx.x >= 32 || t >= a.pl.p) return;
+  if (a.last) epi_store(a.epi, t, a.ev[t], q.x, a.eta * q.y);
+  else a.acc[t] = q;
 }
 
 template <int R>

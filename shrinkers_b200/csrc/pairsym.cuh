@@ -74,4 +74,52 @@ inline SymPlan sym_plan(int64_t p, int tt, int t0, int t1, int ctas) {
   return pl;
 }
 
+__device__ __forceinline__ void sym_add(double& a, double b) { a += b; }
+__device__ __forceinline__ void sym_add(double2& a, double2 b) {
+  a.x += b.x;
+  a.y += b.y;
+}
+
+// Reduction of a phase's partials: a CTA of SYM_NT threads takes 32 targets
+// from t0 (one tile: tiles are multiples of 256 targets).  Warp w adds every
+// eighth partial (the columns of the tiles before theirs, then their rows in
+// CTA order); the eight sums are added in warp order after `acc`, the sums of
+// the earlier phases (null in the first).  The result is valid in warp 0.  (A
+// thread per target walked all its partials alone: 11 us at p = 4096, where
+// the sums themselves take 12.)
+template <typename V>
+__device__ __forceinline__ V sym_collect(const SymPlan& pl, const V* __restrict__ rows,
+                                         const V* __restrict__ cols, const V* acc, int64_t t0) {
+  __shared__ V part[SYM_NT / 32][32];
+  __shared__ int cs[2];
+  constexpr int NW = SYM_NT / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t t = t0 + lane < pl.p ? t0 + lane : pl.p - 1;
+  const int tile = (int)(t0 / pl.tt);
+  const bool own = tile >= pl.t0 && tile < pl.t1;
+  if (threadIdx.x < 2 && own) {
+    const int64_t base0 = pl.before(pl.t0);
+    cs[threadIdx.x] = pl.cta_of(pl.before(tile + threadIdx.x) - base0 - threadIdx.x);
+  }
+  V sum{};
+  const int nc = min(tile, pl.t1) - pl.t0;
+#pragma unroll 4
+  for (int k = warp; k < nc; k += NW) sym_add(sum, cols[(int64_t)k * pl.p + t]);
+  __syncthreads();
+  if (own) {
+    const int c1 = cs[1];
+    const V* row = rows + (int64_t)(tile - pl.t0) * pl.tt + (t - (int64_t)tile * pl.tt);
+#pragma unroll 4
+    for (int c = cs[0] + warp; c <= c1; c += NW) sym_add(sum, row[(int64_t)c * pl.tt]);
+  }
+  part[warp][lane] = sum;
+  __syncthreads();
+  if (warp == 0) {
+    if (acc) sym_add(sum, acc[t]);
+#pragma unroll
+    for (int w = 1; w < NW; ++w) sym_add(sum, part[w][lane]);
+  }
+  return sum;
+}
+
 }  // namespace shrk

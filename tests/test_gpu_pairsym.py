@@ -1,4 +1,5 @@
-"""Exact all-points FP64 sums (each unordered pair evaluated once): sizes at
+"""Exact all-points FP64 sums and their adjoint (each unordered pair evaluated
+once): sizes at
 the edges of the units (64 sources), staged chunks (256), tiles (256, 512 and
 1024 targets) and of the rule that picks the tile, a size that runs in several
 phases, spectra in any order and at any alignment, against the oracle's sums
@@ -70,3 +71,29 @@ def test_diagonal_dominates_at_small_eta(oracle):
         q_re, q_im = oracle.compute_at_points(ev, ev, eta, "blocked")
         scale = np.hypot(q_re, q_im)
         assert np.max(np.hypot(re * p - q_re, im * p - q_im) / scale) < 1e-12
+
+
+@pytest.mark.parametrize("p", [1, 2, 33, 64, 65, 257, 1025, 3071, 3073, 8193, 16383, 16385,
+                               60001])
+def test_symmetric_adjoint(oracle, p):
+    """Against the oracle's direct gradient at the tiles' edges.  Each of the p
+    terms of grad_k is a few roundings of size eps (|w_k| + |w_j| + |v_k| +
+    |v_j|) / (d^2 + eta^2) (|A| and |2 eta d r^2| are at most r), so the sums
+    may differ by 64 eps of the terms' bounds."""
+    rng = np.random.default_rng(p)
+    ev = rng.permutation(spectra.config2(p, seed=p))
+    w, v = rng.standard_normal(p), rng.standard_normal(p)
+    eta = 1.0 / math.sqrt(p)
+    L = _native.load()
+    d = [torch.from_numpy(a).cuda() for a in (ev, w, v)]
+    got = torch.empty_like(d[0])
+    _native.check(L.shrk_stieltjes_adjoint_dev(
+        d[0].data_ptr(), p, eta, d[1].data_ptr(), d[2].data_ptr(), 0, got.data_ptr(),
+        torch.cuda.current_stream().cuda_stream))
+    got = got.cpu().numpy()
+    at = np.unique(np.r_[0:min(p, 40), np.arange(255, p, 256), max(0, p - 40):p])[:400]
+    ref = oracle.adjoint_direct(ev, eta, w, v, idx=at)
+    for i, k in enumerate(at):
+        r = 1.0 / ((ev[k] - ev) ** 2 + eta * eta)
+        bound = np.sum((abs(w[k]) + np.abs(w) + abs(v[k]) + np.abs(v)) * r) / p
+        assert abs(got[k] - ref[i]) <= 64 * np.finfo(float).eps * bound, (k, got[k], ref[i])
