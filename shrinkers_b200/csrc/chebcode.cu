@@ -342,6 +342,12 @@ __global__ void __launch_bounds__(TOPO_NT, 1) tree_topology_cta_kernel(
 // update) applied row after row, so w is the sequential result bit for bit;
 // the divisions of 32 rows run in parallel.  Invalid rows (zero masses, the
 // tail of a batch) are skipped.
+// |d| in [2^-900, 2^900), by its exponent: where rcp_rn_mid holds.
+__device__ __forceinline__ bool row_mid(double d) {
+  const unsigned e = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+  return e - (1023u - 900u) < 1800u;
+}
+
 constexpr int ROW_RS = MAX_N + 1;  // shared tile row stride (doubles)
 constexpr int WEIGHT_NT = 128;     // threads per block of the weight kernels
 
@@ -358,13 +364,26 @@ __device__ __forceinline__ void bary_rows_batch(double x, double mass, bool vali
   int hit = -2;
   double m = 0.0;
   if (valid) {
+    // branch-free quotients lam / d = lam * (1/d) (lam is +-1 or +-1/2), in
+    // flight together; a value outside their range redoes the row
+    bool mid = true;
+    double sum = 0.0;
     hit = -1;
-    for (int j = 0; j < n; ++j)
-      if (hit < 0 && x - rt.t[j] == 0.0) hit = j;
+#pragma unroll 4
+    for (int j = 0; j < n; ++j) {
+      const double d = x - rt.t[j];
+      mid = mid && row_mid(d);
+      if (d == 0.0 && hit < 0) hit = j;
+      const double q = rt.lam[j] * copysign(rcp_rn_mid(fabs(d)), d);
+      rt.q[lane * ROW_RS + j] = q;
+      sum += q;
+    }
     if (hit >= 0) {
       m = mass;
+    } else if (mid && row_mid(sum)) {
+      m = mass * copysign(rcp_rn_mid(fabs(sum)), sum);
     } else {
-      double sum = 0.0;
+      sum = 0.0;
       for (int j = 0; j < n; ++j) {
         const double q = rt.lam[j] / (x - rt.t[j]);
         rt.q[lane * ROW_RS + j] = q;
@@ -485,6 +504,8 @@ __device__ __forceinline__ void mirror_f32(const FlatTree& f, int idx, int n, in
     panel[(int64_t)idx * 2 * n + n + lane] = (float)__ldcg(f.w + (int64_t)idx * n + lane);
   }
 }
+
+#include "chebsub.cuh"
 
 // P2M and M2M of a small tree in one launch over a fixed grid, with no
 // read-back (the node count is the breadth-first slot counter): a warp
@@ -659,14 +680,38 @@ __device__ __forceinline__ int eval_node_count(const EvalArgs& a) {
   return a.nn_dev ? *a.nn_dev : a.nn_host;
 }
 
+// The rounded reciprocal of the evaluation's denominators eta^2 + d^2, and
+// quotient w over one: MID takes the branch-free forms, valid where every
+// denominator of a query lies in [2^-400, 2^400] (mid_query), else the
+// compiler's.  The values are the same.
+template <bool MID>
+__device__ __forceinline__ double den_rcp(double a) {
+  return MID ? rcp_rn_mid(a) : __drcp_rn(a);
+}
+template <bool MID>
+__device__ __forceinline__ double den_div(double w, double a) {
+  if (MID) {
+    const double aw = fabs(w);
+    if (w == 0.0 || (aw >= 0x1p-400 && aw <= 0x1p400)) return div_rn_mid(w, a);
+  }
+  return w / a;
+}
+// Sources and nodes lie in [lo, hi], the root's range.
+__device__ __forceinline__ bool mid_query(double x, double lo, double hi, double eta2) {
+  const double far = fmax(fabs(x - lo), fabs(x - hi));
+  return eta2 >= 0x1p-400 && far * far + eta2 <= 0x1p400;
+}
+
 // Exact leaf sum, F64x2 schedule of chebcode.rs:620-649 (x86 semantics).
+template <bool MID>
 __device__ __forceinline__ void leaf_sum(const double* xs, int64_t len, double x, double eta2,
                                          double& lr_out, double& li_out) {
   double ar0 = 0.0, ar1 = 0.0, ai0 = 0.0, ai1 = 0.0;
   int64_t k = 0;
+#pragma unroll 4
   for (; k + 2 <= len; k += 2) {
     const double d0 = x - xs[k], d1 = x - xs[k + 1];
-    const double inv0 = __drcp_rn(eta2 + d0 * d0), inv1 = __drcp_rn(eta2 + d1 * d1);
+    const double inv0 = den_rcp<MID>(eta2 + d0 * d0), inv1 = den_rcp<MID>(eta2 + d1 * d1);
     ar0 = ar0 + d0 * inv0;
     ar1 = ar1 + d1 * inv1;
     ai0 = ai0 + inv0;
@@ -675,7 +720,7 @@ __device__ __forceinline__ void leaf_sum(const double* xs, int64_t len, double x
   double lr = ar0 + ar1, li = ai0 + ai1;
   for (; k < len; ++k) {
     const double d = x - xs[k];
-    const double inv = __drcp_rn(d * d + eta2);
+    const double inv = den_rcp<MID>(d * d + eta2);
     lr += d * inv;
     li += inv;
   }
@@ -689,6 +734,7 @@ __device__ __forceinline__ void leaf_sum(const double* xs, int64_t len, double x
 // the F64x2 schedule, their sum, then the odd tail -- so the result equals
 // leaf_sum bit for bit.  Used when there are too few queries to fill the GPU
 // with one thread each (the reciprocals dominate, the ordered adds are cheap).
+template <bool MID>
 __device__ __forceinline__ void leaf_sum_warp(const double* xs, int64_t len, double x,
                                               double eta2, int lane, double& lr_out,
                                               double& li_out) {
@@ -699,7 +745,7 @@ __device__ __forceinline__ void leaf_sum_warp(const double* xs, int64_t len, dou
     double vr = 0.0, vi = 0.0;
     if (k < len) {
       const double d = x - xs[k];
-      const double inv = __drcp_rn(eta2 + d * d);  // = d * d + eta2 for the tail
+      const double inv = den_rcp<MID>(eta2 + d * d);  // = d * d + eta2 for the tail
       vr = d * inv;
       vi = inv;
     }
@@ -739,42 +785,23 @@ __device__ __forceinline__ void leaf_sum_warp(const double* xs, int64_t len, dou
   li_out = li;
 }
 
-// chebcode.rs:607-711 contribution_f64.  WARP: a warp per query (all lanes
-// walk the same nodes; leaf sums by leaf_sum_warp; lane 0 stores).
-template <bool WARP>
-__global__ void __launch_bounds__(128) cheb_eval_f64(const EvalArgs a) {
-  extern __shared__ __align__(16) unsigned char stage_raw[];
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t t = WARP ? gt >> 5 : gt;
-  const int lane = WARP ? (int)(threadIdx.x & 31) : 0;
+// The tree as the FP64 walk reads it: global arrays, or node records (and
+// node panels) staged in shared memory.
+struct Walk64 {
+  const NodeHdr64* sh;
+  const double* nodes;
+  const double* w;
+};
+
+// chebcode.rs:607-711 contribution_f64 at x.  WARP: a warp per query (all
+// lanes walk the same nodes; leaf sums by leaf_sum_warp).
+template <bool WARP, bool MID>
+__device__ __forceinline__ void walk_f64(const EvalArgs& a, const Walk64& wk, double x, int lane,
+                                         double& re_out, double& im_out) {
   const DevTreeF64& T = a.t;
+  const NodeHdr64* sh = wk.sh;
   const int n = T.n;
-  // Node records in shared memory when they fit (the same values, so the
-  // same arithmetic); the node count is uniform, so is the branch.
-  const NodeHdr64* sh = nullptr;
-  const double* s_nodes = nullptr;
-  if (a.stage_bytes > 0) {
-    const int nn = eval_node_count(a);
-    const size_t hb = (size_t)nn * sizeof(NodeHdr64), pb = (size_t)nn * 2 * n * sizeof(double);
-    if (hb <= (size_t)a.stage_bytes) {
-      NodeHdr64* h = reinterpret_cast<NodeHdr64*>(stage_raw);
-      for (int i = threadIdx.x; i < nn; i += blockDim.x)
-        h[i] = NodeHdr64{T.lo[i], T.hi[i], T.accept_hw[i], T.lo_idx[i], T.hi_idx[i], T.right[i], 0};
-      sh = h;
-      if (hb + pb <= (size_t)a.stage_bytes) {
-        double* d = reinterpret_cast<double*>(stage_raw + hb);
-        for (int i = threadIdx.x; i < nn * n; i += blockDim.x) {
-          d[i] = T.nodes[i];
-          d[nn * n + i] = T.w[i];
-        }
-        s_nodes = d;
-      }
-    }
-    __syncthreads();
-  }
-  if (t >= a.nq) return;  // WARP: whole warps leave together
-  const int nn_s = s_nodes ? eval_node_count(a) : 0;
-  const double x = a.q[t], eta = a.eta, eta2 = eta * eta;
+  const double eta = a.eta, eta2 = eta * eta;
   int32_t stack[MAX_TREE_DEPTH + 2];
   int top = 0;
   stack[top++] = 0;
@@ -786,8 +813,8 @@ __global__ void __launch_bounds__(128) cheb_eval_f64(const EvalArgs a) {
       double lr, li;
       const int64_t l0 = sh ? sh[node].lo_idx : T.lo_idx[node];
       const int64_t l1 = sh ? sh[node].hi_idx : T.hi_idx[node];
-      if (WARP) leaf_sum_warp(a.sorted + l0, l1 - l0, x, eta2, lane, lr, li);
-      else leaf_sum(a.sorted + l0, l1 - l0, x, eta2, lr, li);
+      if (WARP) leaf_sum_warp<MID>(a.sorted + l0, l1 - l0, x, eta2, lane, lr, li);
+      else leaf_sum<MID>(a.sorted + l0, l1 - l0, x, eta2, lr, li);
       re += lr;
       im += eta * li;
       continue;
@@ -796,13 +823,14 @@ __global__ void __launch_bounds__(128) cheb_eval_f64(const EvalArgs a) {
     const double cl = fmax(fmax(lo - x, x - hi), 0.0);
     const double d_sq = fma(cl, cl, eta2);
     if ((sh ? sh[node].accept_hw : T.accept_hw[node]) < d_sq) {
-      const double* ts = (s_nodes ? s_nodes : T.nodes) + (int64_t)node * n;
-      const double* ws = (s_nodes ? s_nodes + (int64_t)nn_s * n : T.w) + (int64_t)node * n;
+      const double* ts = wk.nodes + (int64_t)node * n;
+      const double* ws = wk.w + (int64_t)node * n;
       double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
       int j = 0;
+#pragma unroll 5
       for (; j + 2 <= n; j += 2) {
         const double d0 = x - ts[j], d1 = x - ts[j + 1];
-        const double inv0 = __drcp_rn(eta2 + d0 * d0), inv1 = __drcp_rn(eta2 + d1 * d1);
+        const double inv0 = den_rcp<MID>(eta2 + d0 * d0), inv1 = den_rcp<MID>(eta2 + d1 * d1);
         const double q0 = ws[j] * inv0, q1 = ws[j + 1] * inv1;
         a0 = a0 + q0 * d0;
         a1 = a1 + q1 * d1;
@@ -812,7 +840,7 @@ __global__ void __launch_bounds__(128) cheb_eval_f64(const EvalArgs a) {
       double fr = a0 + a1, fi = b0 + b1;
       for (; j < n; ++j) {
         const double dj = x - ts[j];
-        const double q = ws[j] / (dj * dj + eta2);
+        const double q = den_div<MID>(ws[j], dj * dj + eta2);
         fr += q * dj;
         fi += q;
       }
@@ -827,10 +855,130 @@ __global__ void __launch_bounds__(128) cheb_eval_f64(const EvalArgs a) {
       stack[top++] = node + 1;
     }
   }
+  re_out = re;
+  im_out = im;
+}
+
+template <bool WARP>
+__global__ void __launch_bounds__(128) cheb_eval_f64(const EvalArgs a) {
+  extern __shared__ __align__(16) unsigned char stage_raw[];
+  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t t = WARP ? gt >> 5 : gt;
+  const int lane = WARP ? (int)(threadIdx.x & 31) : 0;
+  const DevTreeF64& T = a.t;
+  const int n = T.n;
+  // Node records in shared memory when they fit (the same values, so the
+  // same arithmetic); the node count is uniform, so is the branch.
+  Walk64 wk{nullptr, T.nodes, T.w};
+  if (a.stage_bytes > 0) {
+    const int nn = eval_node_count(a);
+    const size_t hb = (size_t)nn * sizeof(NodeHdr64), pb = (size_t)nn * 2 * n * sizeof(double);
+    if (hb <= (size_t)a.stage_bytes) {
+      NodeHdr64* h = reinterpret_cast<NodeHdr64*>(stage_raw);
+      for (int i = threadIdx.x; i < nn; i += blockDim.x)
+        h[i] = NodeHdr64{T.lo[i], T.hi[i], T.accept_hw[i], T.lo_idx[i], T.hi_idx[i], T.right[i], 0};
+      wk.sh = h;
+      if (hb + pb <= (size_t)a.stage_bytes) {
+        double* d = reinterpret_cast<double*>(stage_raw + hb);
+        for (int i = threadIdx.x; i < nn * n; i += blockDim.x) {
+          d[i] = T.nodes[i];
+          d[nn * n + i] = T.w[i];
+        }
+        wk.nodes = d;
+        wk.w = d + (int64_t)nn * n;
+      }
+    }
+    __syncthreads();
+  }
+  if (t >= a.nq) return;  // WARP: whole warps leave together
+  const double x = a.q[t];
+  double re, im;
+  if (mid_query(x, T.lo[0], T.hi[0], a.eta * a.eta)) walk_f64<WARP, true>(a, wk, x, lane, re, im);
+  else walk_f64<WARP, false>(a, wk, x, lane, re, im);
   if (lane == 0) epi_store(a.epi, t, x, re, im);
 }
 
-// chebcode.rs:722-828 contribution_fast32.  WARP as cheb_eval_f64.
+// chebcode.rs:722-828 contribution_fast32 at lambda.  WARP, MID as walk_f64;
+// MID here also needs the FP32 denominators in [2^-100, 2^100].
+template <bool MID>
+__device__ __forceinline__ float den_rcp32(float a) {
+  return MID ? rcp_rn_mid(a) : __frcp_rn(a);
+}
+
+template <bool WARP, bool MID>
+__device__ __forceinline__ void walk_f32(const EvalArgs& a, const NodeF32* nfp,
+                                         const float* panel, double lambda, int lane,
+                                         double& re_out, double& im_out) {
+  const int n = a.t.n;
+  const double eta = a.eta, eta2d = eta * eta;
+  const float x = (float)lambda, e32 = (float)eta, eta2 = e32 * e32;
+  float fre[4] = {0.f, 0.f, 0.f, 0.f}, fim[4] = {0.f, 0.f, 0.f, 0.f};
+  double leaf_re = 0.0, leaf_im = 0.0;
+  int32_t stack[MAX_TREE_DEPTH + 2];
+  int top = 0;
+  stack[top++] = 0;
+  while (top > 0) {
+    const int32_t node = stack[--top];
+    const NodeF32 nd = nfp[node];
+    if (nd.right < 0) {
+      double lr, li;
+      if (WARP)
+        leaf_sum_warp<MID>(a.sorted + nd.lo_idx, (int64_t)(nd.hi_idx - nd.lo_idx), lambda, eta2d,
+                           lane, lr, li);
+      else
+        leaf_sum<MID>(a.sorted + nd.lo_idx, (int64_t)(nd.hi_idx - nd.lo_idx), lambda, eta2d, lr,
+                      li);
+      leaf_re += lr;
+      leaf_im += eta * li;
+      continue;
+    }
+    const float cl = fmaxf(fmaxf(nd.lo - x, x - nd.hi), 0.0f);
+    const float d_sq = fmaf(cl, cl, eta2);
+    const float outside = (cl == 0.0f) ? d_sq : OUTSIDE_THETA2 * d_sq;
+    if (nd.accept_hw < outside) {
+      const float* ts = panel + (int64_t)node * 2 * n;
+      const float* ws = ts + n;
+      int j = 0;
+#pragma unroll 2
+      for (; j + 4 <= n; j += 4) {
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const float d = x - ts[j + l];
+          const float inv = den_rcp32<MID>(eta2 + d * d);
+          const float q = ws[j + l] * inv;
+          fre[l] = fre[l] + q * d;
+          fim[l] = fim[l] + q;
+        }
+      }
+      if (j < n) {
+        float dt[4] = {0.f, 0.f, 0.f, 0.f}, wt[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int k = 0; k < n - j; ++k) {
+          dt[k] = x - ts[j + k];
+          wt[k] = ws[j + k];
+        }
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          const float inv = den_rcp32<MID>(eta2 + dt[l] * dt[l]);
+          const float q = wt[l] * inv;
+          fre[l] = fre[l] + q * dt[l];
+          fim[l] = fim[l] + q;
+        }
+      }
+    } else {
+      if (top + 2 > MAX_TREE_DEPTH + 2) {
+        atomicExch(a.err, DEV_ERR_BOUNDS);
+        break;
+      }
+      stack[top++] = nd.right;
+      stack[top++] = node + 1;
+    }
+  }
+  const float hr = (fre[0] + fre[1]) + (fre[2] + fre[3]);
+  const float hi = (fim[0] + fim[1]) + (fim[2] + fim[3]);
+  re_out = leaf_re + (double)hr;
+  im_out = leaf_im + eta * (double)hi;
+}
+
 template <bool WARP>
 __global__ void __launch_bounds__(128) cheb_eval_f32(const EvalArgs a) {
   extern __shared__ __align__(16) unsigned char stage_raw[];
@@ -857,70 +1005,15 @@ __global__ void __launch_bounds__(128) cheb_eval_f32(const EvalArgs a) {
     __syncthreads();
   }
   if (t >= a.nq) return;  // WARP: whole warps leave together
-  const double lambda = a.q[t], eta = a.eta, eta2d = eta * eta;
-  const float x = (float)lambda, e32 = (float)eta, eta2 = e32 * e32;
-  float fre[4] = {0.f, 0.f, 0.f, 0.f}, fim[4] = {0.f, 0.f, 0.f, 0.f};
-  double leaf_re = 0.0, leaf_im = 0.0;
-  int32_t stack[MAX_TREE_DEPTH + 2];
-  int top = 0;
-  stack[top++] = 0;
-  while (top > 0) {
-    const int32_t node = stack[--top];
-    const NodeF32 nd = nfp[node];
-    if (nd.right < 0) {
-      double lr, li;
-      if (WARP)
-        leaf_sum_warp(a.sorted + nd.lo_idx, (int64_t)(nd.hi_idx - nd.lo_idx), lambda, eta2d,
-                      lane, lr, li);
-      else
-        leaf_sum(a.sorted + nd.lo_idx, (int64_t)(nd.hi_idx - nd.lo_idx), lambda, eta2d, lr, li);
-      leaf_re += lr;
-      leaf_im += eta * li;
-      continue;
-    }
-    const float cl = fmaxf(fmaxf(nd.lo - x, x - nd.hi), 0.0f);
-    const float d_sq = fmaf(cl, cl, eta2);
-    const float outside = (cl == 0.0f) ? d_sq : OUTSIDE_THETA2 * d_sq;
-    if (nd.accept_hw < outside) {
-      const float* ts = panel + (int64_t)node * 2 * n;
-      const float* ws = ts + n;
-      int j = 0;
-      for (; j + 4 <= n; j += 4) {
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          const float d = x - ts[j + l];
-          const float inv = __frcp_rn(eta2 + d * d);
-          const float q = ws[j + l] * inv;
-          fre[l] = fre[l] + q * d;
-          fim[l] = fim[l] + q;
-        }
-      }
-      if (j < n) {
-        float dt[4] = {0.f, 0.f, 0.f, 0.f}, wt[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < n - j; ++k) {
-          dt[k] = x - ts[j + k];
-          wt[k] = ws[j + k];
-        }
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-          const float inv = __frcp_rn(eta2 + dt[l] * dt[l]);
-          const float q = wt[l] * inv;
-          fre[l] = fre[l] + q * dt[l];
-          fim[l] = fim[l] + q;
-        }
-      }
-    } else {
-      if (top + 2 > MAX_TREE_DEPTH + 2) {
-        atomicExch(a.err, DEV_ERR_BOUNDS);
-        break;
-      }
-      stack[top++] = nd.right;
-      stack[top++] = node + 1;
-    }
-  }
-  const float hr = (fre[0] + fre[1]) + (fre[2] + fre[3]);
-  const float hi = (fim[0] + fim[1]) + (fim[2] + fim[3]);
-  if (lane == 0) epi_store(a.epi, t, lambda, leaf_re + (double)hr, leaf_im + eta * (double)hi);
+  const double lambda = a.q[t];
+  const double lo = nfp[0].lo, hi = nfp[0].hi, e32 = (float)a.eta;
+  // the root's range in FP32 is rounded: 2 x covers it
+  const double far = 2.0 * fmax(fabs(lambda - lo), fabs(lambda - hi)) + fmax(fabs(lo), fabs(hi));
+  const bool mid = e32 * e32 >= 0x1p-100 && far * far + e32 * e32 <= 0x1p100;
+  double re, im;
+  if (mid) walk_f32<WARP, true>(a, nfp, panel, lambda, lane, re, im);
+  else walk_f32<WARP, false>(a, nfp, panel, lambda, lane, re, im);
+  if (lane == 0) epi_store(a.epi, t, lambda, re, im);
 }
 
 __global__ void tree_init_kernel(BuildArrays b, int64_t ns) {
@@ -977,6 +1070,43 @@ shrk_status tree_weights(const TreeBuild& tb, const double* d_sorted, const doub
   return SHRK_OK;
 }
 
+void cheb_consts(int n, ChebConsts* k) {
+  k->n = n;
+  for (int j = 0; j < n; ++j) {
+    k->sm1[j] = std::cos((double)j * M_PI / (double)(n - 1));
+    const double sign = (j % 2 == 0) ? 1.0 : -1.0;
+    k->lam[j] = (j == 0 || j == n - 1) ? 0.5 * sign : sign;
+  }
+}
+
+// The flat arrays of nn nodes in the TREE_SLOTS scratch.
+shrk_status flat_tree_alloc(int64_t nn, int n, FlatTree& f) {
+  void* q = nullptr;
+  SHRK_TRY(scratch_get(TREE_SLOTS + 0, sizeof(double) * 3 * (size_t)nn, &q));
+  f.lo = (double*)q;
+  f.hi = f.lo + nn;
+  f.accept_hw = f.hi + nn;
+  SHRK_TRY(scratch_get(TREE_SLOTS + 1, sizeof(int64_t) * 2 * (size_t)nn, &q));
+  f.lo_idx = (int64_t*)q;
+  f.hi_idx = f.lo_idx + nn;
+  SHRK_TRY(scratch_get(TREE_SLOTS + 2, sizeof(int32_t) * (size_t)nn, &q));
+  f.right = (int32_t*)q;
+  SHRK_TRY(scratch_get(TREE_SLOTS + 3, sizeof(double) * 2 * (size_t)nn * n, &q));
+  f.nodes = (double*)q;
+  f.w = f.nodes + (size_t)nn * n;
+  return SHRK_OK;
+}
+
+// The f32 mirror of nn nodes.
+shrk_status flat_mirror_alloc(int64_t nn, int n, NodeF32** nf, float** panel) {
+  void* q = nullptr;
+  SHRK_TRY(scratch_get(TREE_SLOTS + 4, sizeof(NodeF32) * (size_t)nn, &q));
+  *nf = (NodeF32*)q;
+  SHRK_TRY(scratch_get(TREE_SLOTS + 5, sizeof(float) * 2 * (size_t)nn * n, &q));
+  *panel = (float*)q;
+  return SHRK_OK;
+}
+
 // Builds the flat tree of d_sorted (ascending) into the TREE_SLOTS scratch.
 // Scratch slots 25/26 hold the breadth-first build arrays.
 shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams& prm,
@@ -988,12 +1118,7 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
     return SHRK_EINVAL;
   }
   ChebConsts k;
-  k.n = prm.n;
-  for (int j = 0; j < prm.n; ++j) {
-    k.sm1[j] = std::cos((double)j * M_PI / (double)(prm.n - 1));
-    const double sign = (j % 2 == 0) ? 1.0 : -1.0;
-    k.lam[j] = (j == 0 || j == prm.n - 1) ? 0.5 * sign : sign;
-  }
+  cheb_consts(prm.n, &k);
   void* p64 = nullptr;
   void* p32 = nullptr;
   SHRK_TRY(scratch_get(25, sizeof(int64_t) * 2 * (size_t)cap, &p64));
@@ -1018,19 +1143,7 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
   if (ns / std::max<int64_t>(prm.leaf_cap, 1) <= SMALL_TREE_LEAVES) {
     // small tree: the whole topology in one CTA, one read-back of the levels
     // (the flat arrays are sized for the 2 ns node bound)
-    void* q = nullptr;
-    SHRK_TRY(scratch_get(TREE_SLOTS + 0, sizeof(double) * 3 * (size_t)cap, &q));
-    f.lo = (double*)q;
-    f.hi = f.lo + cap;
-    f.accept_hw = f.hi + cap;
-    SHRK_TRY(scratch_get(TREE_SLOTS + 1, sizeof(int64_t) * 2 * (size_t)cap, &q));
-    f.lo_idx = (int64_t*)q;
-    f.hi_idx = f.lo_idx + cap;
-    SHRK_TRY(scratch_get(TREE_SLOTS + 2, sizeof(int32_t) * (size_t)cap, &q));
-    f.right = (int32_t*)q;
-    SHRK_TRY(scratch_get(TREE_SLOTS + 3, sizeof(double) * 2 * (size_t)cap * prm.n, &q));
-    f.nodes = (double*)q;
-    f.w = f.nodes + (size_t)cap * prm.n;
+    SHRK_TRY(flat_tree_alloc(cap, prm.n, f));
     {
       LaunchScope ls("cheb_build", s);
       tree_topology_cta_kernel<<<1, TOPO_NT, 0, s>>>(d_sorted, b, ns, (int64_t)prm.leaf_cap, f, k,
@@ -1116,19 +1229,7 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
     add_launches(3);  // flags, the scan's two kernels, order
   }
   // 3. flat arrays
-  void* q = nullptr;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 0, sizeof(double) * 3 * (size_t)nn, &q));
-  f.lo = (double*)q;
-  f.hi = f.lo + nn;
-  f.accept_hw = f.hi + nn;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 1, sizeof(int64_t) * 2 * (size_t)nn, &q));
-  f.lo_idx = (int64_t*)q;
-  f.hi_idx = f.lo_idx + nn;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 2, sizeof(int32_t) * (size_t)nn, &q));
-  f.right = (int32_t*)q;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 3, sizeof(double) * 2 * (size_t)nn * prm.n, &q));
-  f.nodes = (double*)q;
-  f.w = f.nodes + (size_t)nn * prm.n;
+  SHRK_TRY(flat_tree_alloc(nn, prm.n, f));
   tree_fill_kernel<<<blocks_for(nn, BS), BS, 0, s>>>(d_sorted, b, nn, f, k,
                                                      prm.theta * prm.theta);
   SHRK_CUDA(cudaGetLastError());
@@ -1142,6 +1243,103 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
   //    level-parallel launch per level: at this size the climbing form of
   //    the small trees was measured 2.3x slower)
   return tree_weights(tb, d_sorted, nullptr, f.w, s);
+}
+
+template <int N, int NS>
+shrk_status launch_sub_weights(const double* d_sorted, int leaf_cap, int S, const SubArrays& a,
+                               const FlatTree& f, const SubCharges<NS>& ch, const ChebConsts& k,
+                               double theta_sq, NodeF32* nf, float* panel, int n_sub,
+                               cudaStream_t s) {
+  const size_t bytes = sizeof(double) * S + (SUB_NT / 32) * sizeof(RowSet<N, NS>);
+  SHRK_CUDA(cudaFuncSetAttribute(sub_weights_kernel<N, NS>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  sub_weights_kernel<N, NS><<<n_sub, SUB_NT, bytes, s>>>(d_sorted, leaf_cap, S, a, f, ch, k,
+                                                         theta_sq, nf, panel);
+  SHRK_CUDA(cudaGetLastError());
+  return SHRK_OK;
+}
+
+// The tree of a larger spectrum, subtree by subtree (chebsub.cuh), with the
+// node weights of the NS charge sets in `c` (null: unit masses; set 0 goes to
+// f.w, the others to *wx, contiguous) and, with nf given, the f32 mirror.
+template <int NS>
+shrk_status build_tree_sub(const double* d_sorted, int64_t ns, const ChebParams& prm,
+                           const double* const (&c)[NS], TreeBuild& tb, double** wx, NodeF32** nf,
+                           float** panel, cudaStream_t s) {
+  const int n = prm.n, leaf_cap = (int)std::min<int64_t>(prm.leaf_cap, ns);
+  const int S = sub_sources(ns);
+  ChebConsts k;
+  cheb_consts(n, &k);
+  // Top nodes: at most ns / S inner nodes on each of 48 levels.
+  const size_t tc = 2 * (size_t)(MAX_TREE_DEPTH + 1) * (size_t)(ns / S + 1) + 4;
+  void *p32 = nullptr, *prec = nullptr;
+  SHRK_TRY(scratch_get(26, sizeof(int) * (11 * tc + 8) + sizeof(uint16_t) * SUB_LEVELS * tc,
+                       &p32));
+  SHRK_TRY(scratch_get(25, sizeof(uint2) * 2 * (size_t)ns, &prec));
+  SubArrays a;
+  a.count = (int*)p32;
+  a.t_lo = a.count + 8;
+  a.t_hi = a.t_lo + tc;
+  a.t_lc = a.t_hi + tc;
+  a.t_dep = a.t_lc + tc;
+  a.t_rt = a.t_dep + tc;
+  a.t_up = a.t_rt + tc;
+  a.t_pre = a.t_up + tc;
+  a.t_arrive = a.t_pre + tc;
+  a.s_slot = a.t_arrive + tc;
+  a.s_lo = a.s_slot + tc;
+  a.s_leaves = a.s_lo + tc;
+  a.s_lev = (uint16_t*)(a.s_leaves + tc);
+  a.rec = (uint2*)prec;
+  const double theta_sq = prm.theta * prm.theta;
+  {
+    LaunchScope ls("cheb_build", s);
+    SHRK_CUDA(cudaFuncSetAttribute(top_tree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)TOP_SMEM));
+    top_tree_kernel<<<1, TOP_NT, TOP_SMEM, s>>>(d_sorted, (int)ns, leaf_cap, S, a);
+    SHRK_CUDA(cudaGetLastError());
+    const size_t bytes = sub_topo_bytes(S);
+    SHRK_CUDA(cudaFuncSetAttribute(sub_topology_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // the subtrees of an even spectrum have at least S / 2 sources
+    const int grid = (int)std::min<int64_t>(4 * sm_count(), 2 * (ns / S) + 8);
+    sub_topology_kernel<<<grid, SUB_NT, bytes, s>>>(d_sorted, leaf_cap, S, a);
+    SHRK_CUDA(cudaGetLastError());
+    add_launches(1);
+  }
+  int h[3];
+  SHRK_CUDA(cudaMemcpyAsync(h, a.count, sizeof(h), cudaMemcpyDeviceToHost, s));
+  SHRK_CUDA(cudaStreamSynchronize(s));
+  const int n_sub = h[1], nn = 2 * h[2] - 1;
+  tb.nn = nn;
+  tb.k = k;
+  SHRK_TRY(flat_tree_alloc(nn, n, tb.f));
+  const FlatTree& f = tb.f;
+  SubCharges<NS> ch;
+  ch.c[0] = c[0];
+  ch.w[0] = f.w;
+  if (NS > 1) {
+    void* q = nullptr;
+    SHRK_TRY(scratch_get(31, sizeof(double) * (NS - 1) * (size_t)nn * n, &q));
+    *wx = (double*)q;
+    for (int i = 1; i < NS; ++i) {
+      ch.c[i] = c[i];
+      ch.w[i] = *wx + (size_t)(i - 1) * nn * n;
+    }
+  }
+  NodeF32* m_nf = nullptr;
+  float* m_panel = nullptr;
+  if (nf) {
+    SHRK_TRY(flat_mirror_alloc(nn, n, &m_nf, &m_panel));
+    *nf = m_nf;
+    *panel = m_panel;
+  }
+  LaunchScope ls("cheb_build_weights", s);
+  if (n == 8)
+    return launch_sub_weights<8, NS>(d_sorted, leaf_cap, S, a, f, ch, k, theta_sq, m_nf, m_panel,
+                                     n_sub, s);
+  return launch_sub_weights<11, NS>(d_sorted, leaf_cap, S, a, f, ch, k, theta_sq, m_nf, m_panel,
+                                    n_sub, s);
 }
 
 // ------------------------------------------------------ multi-eta --
@@ -1354,18 +1552,18 @@ static bool fused_build_ok(int64_t ns, const ChebParams& prm) {
   return ns / std::max<int64_t>(prm.leaf_cap, 1) <= SMALL_TREE_LEAVES;
 }
 
+// Spectra whose tree is built subtree by subtree.
+static bool sub_build_ok(int64_t ns, const ChebParams& prm) {
+  return ns > 4096 && ns <= SUB_MAX_NS && (prm.n == 8 || prm.n == 11);
+}
+
 static shrk_status build_tree_fused(const double* d_sorted, int64_t ns, const ChebParams& prm,
                                     FlatTree& f, NodeF32** nf, float** panel, const int** d_nn,
                                     cudaStream_t s) {
   const int64_t cap = std::max<int64_t>(2 * ns, 2);
   const int n = prm.n;
   ChebConsts k;
-  k.n = n;
-  for (int j = 0; j < n; ++j) {
-    k.sm1[j] = std::cos((double)j * M_PI / (double)(n - 1));
-    const double sign = (j % 2 == 0) ? 1.0 : -1.0;
-    k.lam[j] = (j == 0 || j == n - 1) ? 0.5 * sign : sign;
-  }
+  cheb_consts(n, &k);
   constexpr int NLEV = MAX_TREE_DEPTH + 2;
   void* p64 = nullptr;
   void* p32 = nullptr;
@@ -1386,27 +1584,10 @@ static shrk_status build_tree_fused(const double* d_sorted, int64_t ns, const Ch
   b.dep = b.arrive + cap;
   b.rturn = b.dep + cap;
   b.leafpre = b.rturn + cap;
-  void* q = nullptr;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 0, sizeof(double) * 3 * (size_t)cap, &q));
-  f.lo = (double*)q;
-  f.hi = f.lo + cap;
-  f.accept_hw = f.hi + cap;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 1, sizeof(int64_t) * 2 * (size_t)cap, &q));
-  f.lo_idx = (int64_t*)q;
-  f.hi_idx = f.lo_idx + cap;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 2, sizeof(int32_t) * (size_t)cap, &q));
-  f.right = (int32_t*)q;
-  SHRK_TRY(scratch_get(TREE_SLOTS + 3, sizeof(double) * 2 * (size_t)cap * n, &q));
-  f.nodes = (double*)q;
-  f.w = f.nodes + (size_t)cap * n;
+  SHRK_TRY(flat_tree_alloc(cap, n, f));
   NodeF32* mirror = nullptr;
   float* mpanel = nullptr;
-  if (prm.f32) {
-    SHRK_TRY(scratch_get(TREE_SLOTS + 4, sizeof(NodeF32) * (size_t)cap, &q));
-    mirror = (NodeF32*)q;
-    SHRK_TRY(scratch_get(TREE_SLOTS + 5, sizeof(float) * 2 * (size_t)cap * n, &q));
-    mpanel = (float*)q;
-  }
+  if (prm.f32) SHRK_TRY(flat_mirror_alloc(cap, n, &mirror, &mpanel));
   if (ns <= TINY_NS && prm.leaf_cap >= 1) {
     // all the shared memory a CTA may have: what the arrays leave over holds
     // the nodes and weights of a small enough tree
@@ -1464,7 +1645,14 @@ shrk_status chebcode_points(const double* d_q, int64_t nq, const double* d_sorte
   const bool fused = fused_build_ok(ns, prm);
   if (fused)
     SHRK_TRY(build_tree_fused(d_sorted_src, ns, prm, tb.f, &fused_nf, &fused_panel, &d_nn, s));
-  else SHRK_TRY(build_tree_gpu(d_sorted_src, ns, prm, tb, s));
+  bool built = fused;
+  if (!built && sub_build_ok(ns, prm)) {
+    const double* const unit[1] = {nullptr};
+    SHRK_TRY(build_tree_sub<1>(d_sorted_src, ns, prm, unit, tb, nullptr,
+                               prm.f32 ? &fused_nf : nullptr, &fused_panel, s));
+    built = true;
+  }
+  if (!built) SHRK_TRY(build_tree_gpu(d_sorted_src, ns, prm, tb, s));
   const FlatTree& f = tb.f;
   const int nn = tb.nn;
   EvalArgs a;
@@ -1502,12 +1690,8 @@ shrk_status chebcode_points(const double* d_q, int64_t nq, const double* d_sorte
   } else {
     NodeF32* nf = fused_nf;
     float* panel = fused_panel;
-    if (!fused) {
-      void* q = nullptr;
-      SHRK_TRY(scratch_get(TREE_SLOTS + 4, sizeof(NodeF32) * (size_t)nn, &q));
-      nf = (NodeF32*)q;
-      SHRK_TRY(scratch_get(TREE_SLOTS + 5, sizeof(float) * 2 * (size_t)nn * prm.n, &q));
-      panel = (float*)q;
+    if (!built) {
+      SHRK_TRY(flat_mirror_alloc(nn, prm.n, &nf, &panel));
       LaunchScope ls("cheb_build", s);
       tree_f32_kernel<<<blocks_for(nn, 256), 256, 0, s>>>(f, nn, prm.n, nf, panel);
       SHRK_CUDA(cudaGetLastError());
@@ -1544,12 +1728,21 @@ shrk_status chebcode_adjoint(const double* d_ev, int64_t p, double eta, const do
     SHRK_CUDA(cudaGetLastError());
   }
   TreeBuild tb;
-  SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
-  SHRK_TRY(scratch_get(31, sizeof(double) * 2 * (size_t)tb.nn * prm.n, &q));
-  double* ww = (double*)q;
+  double* ww = nullptr;
+  bool built = false;
+  if (sub_build_ok(p, prm)) {
+    const double* const charges[3] = {nullptr, cw, cv};
+    SHRK_TRY(build_tree_sub<3>(ds, p, prm, charges, tb, &ww, nullptr, nullptr, s));
+    built = true;
+  }
+  if (!built) {
+    SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
+    SHRK_TRY(scratch_get(31, sizeof(double) * 2 * (size_t)tb.nn * prm.n, &q));
+    ww = (double*)q;
+    SHRK_TRY(tree_weights(tb, ds, cw, ww, s));
+    SHRK_TRY(tree_weights(tb, ds, cv, ww + (size_t)tb.nn * prm.n, s));
+  }
   double* wv = ww + (size_t)tb.nn * prm.n;
-  SHRK_TRY(tree_weights(tb, ds, cw, ww, s));
-  SHRK_TRY(tree_weights(tb, ds, cv, wv, s));
   AdjEvalArgs a;
   a.x = d_ev;
   a.w = d_gre;
@@ -1590,7 +1783,13 @@ shrk_status chebcode_evaluate_many(const double* d_ev, int64_t p, const double* 
   double first = 0.0, last = 0.0;
   SHRK_TRY(sorted_sources(d_ev, p, &ds, &first, &last, s));
   TreeBuild tb;
-  SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
+  bool built = false;
+  if (sub_build_ok(p, prm)) {
+    const double* const unit[1] = {nullptr};
+    SHRK_TRY(build_tree_sub<1>(ds, p, prm, unit, tb, nullptr, nullptr, nullptr, s));
+    built = true;
+  }
+  if (!built) SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
   ManyArgs a;
   a.x = d_ev;
   a.p = p;
