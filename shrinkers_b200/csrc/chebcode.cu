@@ -55,8 +55,9 @@ struct NodeF32 {
 //      index order (fill_leaves 401-460), 32 rows per step;
 //   5. M2M: from the deepest level up, a warp per internal node merges the
 //      left then the right child's node masses (merge_all_weights 474-506)
-//      -- a launch per level for large trees, the P2M warps climbing from
-//      their leaves for small ones.
+//      -- a launch per level.
+// This level-by-level build serves spectra above 4 194 304 values; the others
+// are built subtree by subtree (chebsub.cuh) or, up to 2 048 values, in one CTA.
 // Every weight is accumulated in the reference's order with the same
 // operations (IEEE division, fused fma where it uses mul_add), so the tree is
 // identical to the sequential build.
@@ -78,7 +79,7 @@ struct BuildArrays {
   int* counter;  // next free BFS slot
   int* levels;   // level L = BFS slots [levels[2L], levels[2L+1])
   int32_t* parent;  // parent slot (-1 at the root)
-  int32_t* arrive;  // children finished per node (the climbing P2M/M2M)
+  int32_t* arrive;  // the leaf starts' prefix count
   int32_t* dep;     // depth
   int32_t* rturn;   // right turns on the path from the root
   int32_t* leafpre; // [ns + 1]: leaf starts, then their exclusive prefix count
@@ -248,22 +249,13 @@ __global__ void tree_fill_kernel(const double* __restrict__ sorted, BuildArrays 
   tree_fill_node(sorted, b, i, f, k, theta_sq);
 }
 
-// The topology of a small tree in one CTA (no launch or read-back per
-// level): splits level by level with a barrier between levels, subtree sizes
-// bottom-up, pre-order indices top-down, the flat arrays.  A warp splits a
-// node: its upper_bound of mid probes 32 evenly spaced positions per step
-// (the range shrinks 33-fold), then scans the last <= 32 -- the same index as
-// tree_split_node's binary search, so the tree is identical.  The levels
-// table is left for the host to read once.
-constexpr int TOPO_NT = 1024;
-// Trees of at most this many leaf-capacities of sources (ns / leaf_cap) are
-// built by tree_topology_cta_kernel: a few hundred to ~2 000 nodes, where one
-// CTA beats two launches per level (a query-grid tree, a small spectrum).
-constexpr int64_t SMALL_TREE_LEAVES = 512;
-
-// The body, for a CTA of any size; parent, dep, rturn and arrive may be null
-// (the one-CTA build of tiny trees keeps its node arrays in shared memory and
-// needs none of them).  Returns the number of levels.
+// The topology of a tiny tree in one CTA: splits level by level with a barrier
+// between levels, subtree sizes bottom-up, pre-order indices top-down, the flat
+// arrays.  A warp splits a node: its upper_bound of mid probes 32 evenly spaced
+// positions per step (the range shrinks 33-fold), then scans the last <= 32 --
+// the same index as tree_split_node's binary search, so the tree is identical.
+// The node arrays are in shared memory; parent, dep, rturn and arrive are not
+// needed (null).  Returns the number of levels.
 __device__ int topology_cta(const double* __restrict__ sorted, BuildArrays b, int64_t ns,
                             int64_t leaf_cap, FlatTree f, ChebConsts k, double theta_sq) {
   constexpr int NLEV = MAX_TREE_DEPTH + 2;
@@ -324,12 +316,6 @@ __device__ int topology_cta(const double* __restrict__ sorted, BuildArrays b, in
   const int nn = b.levels[2 * last - 1];
   for (int i = tid; i < nn; i += nt) tree_fill_node(sorted, b, i, f, k, theta_sq);
   return last;
-}
-
-__global__ void __launch_bounds__(TOPO_NT, 1) tree_topology_cta_kernel(
-    const double* __restrict__ sorted, BuildArrays b, int64_t ns, int64_t leaf_cap, FlatTree f,
-    ChebConsts k, double theta_sq) {
-  (void)topology_cta(sorted, b, ns, leaf_cap, f, k, theta_sq);
 }
 
 // Up to 32 barycentric rows at once, one warp: lane r computes row r's
@@ -506,41 +492,6 @@ __device__ __forceinline__ void mirror_f32(const FlatTree& f, int idx, int n, in
 }
 
 #include "chebsub.cuh"
-
-// P2M and M2M of a small tree in one launch over a fixed grid, with no
-// read-back (the node count is the breadth-first slot counter): a warp
-// fills a leaf, then climbs -- it fences its weights and counts itself in at
-// the parent; the warp that brings the count to two (the last child done)
-// merges the parent (m2m_node, children's weights read past L1) and goes on
-// up, the other stops.  No warp waits on another.  Each node's f32 mirror
-// entry is written once its weights are final (nf null: none).
-__global__ void __launch_bounds__(WEIGHT_NT, 1) tree_p2m_grid_kernel(
-    const double* __restrict__ sorted, BuildArrays b, FlatTree f, double* wout, ChebConsts k,
-    NodeF32* nf, float* panel) {
-  __shared__ RowTile tiles[WEIGHT_NT / 32];
-  RowTile& rt = tiles[threadIdx.x >> 5];
-  const int nn = *b.counter;
-  const int lane = threadIdx.x & 31;
-  const int nw = (int)((gridDim.x * blockDim.x) >> 5);
-  for (int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i < nn; i += nw) {
-    if (b.lc[i] >= 0) continue;  // warp-uniform
-    p2m_leaf(sorted, nullptr, b, i, lane, f, wout, k, rt);
-    if (nf) mirror_f32(f, b.pre[i], k.n, lane, nf, panel);
-    for (int node = i;;) {
-      const int par = b.parent[node];
-      if (par < 0) break;
-      __threadfence();  // this node's weights before the count
-      int seen = 0;
-      if (lane == 0) seen = atomicAdd(&b.arrive[par], 1);
-      seen = __shfl_sync(0xffffffffu, seen, 0);
-      if (seen == 0) break;  // the sibling's warp merges the parent
-      __threadfence();
-      m2m_node(b, par, lane, f, wout, k, true, rt);
-      if (nf) mirror_f32(f, b.pre[par], k.n, lane, nf, panel);
-      node = par;
-    }
-  }
-}
 
 // The whole build of a tiny tree (ns <= TINY_NS sources) in one CTA and one
 // launch: the spectrum and every node array of the topology in shared memory
@@ -1140,37 +1091,6 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
   b.rturn = b.dep + cap;
   b.leafpre = b.rturn + cap;
   constexpr int BS = 256;
-  if (ns / std::max<int64_t>(prm.leaf_cap, 1) <= SMALL_TREE_LEAVES) {
-    // small tree: the whole topology in one CTA, one read-back of the levels
-    // (the flat arrays are sized for the 2 ns node bound)
-    SHRK_TRY(flat_tree_alloc(cap, prm.n, f));
-    {
-      LaunchScope ls("cheb_build", s);
-      tree_topology_cta_kernel<<<1, TOPO_NT, 0, s>>>(d_sorted, b, ns, (int64_t)prm.leaf_cap, f, k,
-                                                     prm.theta * prm.theta);
-      SHRK_CUDA(cudaGetLastError());
-    }
-    int h_lev[2 * NLEV];
-    SHRK_CUDA(cudaMemcpyAsync(h_lev, b.levels, sizeof(h_lev), cudaMemcpyDeviceToHost, s));
-    SHRK_CUDA(cudaStreamSynchronize(s));
-    int last = NLEV - 1;
-    for (int L = 1; L < NLEV; ++L)
-      if (h_lev[2 * L] == h_lev[2 * L + 1]) {
-        last = L;
-        break;
-      }
-    std::vector<int> lb, le;
-    for (int L = 0; L < last; ++L) {
-      lb.push_back(h_lev[2 * L]);
-      le.push_back(h_lev[2 * L + 1]);
-    }
-    tb.nn = le.back();
-    tb.lb = lb;
-    tb.le = le;
-    tb.b = b;
-    tb.k = k;
-    return tree_weights(tb, d_sorted, nullptr, f.w, s);
-  }
   {
     LaunchScope ls("cheb_build", s);
     tree_init_kernel<<<1, 1, 0, s>>>(b, ns);
@@ -1239,9 +1159,7 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
   tb.le = le;
   tb.b = b;
   tb.k = k;
-  // 4. P2M at the leaves; 5. M2M from the deepest internal level up (a
-  //    level-parallel launch per level: at this size the climbing form of
-  //    the small trees was measured 2.3x slower)
+  // 4. P2M at the leaves; 5. M2M from the deepest internal level up
   return tree_weights(tb, d_sorted, nullptr, f.w, s);
 }
 
@@ -1273,9 +1191,10 @@ shrk_status build_tree_sub(const double* d_sorted, int64_t ns, const ChebParams&
   // Top nodes: at most ns / S inner nodes on each of 48 levels.
   const size_t tc = 2 * (size_t)(MAX_TREE_DEPTH + 1) * (size_t)(ns / S + 1) + 4;
   void *p32 = nullptr, *prec = nullptr;
-  SHRK_TRY(scratch_get(26, sizeof(int) * (11 * tc + 8) + sizeof(uint16_t) * SUB_LEVELS * tc,
+  SHRK_TRY(scratch_get(26, sizeof(int) * (10 * tc + 8) + sizeof(uint16_t) * SUB_LEVELS * tc,
                        &p32));
-  SHRK_TRY(scratch_get(25, sizeof(uint2) * 2 * (size_t)ns, &prec));
+  SHRK_TRY(scratch_get(25, sizeof(uint2) * 2 * (size_t)ns + sizeof(double) * (3 + NS * n) * tc,
+                       &prec));
   SubArrays a;
   a.count = (int*)p32;
   a.t_lo = a.count + 8;
@@ -1284,13 +1203,13 @@ shrk_status build_tree_sub(const double* d_sorted, int64_t ns, const ChebParams&
   a.t_dep = a.t_lc + tc;
   a.t_rt = a.t_dep + tc;
   a.t_up = a.t_rt + tc;
-  a.t_pre = a.t_up + tc;
-  a.t_arrive = a.t_pre + tc;
+  a.t_arrive = a.t_up + tc;
   a.s_slot = a.t_arrive + tc;
   a.s_lo = a.s_slot + tc;
   a.s_leaves = a.s_lo + tc;
   a.s_lev = (uint16_t*)(a.s_leaves + tc);
   a.rec = (uint2*)prec;
+  a.t_rec = (double*)(a.rec + 2 * ns);
   const double theta_sq = prm.theta * prm.theta;
   {
     LaunchScope ls("cheb_build", s);
@@ -1544,89 +1463,56 @@ size_t grid_leaf_cap(size_t n, size_t p, size_t nq, size_t preset_leaf) {
   return std::min(std::max(r, preset_leaf), hi);
 }
 
-// The forward evaluation's tree for a small spectrum (ns / leaf_cap <=
-// SMALL_TREE_LEAVES) with no read-back: the topology in one CTA, then P2M,
-// M2M and the f32 mirror in one launch over a fixed grid
-// (tree_p2m_grid_kernel).
-static bool fused_build_ok(int64_t ns, const ChebParams& prm) {
-  return ns / std::max<int64_t>(prm.leaf_cap, 1) <= SMALL_TREE_LEAVES;
+// Trees built in one CTA: below 2 048 sources a launch more costs what the
+// CTA's barriers do.
+static bool tiny_build_ok(int64_t ns, const ChebParams& prm) {
+  return ns <= TINY_NS && prm.leaf_cap >= 1;
 }
-
-// Spectra whose tree is built subtree by subtree.
+// Trees built subtree by subtree: every other one whose top tree fits one CTA
+// (chebcode, us a call, the level-by-level build against this one: 4 097 values
+// 251 / 180, 20 000 384 / 187, 200 003 531 / 289, 1e6 1 084 / 735).
 static bool sub_build_ok(int64_t ns, const ChebParams& prm) {
-  return ns > 4096 && ns <= SUB_MAX_NS && (prm.n == 8 || prm.n == 11);
+  return ns <= SUB_MAX_NS && (prm.n == 8 || prm.n == 11);
 }
 
-static shrk_status build_tree_fused(const double* d_sorted, int64_t ns, const ChebParams& prm,
-                                    FlatTree& f, NodeF32** nf, float** panel, const int** d_nn,
-                                    cudaStream_t s) {
+// The whole tree of a tiny spectrum in one launch, its node count left on the
+// device.
+static shrk_status build_tree_tiny(const double* d_sorted, int64_t ns, const ChebParams& prm,
+                                   FlatTree& f, NodeF32** nf, float** panel, const int** d_nn,
+                                   cudaStream_t s) {
   const int64_t cap = std::max<int64_t>(2 * ns, 2);
-  const int n = prm.n;
   ChebConsts k;
-  cheb_consts(n, &k);
-  constexpr int NLEV = MAX_TREE_DEPTH + 2;
-  void* p64 = nullptr;
-  void* p32 = nullptr;
-  SHRK_TRY(scratch_get(25, sizeof(int64_t) * 2 * (size_t)cap, &p64));
-  SHRK_TRY(scratch_get(26, sizeof(int32_t) * (8 * (size_t)cap + (size_t)ns + 2 + 8 + 2 * NLEV),
-                       &p32));
-  BuildArrays b;
-  b.blo = (int64_t*)p64;
-  b.bhi = b.blo + cap;
-  b.lc = (int32_t*)p32;
-  b.rc = b.lc + cap;
-  b.size = b.rc + cap;
-  b.pre = b.size + cap;
-  b.counter = (int*)(b.pre + cap);
-  b.levels = b.counter + 8;
-  b.parent = b.levels + 2 * NLEV;
-  b.arrive = b.parent + cap;
-  b.dep = b.arrive + cap;
-  b.rturn = b.dep + cap;
-  b.leafpre = b.rturn + cap;
-  SHRK_TRY(flat_tree_alloc(cap, n, f));
+  cheb_consts(prm.n, &k);
+  void* q = nullptr;
+  SHRK_TRY(scratch_get(26, sizeof(int) * 8, &q));
+  int* nn = (int*)q;
+  SHRK_TRY(flat_tree_alloc(cap, prm.n, f));
   NodeF32* mirror = nullptr;
   float* mpanel = nullptr;
-  if (prm.f32) SHRK_TRY(flat_mirror_alloc(cap, n, &mirror, &mpanel));
-  if (ns <= TINY_NS && prm.leaf_cap >= 1) {
-    // all the shared memory a CTA may have: what the arrays leave over holds
-    // the nodes and weights of a small enough tree
-    static std::atomic<int> optin[64];
-    int dev = 0;
-    SHRK_CUDA(cudaGetDevice(&dev));
-    int smem = dev >= 0 && dev < 64 ? optin[dev].load() : 0;
-    if (smem == 0) {
-      SHRK_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-      SHRK_CUDA(cudaFuncSetAttribute(tree_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     smem));
-      if (dev >= 0 && dev < 64) optin[dev] = smem;
-    }
-    if ((size_t)smem < tiny_smem_bytes(ns)) {
-      set_error("chebcode: the device has too little shared memory per block");
-      return SHRK_ECUDA;
-    }
-    LaunchScope ls("cheb_build", s);
-    tree_tiny_kernel<<<1, TINY_NT, (size_t)smem, s>>>(
-        d_sorted, ns, (int64_t)prm.leaf_cap, f, k, prm.theta * prm.theta, mirror, mpanel,
-        b.counter);
-    SHRK_CUDA(cudaGetLastError());
-  } else {
-    {
-      LaunchScope ls("cheb_build", s);
-      tree_topology_cta_kernel<<<1, TOPO_NT, 0, s>>>(d_sorted, b, ns, (int64_t)prm.leaf_cap, f,
-                                                     k, prm.theta * prm.theta);
-      SHRK_CUDA(cudaGetLastError());
-    }
-    {
-      LaunchScope ls("cheb_build_weights", s);
-      tree_p2m_grid_kernel<<<sm_count() * 4, WEIGHT_NT, 0, s>>>(d_sorted, b, f, f.w, k, mirror,
-                                                                mpanel);
-      SHRK_CUDA(cudaGetLastError());
-    }
+  if (prm.f32) SHRK_TRY(flat_mirror_alloc(cap, prm.n, &mirror, &mpanel));
+  // all the shared memory a CTA may have: what the arrays leave over holds
+  // the nodes and weights of a small enough tree
+  static std::atomic<int> optin[64];
+  int dev = 0;
+  SHRK_CUDA(cudaGetDevice(&dev));
+  int smem = dev >= 0 && dev < 64 ? optin[dev].load() : 0;
+  if (smem == 0) {
+    SHRK_CUDA(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    SHRK_CUDA(cudaFuncSetAttribute(tree_tiny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   smem));
+    if (dev >= 0 && dev < 64) optin[dev] = smem;
   }
+  if ((size_t)smem < tiny_smem_bytes(ns)) {
+    set_error("chebcode: the device has too little shared memory per block");
+    return SHRK_ECUDA;
+  }
+  LaunchScope ls("cheb_build", s);
+  tree_tiny_kernel<<<1, TINY_NT, (size_t)smem, s>>>(d_sorted, ns, (int64_t)prm.leaf_cap, f, k,
+                                                    prm.theta * prm.theta, mirror, mpanel, nn);
+  SHRK_CUDA(cudaGetLastError());
   *nf = mirror;
   *panel = mpanel;
-  *d_nn = b.counter;  // the node count, left on the device by the build
+  *d_nn = nn;
   return SHRK_OK;
 }
 
@@ -1639,20 +1525,20 @@ shrk_status chebcode_points(const double* d_q, int64_t nq, const double* d_sorte
     return SHRK_EINVAL;
   }
   TreeBuild tb;
-  NodeF32* fused_nf = nullptr;
-  float* fused_panel = nullptr;
+  NodeF32* nf = nullptr;
+  float* panel = nullptr;
   const int* d_nn = nullptr;
-  const bool fused = fused_build_ok(ns, prm);
-  if (fused)
-    SHRK_TRY(build_tree_fused(d_sorted_src, ns, prm, tb.f, &fused_nf, &fused_panel, &d_nn, s));
-  bool built = fused;
-  if (!built && sub_build_ok(ns, prm)) {
+  bool built = true;  // the f32 mirror included
+  if (tiny_build_ok(ns, prm)) {
+    SHRK_TRY(build_tree_tiny(d_sorted_src, ns, prm, tb.f, &nf, &panel, &d_nn, s));
+  } else if (sub_build_ok(ns, prm)) {
     const double* const unit[1] = {nullptr};
-    SHRK_TRY(build_tree_sub<1>(d_sorted_src, ns, prm, unit, tb, nullptr,
-                               prm.f32 ? &fused_nf : nullptr, &fused_panel, s));
-    built = true;
+    SHRK_TRY(build_tree_sub<1>(d_sorted_src, ns, prm, unit, tb, nullptr, prm.f32 ? &nf : nullptr,
+                               &panel, s));
+  } else {
+    built = false;
+    SHRK_TRY(build_tree_gpu(d_sorted_src, ns, prm, tb, s));
   }
-  if (!built) SHRK_TRY(build_tree_gpu(d_sorted_src, ns, prm, tb, s));
   const FlatTree& f = tb.f;
   const int nn = tb.nn;
   EvalArgs a;
@@ -1688,8 +1574,6 @@ shrk_status chebcode_points(const double* d_q, int64_t nq, const double* d_sorte
     else cheb_eval_f64<false><<<ctas, 128, smem, s>>>(a);
     SHRK_CUDA(cudaGetLastError());
   } else {
-    NodeF32* nf = fused_nf;
-    float* panel = fused_panel;
     if (!built) {
       SHRK_TRY(flat_mirror_alloc(nn, prm.n, &nf, &panel));
       LaunchScope ls("cheb_build", s);
@@ -1729,13 +1613,10 @@ shrk_status chebcode_adjoint(const double* d_ev, int64_t p, double eta, const do
   }
   TreeBuild tb;
   double* ww = nullptr;
-  bool built = false;
   if (sub_build_ok(p, prm)) {
     const double* const charges[3] = {nullptr, cw, cv};
     SHRK_TRY(build_tree_sub<3>(ds, p, prm, charges, tb, &ww, nullptr, nullptr, s));
-    built = true;
-  }
-  if (!built) {
+  } else {
     SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
     SHRK_TRY(scratch_get(31, sizeof(double) * 2 * (size_t)tb.nn * prm.n, &q));
     ww = (double*)q;
@@ -1783,13 +1664,12 @@ shrk_status chebcode_evaluate_many(const double* d_ev, int64_t p, const double* 
   double first = 0.0, last = 0.0;
   SHRK_TRY(sorted_sources(d_ev, p, &ds, &first, &last, s));
   TreeBuild tb;
-  bool built = false;
   if (sub_build_ok(p, prm)) {
     const double* const unit[1] = {nullptr};
     SHRK_TRY(build_tree_sub<1>(ds, p, prm, unit, tb, nullptr, nullptr, nullptr, s));
-    built = true;
+  } else {
+    SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
   }
-  if (!built) SHRK_TRY(build_tree_gpu(ds, p, prm, tb, s));
   ManyArgs a;
   a.x = d_ev;
   a.p = p;

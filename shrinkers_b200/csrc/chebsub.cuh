@@ -6,7 +6,7 @@
 // Here the topology and the weights take three launches:
 //   1. top_tree_kernel (one CTA): splits nodes until they hold at most S
 //      sources (or are leaves); each of those roots a subtree.  The searches
-//      start on every (ns/16384)-th source, kept in shared memory, and end
+//      start on every (ns/12000)-th source, kept in shared memory, and end
 //      with one window of loads, so a level costs two memory round trips.
 //   2. sub_topology_kernel (a CTA per subtree): splits on in shared memory,
 //      local breadth-first order, and counts leaves.  The tree is full, so a
@@ -22,26 +22,30 @@
 // same bit for bit.  Up to three charge sets share the rows' quotients.
 #pragma once
 
-constexpr int SUB_S_MAX = 4096;    // most sources of a subtree with inner nodes
+constexpr int SUB_S_MAX = 2048;    // most sources of a subtree with inner nodes
 constexpr int SUB_S_MIN = 512;
 constexpr int SUB_NT = 256;
 constexpr int TOP_NT = 1024;
-constexpr int TOP_COARSE = 16384;  // sources of the coarse search table
-constexpr int TOP_FRONT = 1024;    // nodes still to split on one level: ns / S
+constexpr int TOP_COARSE = 12000;  // sources of the coarse search table
+constexpr int TOP_FRONT = 2048;    // nodes still to split on one level: ns / S
 constexpr int64_t SUB_MAX_NS = (int64_t)TOP_FRONT * SUB_S_MAX;
+constexpr int SUB_REC = 512;        // node records staged in shared memory
 constexpr int SUB_LEVELS = MAX_TREE_DEPTH + 2;
 
-// Sources of a subtree: about 256 - 512 subtrees, one or two CTAs per SM.
+// Sources of a subtree: several hundred subtrees, whose uneven sizes then
+// average out over the SMs (with subtrees of 4 096 at p = 1e6, 375 CTAs, the SM
+// with the most work had 2.8 times the mean).
 inline int sub_sources(int64_t ns) {
   int S = SUB_S_MIN;
-  while (S < SUB_S_MAX && ns / S > 256) S *= 2;
+  while (S < SUB_S_MAX && ns / S > 512) S *= 2;
   return S;
 }
 
 struct SubArrays {
   // top nodes by breadth-first slot; rc = lc + 1, lc < 0: a subtree's root; t_up:
-  // parent (-1: none), t_pre: pre-order index, t_arrive: children finished
-  int *t_lo, *t_hi, *t_lc, *t_dep, *t_rt, *t_up, *t_pre, *t_arrive;
+  // parent (-1: none), t_arrive: children finished
+  int *t_lo, *t_hi, *t_lc, *t_dep, *t_rt, *t_up, *t_arrive;
+  double* t_rec;              // [top node][3 + NS n]: range, pre-order index, node weights
   int *s_slot, *s_lo, *s_leaves;
   uint16_t* s_lev;            // [subtree][SUB_LEVELS]: local level starts
   uint2* rec;                 // subtree at source lo: nodes from rec[2 lo], local order:
@@ -64,7 +68,9 @@ __global__ void __launch_bounds__(TOP_NT, 1) top_tree_kernel(const double* __res
   TopNode* front = reinterpret_cast<TopNode*>(coarse + TOP_COARSE);
   __shared__ int n_top, n_sub, n_next;
   constexpr int GL = 8;  // lanes per node
-  const int tid = threadIdx.x, gl = tid % GL, grp = tid / GL;
+  const int tid = threadIdx.x, gl = tid % GL;
+  // the first 32 nodes of a level go to 32 warps
+  const int grp = (tid >> 5) + (TOP_NT / 32) * ((tid & 31) / GL);
   const unsigned gmask = 0xffu << (tid & 24);
   const int g = (ns + TOP_COARSE - 1) / TOP_COARSE, nc = (ns + g - 1) / g;
   const int most = max(S, leaf_cap);
@@ -106,17 +112,20 @@ __global__ void __launch_bounds__(TOP_NT, 1) top_tree_kernel(const double* __res
       // first coarse source of the node above mid, then the window before it
       const int c0 = e.lo / g + 1, c1 = (e.hi - 1) / g + 1;
       int x = c0, y = c1;
-      while (x < y) {
-        const int m = (x + y) >> 1;
-        if (mid < coarse[m]) y = m;
-        else x = m + 1;
+      while (x < y) {  // a group's lanes probe 8 positions a round
+        const int span = y - x, m = x + (int)(((unsigned)span * (2 * gl + 1)) >> 4);
+        const unsigned up = __ballot_sync(gmask, mid < coarse[m]) >> (tid & 24) & 0xffu;
+        const int f = up ? __ffs(up) - 1 : GL;  // first probe above mid
+        const int below = x + (int)(((unsigned)span * (2 * f - 1)) >> 4);
+        if (f < GL) y = x + (int)(((unsigned)span * (2 * f + 1)) >> 4);
+        if (f > 0) x = below + 1;
       }
       const int from = x > c0 ? (x - 1) * g + 1 : e.lo, to = x < c1 ? x * g : e.hi;
       int split = to;
-      for (int b = from; b < to && split == to; b += 8 * GL) {
+      for (int b = from; b < to && split == to; b += 12 * GL) {
         unsigned gt = 0;  // bit u: source b + u GL + gl is above mid
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
+        for (int u = 0; u < 12; ++u) {
           const int i = b + u * GL + gl;
           if (i < to && mid < sorted[i]) gt |= 1u << u;
         }
@@ -127,15 +136,13 @@ __global__ void __launch_bounds__(TOP_NT, 1) top_tree_kernel(const double* __res
       }
       if (split == e.lo || split == e.hi) split = (int)(((int64_t)e.lo + e.hi) / 2);
       if (gl < 2) {  // lane 0: the left child, lane 1: the right one
-        int slot = 0;
-        if (gl == 0) {
-          slot = atomicAdd(&n_top, 2);
-          a.t_lc[e.slot] = slot;
-        }
-        slot = __shfl_sync(3u << (tid & 24), slot, tid & 24) + gl;
         const double edge = sorted[split - 1 + gl];
-        if (gl == 0) place(slot, e.slot, e.lo, split, depth + 1, e.rt, e.lov, edge, next);
-        else place(slot, e.slot, split, e.hi, depth + 1, e.rt + 1, edge, e.hiv, next);
+        int slot = 0;
+        if (gl == 0) slot = atomicAdd(&n_top, 2);
+        slot = __shfl_sync(3u << (tid & 24), slot, tid & 24);
+        if (gl == 0) a.t_lc[e.slot] = slot;
+        place(slot + gl, e.slot, gl ? split : e.lo, gl ? e.hi : split, depth + 1, e.rt + gl,
+              gl ? edge : e.lov, gl ? e.hiv : edge, next);
       }
     }
     __syncthreads();
@@ -294,8 +301,11 @@ __device__ __forceinline__ void bary_rows_set(double x, const double (&mass)[NS]
     for (int j = N - 1; j >= 0; --j) {
       const double d = x - rs.t[j];
       plain = plain && row_mid(d);
-      if (d == 0.0) hit = j;  // the first one counts
-      q[j] = copysign(k.lam[j] * rcp_rn_mid(fabs(d)), (j & 1) ? -d : d);  // lam_j: sign (-1)^j
+      if (((__double2hiint(d) & 0x7fffffff) | __double2loint(d)) == 0) hit = j;  // the first counts
+      // lam_j = (-1)^j, halved at both ends
+      double r = rcp_rn_mid(fabs(d));
+      if (j == 0 || j == N - 1) r *= 0.5;
+      q[j] = copysign(r, (j & 1) ? -d : d);
     }
 #pragma unroll
     for (int j = 0; j < N; ++j) sum += q[j];
@@ -368,9 +378,10 @@ struct SubCharges {
 template <int N, int NS>
 __device__ __forceinline__ void p2m_set(const double* src, int64_t g0, int64_t cnt, double lo,
                                         double hi, int64_t idx, const SubCharges<NS>& ch,
-                                        const ChebConsts& k, int lane, RowSet<N, NS>& rs) {
+                                        const ChebConsts& k, const double* sm1, int lane,
+                                        RowSet<N, NS>& rs) {
   const double c = 0.5 * (lo + hi), l = 0.5 * (hi - lo);
-  if (lane < N) rs.t[lane] = c + l * k.sm1[lane];
+  if (lane < N) rs.t[lane] = c + l * sm1[lane];
   __syncwarp();
   double w[NS] = {};
   for (int64_t q0 = 0; q0 < cnt; q0 += 32) {
@@ -390,24 +401,23 @@ __device__ __forceinline__ void p2m_set(const double* src, int64_t g0, int64_t c
 
 // M2M of node idx over [lo, hi]: its children (flat indices kid, over
 // [klo, khi], per lane: the left child for lanes below N, the right above).
-// CG: the children's weights may come from another SM in this launch.
-template <int N, int NS, bool CG>
+template <int N, int NS>
 __device__ __forceinline__ void m2m_set(double lo, double hi, int64_t idx, double klo, double khi,
                                         int64_t kid, const SubCharges<NS>& ch,
-                                        const ChebConsts& k, int lane, RowSet<N, NS>& rs) {
+                                        const ChebConsts& k, const double* sm1, int lane,
+                                        RowSet<N, NS>& rs) {
   const double c = 0.5 * (lo + hi), l = 0.5 * (hi - lo);
-  if (lane < N) rs.t[lane] = c + l * k.sm1[lane];
+  if (lane < N) rs.t[lane] = c + l * sm1[lane];
   __syncwarp();
   double x = 0.0, mass[NS] = {}, w[NS] = {};
   int on = 0;
   if (lane < 2 * N) {
     const int ti = lane < N ? lane : lane - N;
     const double kc = 0.5 * (klo + khi), kl = 0.5 * (khi - klo);
-    x = kc + kl * k.sm1[ti];
+    x = kc + kl * sm1[ti];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const double* mp = ch.w[s] + kid * N + ti;
-      mass[s] = CG ? __ldcg(mp) : *mp;
+      mass[s] = ch.w[s][kid * N + ti];
       if (mass[s] != 0.0) on |= 1 << s;
     }
   }
@@ -430,12 +440,14 @@ __device__ __forceinline__ void fill_flat(const FlatTree& f, int64_t idx, double
 }
 
 template <int N, int NS>
-__global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
+__global__ void __launch_bounds__(SUB_NT, 4) sub_weights_kernel(
     const double* __restrict__ sorted, int leaf_cap, int S, SubArrays a, FlatTree f,
     SubCharges<NS> ch, ChebConsts k, double theta_sq, NodeF32* nf, float* panel) {
   extern __shared__ __align__(16) unsigned char sub_sm[];
   double* src = reinterpret_cast<double*>(sub_sm);
   __shared__ uint16_t lev[SUB_LEVELS];
+  __shared__ uint2 rec_s[SUB_REC];
+  __shared__ double sm1[N];
   __shared__ int part[SUB_NT / 32], n_lev;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   RowSet<N, NS>& rs = reinterpret_cast<RowSet<N, NS>*>(src + S)[warp];
@@ -448,6 +460,7 @@ __global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
     if (a.s_lo[i] < lo0) b += a.s_leaves[i];
   b = __reduce_add_sync(0xffffffffu, b);
   if (lane == 0) part[warp] = b;
+  if (tid < N) sm1[tid] = k.sm1[tid];
   const bool leaf = cnt <= leaf_cap || d0 >= MAX_TREE_DEPTH;
   if (!leaf) {
     for (int i = tid; i < cnt; i += SUB_NT) src[i] = sorted[lo0 + i];
@@ -461,9 +474,9 @@ __global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
   if (leaf) {
     const double lo = sorted[lo0], hi = sorted[lo0 + cnt - 1];
     if (tid == 0) fill_flat(f, root, lo, hi, lo0, (int64_t)lo0 + cnt, -1, theta_sq);
-    if (tid < N) f.nodes[root * N + tid] = 0.5 * (lo + hi) + 0.5 * (hi - lo) * k.sm1[tid];
+    if (tid < N) f.nodes[root * N + tid] = 0.5 * (lo + hi) + 0.5 * (hi - lo) * sm1[tid];
     if (warp == 0) {
-      p2m_set<N, NS>(sorted + lo0, lo0, cnt, lo, hi, root, ch, k, lane, rs);
+      p2m_set<N, NS>(sorted + lo0, lo0, cnt, lo, hi, root, ch, k, sm1, lane, rs);
       __syncwarp();
       if (nf) mirror_f32(f, (int)root, N, lane, nf, panel);
     }
@@ -475,14 +488,20 @@ __global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
     }
     __syncthreads();
     const int levels = n_lev, nn = lev[levels];
+    // the node records, in shared memory unless there are very many
     const uint2* rec = a.rec + 2 * (int64_t)lo0;
+    if (nn <= SUB_REC) {
+      for (int i = tid; i < nn; i += SUB_NT) rec_s[i] = rec[i];
+      __syncthreads();
+      rec = rec_s;
+    }
     // P2M first: the longest chains of work start at once
     for (int i = warp; i < nn; i += SUB_NT / 32) {
       const uint2 r = rec[i];
       if (r.y & 0xffff) continue;
       const int lo = r.x & 0xffff, hi = r.x >> 16;
       p2m_set<N, NS>(src + lo, (int64_t)lo0 + lo, hi - lo, src[lo], src[hi - 1],
-                     root + (r.y >> 16), ch, k, lane, rs);
+                     root + (r.y >> 16), ch, k, sm1, lane, rs);
     }
     for (int i = tid; i < nn; i += SUB_NT) {
       const uint2 r = rec[i];
@@ -494,7 +513,7 @@ __global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
       const int i = e / N, j = e - i * N;
       const uint2 r = rec[i];
       const double lo = src[r.x & 0xffff], hi = src[(r.x >> 16) - 1];
-      f.nodes[(root + (r.y >> 16)) * N + j] = 0.5 * (lo + hi) + 0.5 * (hi - lo) * k.sm1[j];
+      f.nodes[(root + (r.y >> 16)) * N + j] = 0.5 * (lo + hi) + 0.5 * (hi - lo) * sm1[j];
     }
     for (int l = levels - 2; l >= 0; --l) {
       __syncthreads();
@@ -503,9 +522,9 @@ __global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
         const int lc = r.y & 0xffff;
         if (!lc) continue;
         const uint2 kr = rec[lane < N ? lc : lc + 1];
-        m2m_set<N, NS, false>(src[r.x & 0xffff], src[(r.x >> 16) - 1], root + (r.y >> 16),
+        m2m_set<N, NS>(src[r.x & 0xffff], src[(r.x >> 16) - 1], root + (r.y >> 16),
                               src[kr.x & 0xffff], src[(kr.x >> 16) - 1], root + (kr.y >> 16), ch,
-                              k, lane, rs);
+                              k, sm1, lane, rs);
       }
     }
     if (nf) {
@@ -515,31 +534,72 @@ __global__ void __launch_bounds__(SUB_NT, 3) sub_weights_kernel(
     }
   }
   if (warp != 0) return;
-  // Warp 0 did (or passed a barrier after) the root's weights.  Up the top
-  // tree: in pre-order a left child follows its parent, so the parent's index
-  // and range come from its children's.
+  // Up the top tree.  Warp 0 did (or passed a barrier after) the root's
+  // weights.  In pre-order a left child follows its parent, so the parent's
+  // index and range come from its children's; each finished top node leaves
+  // them and its weights in one record (slot pairs are (odd, even)), so that a
+  // merge waits for one load after the count.
+  constexpr int TW = 3 + NS * N;
   int64_t idx = root;
-  for (int up = a.t_up[slot]; up >= 0; up = a.t_up[slot]) {
-    if (lane == 0) a.t_pre[slot] = (int)idx;
-    __syncwarp();
-    __threadfence();  // this node's index, range and weights before the count
+  double lo = sorted[lo0], hi = sorted[lo0 + cnt - 1], w[NS];
+#pragma unroll
+  for (int c = 0; c < NS; ++c) w[c] = lane < N ? ch.w[c][idx * N + lane] : 0.0;
+  for (int up = a.t_up[slot]; up >= 0;) {
+    double* mine = a.t_rec + (int64_t)slot * TW;
+    if (lane == 0) {
+      mine[0] = lo;
+      mine[1] = hi;
+      mine[2] = (double)idx;
+    }
+#pragma unroll
+    for (int c = 0; c < NS; ++c)
+      if (lane < N) mine[3 + c * N + lane] = w[c];
+    const int next_up = a.t_up[up], up_lo = a.t_lo[up], up_hi = a.t_hi[up];
+    __threadfence();  // this node's record before the count
     __syncwarp();
     int seen = 0;
     if (lane == 0) seen = atomicAdd(&a.t_arrive[up], 1);
     seen = __shfl_sync(0xffffffffu, seen, 0);
     if (seen == 0) return;  // the sibling's warp merges the parent
     __threadfence();
-    const int lc = a.t_lc[up];
-    const int64_t left = __ldcg(&a.t_pre[lc]), right = __ldcg(&a.t_pre[lc + 1]);
-    const double lo = __ldcg(&f.lo[left]), lhi = __ldcg(&f.hi[left]);
-    const double rlo = __ldcg(&f.lo[right]), hi = __ldcg(&f.hi[right]);
-    idx = left - 1;
-    if (lane == 0) fill_flat(f, idx, lo, hi, a.t_lo[up], a.t_hi[up], (int)right, theta_sq);
-    if (lane < N) f.nodes[idx * N + lane] = 0.5 * (lo + hi) + 0.5 * (hi - lo) * k.sm1[lane];
-    m2m_set<N, NS, true>(lo, hi, idx, lane < N ? lo : rlo, lane < N ? lhi : hi,
-                         lane < N ? left : right, ch, k, lane, rs);
+    const bool is_left = slot & 1;
+    const double* other = a.t_rec + (int64_t)(is_left ? slot + 1 : slot - 1) * TW;
+    const double o_lo = __ldcg(other), o_hi = __ldcg(other + 1), o_idx = __ldcg(other + 2);
+    const int ti = lane < N ? lane : lane - N;
+    const bool from_left = lane < N, own = from_left == is_left;
+    double mass[NS];
+    int on = 0;
+#pragma unroll
+    for (int c = 0; c < NS; ++c) {
+      const double o = lane < 2 * N ? __ldcg(other + 3 + c * N + ti) : 0.0;
+      const double m = __shfl_sync(0xffffffffu, w[c], ti & 31);
+      mass[c] = lane < 2 * N ? (own ? m : o) : 0.0;
+      if (mass[c] != 0.0) on |= 1 << c;
+    }
+    const double llo = is_left ? lo : o_lo, lhi = is_left ? hi : o_hi;
+    const double rlo = is_left ? o_lo : lo, rhi = is_left ? o_hi : hi;
+    const int64_t right = is_left ? (int64_t)o_idx : idx;
+    idx = (is_left ? idx : (int64_t)o_idx) - 1;
+    lo = llo;
+    hi = rhi;
+    const double pc = 0.5 * (lo + hi), pl = 0.5 * (hi - lo);
+    if (lane == 0) fill_flat(f, idx, lo, hi, up_lo, up_hi, (int)right, theta_sq);
+    if (lane < N) {
+      rs.t[lane] = pc + pl * sm1[lane];
+      f.nodes[idx * N + lane] = rs.t[lane];
+    }
+    __syncwarp();
+    const double klo = from_left ? llo : rlo, khi = from_left ? lhi : rhi;
+    const double x = lane < 2 * N ? 0.5 * (klo + khi) + 0.5 * (khi - klo) * sm1[ti] : 0.0;
+#pragma unroll
+    for (int c = 0; c < NS; ++c) w[c] = 0.0;
+    bary_rows_set<N, NS>(x, mass, on, 2 * N, k, lane, rs, w);
+#pragma unroll
+    for (int c = 0; c < NS; ++c)
+      if (lane < N) ch.w[c][idx * N + lane] = w[c];
     __syncwarp();
     if (nf) mirror_f32(f, (int)idx, N, lane, nf, panel);
     slot = up;
+    up = next_up;
   }
 }
