@@ -399,6 +399,7 @@ struct Tri1Args {
   double* part;    // [2][gridDim.x]
   double* vb;      // [gridDim.x][2][p] per-CTA reflector copies (global form)
   double* wb;      // [gridDim.x][p] per-CTA w = p_j - K v_j (global form)
+  int64_t stop;    // phases to run (the resident kernel takes over there), at most p - 2
 };
 
 // The per-CTA vectors (two reflectors and w, 3 p doubles) live in shared
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(TRI_NT, 1) tridiag1_kernel(const Tri1Args a) {
     if (threadIdx.x == 0) a.part[blockIdx.x] = t;
   }
   grid.sync();
-  for (int64_t j = 0; j + 2 < p; ++j) {
+  for (int64_t j = 0; j < a.stop; ++j) {
     const int par = (int)(j & 1), nxt = par ^ 1;
     vcur = vb + par * p;
     double* vnext = vb + nxt * p;
@@ -609,7 +610,353 @@ __global__ void __launch_bounds__(TRI_NT, 1) tridiag1_kernel(const Tri1Args a) {
     bcur = bnext;
     grid.sync();
   }
-  if (lead && threadIdx.x == 0) a.d[p - 1] = A[(p - 1) + (p - 1) * p];
+  if (lead && threadIdx.x == 0 && a.stop + 2 >= p) a.d[p - 1] = A[(p - 1) + (p - 1) * p];
+}
+
+// ------------------------------------------- resident tridiagonalisation --
+// The one-barrier reduction with the trailing matrix in shared memory: the
+// columns of the last n rows and columns, dealt to the CTAs in turn (14
+// columns of 2 048 rows are 224 KB), stay there until they are used up.
+//
+// tridiag1_kernel moves every trailing element through L2 twice a column and
+// waits for it in rounds: 9.3 us a column at p = 2 048, 5.2 us at 501, where
+// the whole matrix is 2 MB.  Here a column costs one exchange of two vectors
+// and a pass over shared memory.  A thread keeps its rows (tid, tid + NT,
+// ...) of v_j, p_j, w_j and v_{j+1} in registers and walks the CTA's columns
+// eight at a time.  The pivot column of the next phase travels with p_{j+1}:
+// by symmetry its entry r is the pivot row's entry in column r, so each CTA
+// contributes both for its own columns, 16 bytes a column (the update is
+// written so that both triangles round alike).  p_j^T v_j and the reflector
+// come from block sums that every CTA forms from the same values in the same
+// order, so all hold the same bits.
+//
+// CTAs meet once a column at a counter: each adds its arrival (a release after
+// its part) and one thread of each watches for the last (3 100 clocks with 148
+// CTAs, data included; a flag word per CTA, watched by 148 threads of every
+// CTA, took 11 900: the polls queue at the flags' lines).  The launch is
+// cooperative, so all CTAs are resident; a watcher gives up after its budget,
+// records a timeout and the CTA returns, and so do then the others.  One
+// cluster of 16 CTAs with the exchange through distributed shared memory was
+// no faster at 450 columns and below (1.71 ms against 1.65): its barrier takes
+// 1 400 clocks and the scattered remote stores 2 500.
+constexpr size_t RES_SMEM = 224 * 1024;  // for the columns (227 KB less the static part)
+constexpr int RES_COLS = 16;             // most columns of a CTA
+
+struct ResArgs {
+  double* A;        // p x p column-major (both triangles)
+  int64_t p;
+  int resume;       // 0: column 0's reflector first (r0 = 1); 1: from tridiag1_kernel at
+                    // phase r0 - 2, whose reflector (in row r0 - 2) and p vector are in place
+  int r0;           // first row and column held in shared memory
+  double* d;
+  double* e;
+  double* vhead;
+  double* beta;
+  const double* pv;    // resume: p vectors [2][p]
+  double2* px;         // [2][p] (p vector, pivot column) by row
+  unsigned* arrived;   // zeroed: CTAs past their part of the exchanges so far
+  int* err;
+  long long wait_cycles;
+};
+
+template <int NT>
+__device__ __forceinline__ double res_block_sum(double v, double* red) {
+  constexpr int RES_WARPS = NT / 32;
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int w = 0; w < RES_WARPS; ++w) t[w & 3] += red[w];
+  return (t[0] + t[1]) + (t[2] + t[3]);
+}
+
+// Eight per-lane values summed over the warp; lane 4 q gets the sum of c[q].
+__device__ __forceinline__ double warp_sum_of8(const double (&c)[8], int lane) {
+  double h[4], g[2];
+  const bool hi16 = (lane & 16) != 0, hi8 = (lane & 8) != 0, hi4 = (lane & 4) != 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    h[i] = (hi16 ? c[i + 4] : c[i]) + __shfl_xor_sync(0xffffffffu, hi16 ? c[i] : c[i + 4], 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    g[i] = (hi8 ? h[i + 2] : h[i]) + __shfl_xor_sync(0xffffffffu, hi8 ? h[i] : h[i + 2], 8);
+  double v = (hi4 ? g[1] : g[0]) + __shfl_xor_sync(0xffffffffu, hi4 ? g[0] : g[1], 4);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v;
+}
+
+// The reflector of a vector of squared norm norm2 and first entry x0.
+__device__ __forceinline__ void res_reflector(double norm2, double x0, double& alpha, double& head,
+                                              double& beta) {
+  const double sig = norm2 - x0 * x0;
+  alpha = head = x0;
+  beta = 0.0;
+  if (sig > 0.0) {
+    const double nrm = sqrt(norm2);
+    alpha = x0 >= 0.0 ? -nrm : nrm;
+    head = x0 - alpha;
+    beta = 2.0 / (sig + head * head);
+  }
+}
+
+template <int RES_NT, int U>
+__global__ void __launch_bounds__(RES_NT, 1) tridiag_res_kernel(const ResArgs a) {
+  constexpr int RES_WARPS = RES_NT / 32;
+  extern __shared__ double res_s[];  // column lc at lc * n
+  __shared__ double red[2][RES_WARPS], colsum[RES_WARPS][RES_COLS];
+  __shared__ double2 sc[RES_COLS];   // (v, w) at the CTA's own columns
+  __shared__ double xr[RES_COLS];    // the next pivot row at them
+  __shared__ double s_x0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = (int)gridDim.x, b = (int)blockIdx.x;
+  const int p = (int)a.p, r0 = a.r0, n = p - r0;
+  const int C = n > b ? (n - b + G - 1) / G : 0;  // columns r0 + b + lc G
+  for (int lc = 0; lc < C; ++lc) {
+    const double* src = a.A + (int64_t)(r0 + b + lc * G) * p + r0;
+    for (int i = tid; i < n; i += RES_NT) res_s[lc * n + i] = src[i];
+  }
+  int own[U];  // the CTA's column that is row tid + NT u, or -1
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = tid + u * RES_NT;
+    own[u] = i < n && i % G == b ? i / G : -1;
+  }
+  double v[U];  // v_j at this thread's rows
+  double bcur, head;
+  unsigned epoch = 0;
+  // Warp 0 sums the columns' products over the CTA (a lane a column) and
+  // publishes p and the pivot row.
+  auto exchange = [&](int lcs, double bn, int par) {
+    __syncthreads();  // colsum and xr are complete
+    ++epoch;
+    if (warp != 0) return;
+    const bool mine = lane >= lcs && lane < C;
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    if (mine)
+#pragma unroll
+      for (int w = 0; w < RES_WARPS; ++w) t[w & 3] += colsum[w][lane];
+    const double pc = ((t[0] + t[1]) + (t[2] + t[3])) * bn;
+    if (mine) a.px[(int64_t)par * p + r0 + b + lane * G] = make_double2(pc, xr[lane]);
+    __syncwarp();
+    if (lane == 0)
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.arrived) : "memory");
+  };
+  // Everyone's part of the last exchange; false (in every thread) on timeout.
+  auto wait_all = [&]() -> bool {
+    bool ok = a.wait_cycles > 0;
+    if (ok && tid == 0) {
+      const unsigned want = epoch * (unsigned)G;
+      const long long t0 = clock64();
+      for (;;) {
+        unsigned seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.arrived) : "memory");
+        if (seen >= want) break;
+        if (clock64() - t0 > a.wait_cycles) {
+          ok = false;
+          break;
+        }
+      }
+    }
+    if (!__syncthreads_and(ok)) {
+      if (tid == 0) atomicExch(a.err, DEV_ERR_TIMEOUT);
+      return false;
+    }
+    return true;
+  };
+  // This thread's rows from i2 on of the columns from lcs on: A -= v w_c + w
+  // v_c (upd), then the columns' products with vn into colsum.
+  auto walk = [&](int i2, int lcs, bool upd, const double (&w)[U], const double (&vn)[U]) {
+    for (int lc = lcs; lc < C; lc += 8) {
+      double t[8] = {};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (lc + q >= C) continue;
+        const double2 vw = upd ? sc[lc + q] : make_double2(0.0, 0.0);
+        double* col = res_s + (lc + q) * n;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = tid + u * RES_NT;
+          if (i >= i2 && i < n) {
+            double x = col[i];
+            if (upd) {
+              x = x - (v[u] * vw.y + w[u] * vw.x);
+              col[i] = x;
+            }
+            t[q] = fma(x, vn[u], t[q]);
+            if (i == i2) xr[lc + q] = x;
+          }
+        }
+      }
+      const double ws = warp_sum_of8(t, lane);
+      if ((lane & 3) == 0 && lc + (lane >> 2) < C) colsum[warp][lc + (lane >> 2)] = ws;
+    }
+  };
+
+  int j = r0 - 2, turn = 0;  // turn: the CTA that writes phase j's scalars
+  if (!a.resume) {
+    // reflector 0 from column 0, then p_0 over the columns c >= 1
+    j = 0;
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = tid + u * RES_NT;
+      v[u] = i < n ? a.A[r0 + i] : 0.0;
+      s = fma(v[u], v[u], s);
+    }
+    const double norm2 = res_block_sum<RES_NT>(s, red[0]);  // (a barrier: the columns are in place)
+    double alpha;
+    res_reflector(norm2, a.A[r0], alpha, head, bcur);
+    if (tid == 0) v[0] = head;
+    if (b == 0 && tid == 0) {
+      a.d[0] = a.A[0];
+      a.e[0] = alpha;
+      a.vhead[0] = head;
+      a.beta[0] = bcur;
+    }
+    walk(0, 0, false, v, v);
+    exchange(0, bcur, 0);
+  } else {
+    head = a.vhead[j];
+    bcur = a.beta[j];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = tid + u * RES_NT;
+      v[u] = i < n ? a.A[j + (int64_t)(r0 + i) * p] : 0.0;
+    }
+    __syncthreads();
+  }
+  for (; j + 2 < p; ++j, turn = turn + 1 == G ? 0 : turn + 1) {
+    if (epoch > 0 && !wait_all()) return;
+    const int par = j & 1, k1 = j + 1, k2 = j + 2, i2 = k2 - r0;
+    // p_j, and column j + 1 (rows from j + 1 on) before reflector j
+    double w[U], vn[U], g = 0.0;
+    double2 q1;
+    if (epoch > 0) {
+      const double2* px = a.px + (int64_t)par * p;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = tid + u * RES_NT;
+        const double2 q = i >= i2 && i < n ? __ldcg(px + r0 + i) : make_double2(0.0, 0.0);
+        w[u] = q.x;
+        vn[u] = q.y;
+      }
+      q1 = __ldcg(px + k1);
+    } else {  // the first phase after tridiag1_kernel
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = tid + u * RES_NT;
+        const bool on = i >= i2 && i < n;
+        w[u] = on ? a.pv[(int64_t)par * p + r0 + i] : 0.0;
+        vn[u] = on ? a.A[(r0 + i) + (int64_t)k1 * p] : 0.0;
+      }
+      q1 = make_double2(a.pv[(int64_t)par * p + k1], a.A[k1 + (int64_t)k1 * p]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = tid + u * RES_NT;
+      if (i < i2 || i >= n) v[u] = 0.0;
+      g = fma(w[u], v[u], g);
+    }
+    g = res_block_sum<RES_NT>(g, red[0]) + q1.x * head;
+    if (b == turn) {  // reflector j, below the diagonal of column j
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = tid + u * RES_NT;
+        if (i >= i2 && i < n) a.A[(r0 + i) + (int64_t)j * p] = v[u];
+      }
+    }
+    const bool upd = bcur != 0.0;
+    const double K = 0.5 * bcur * g;
+    const double wj1 = upd ? q1.x - K * head : 0.0;
+    double s = 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = tid + u * RES_NT;
+      const bool on = i >= i2 && i < n;
+      w[u] = upd && on ? w[u] - K * v[u] : 0.0;
+      vn[u] = on ? vn[u] - (v[u] * wj1 + w[u] * head) : 0.0;
+      s = fma(vn[u], vn[u], s);
+      if (i == i2) s_x0 = vn[u];
+      if (on && own[u] >= 0) sc[own[u]] = make_double2(v[u], w[u]);
+    }
+    const double norm2 = res_block_sum<RES_NT>(s, red[1]);  // its barrier covers s_x0 and sc
+    const double dnew = q1.y - 2.0 * head * wj1;
+    const bool last = k2 + 1 >= p;
+    double alpha = s_x0, head_next = s_x0, bnext = 0.0;
+    if (!last) {
+      res_reflector(norm2, s_x0, alpha, head_next, bnext);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (tid + u * RES_NT == i2) vn[u] = head_next;
+    }
+    if (b == turn && tid == 0) {
+      a.d[k1] = dnew;
+      a.e[k1] = alpha;
+      if (!last) {
+        a.vhead[k1] = head_next;
+        a.beta[k1] = bnext;
+      }
+    }
+    // trailing columns c >= j + 2: rank-2 update and the next product
+    const int lcs = i2 > b ? (i2 - b + G - 1) / G : 0;
+    walk(i2, lcs, true, w, vn);
+    if (last) {  // the only entry left
+      __syncthreads();
+      if (tid == 0 && lcs < C) a.d[p - 1] = xr[lcs];
+      break;
+    }
+    exchange(lcs, bnext, par ^ 1);
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = vn[u];
+    head = head_next;
+    bcur = bnext;
+  }
+}
+
+// Rows and columns the kernel holds with `blocks` CTAs.
+int64_t resident_rows(int blocks) {
+  int64_t n = 1;
+  while (sizeof(double) * (size_t)(n + 1) * (size_t)((n + blocks) / blocks) <= RES_SMEM &&
+         (n + blocks) / blocks <= RES_COLS)
+    ++n;
+  return n;
+}
+
+template <int NT, int U>
+shrk_status launch_resident(const ResArgs& a, int blocks, cudaStream_t s) {
+  const int64_t n = a.p - a.r0;
+  const size_t bytes = sizeof(double) * (size_t)n * (size_t)((n + blocks - 1) / blocks);
+  const void* fn = (const void*)tridiag_res_kernel<NT, U>;
+  SHRK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  SHRK_CUDA(cudaMemsetAsync(a.arrived, 0, sizeof(unsigned), s));
+  ResArgs copy = a;
+  void* args[] = {&copy};
+  SHRK_CUDA(cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(NT), args, bytes, s));
+  return SHRK_OK;
+}
+
+// Threads by size (measured, ms for 256 / 512): p = 501 1.55 / 1.67, 1 000
+// 3.55 / 3.82, 1 500 6.58 / 6.48, 2 048 11.57 / 10.26: fewer warps make the
+// block sums short, more of them the update.
+shrk_status tridiag_resident(const ResArgs& a, int blocks, cudaStream_t s) {
+  const int n = (int)(a.p - a.r0);
+  if (n <= 1280) {
+    switch ((n + 255) / 256) {
+      case 0:
+      case 1: return launch_resident<256, 1>(a, blocks, s);
+      case 2: return launch_resident<256, 2>(a, blocks, s);
+      case 3: return launch_resident<256, 3>(a, blocks, s);
+      case 4: return launch_resident<256, 4>(a, blocks, s);
+      default: return launch_resident<256, 5>(a, blocks, s);
+    }
+  }
+  switch ((n + 511) / 512) {
+    case 3: return launch_resident<512, 3>(a, blocks, s);
+    case 4: return launch_resident<512, 4>(a, blocks, s);
+    default: return launch_resident<512, 5>(a, blocks, s);
+  }
 }
 
 // ------------------------------------------------------------ bisection --
@@ -929,11 +1276,11 @@ __global__ void ns_matrix_kernel(double* __restrict__ g, int64_t p) {
 
 // Y[r, jj] = v_{j0+jj}[j0+1+r] (rows of the block's reach, zero above the
 // reflector's first entry), n = p - j0 - 1 rows, nb columns.  Reflector j
-// sits below the diagonal in column j (rowstore 0) or right of it in row j
-// (rowstore 1), its head in vhead[j].
+// sits right of the diagonal in row j (j < in_rows) or below it in column j,
+// its head in vhead[j].
 __global__ void build_y_kernel(const double* __restrict__ A, const double* __restrict__ vhead,
                                const double* __restrict__ beta, int64_t p, int64_t j0, int nb,
-                               int rowstore, double* __restrict__ Y) {
+                               int64_t in_rows, double* __restrict__ Y) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y;
   const int64_t n = p - j0 - 1;
@@ -943,7 +1290,7 @@ __global__ void build_y_kernel(const double* __restrict__ A, const double* __res
   double v = 0.0;
   if (beta[j] == 0.0) v = 0.0;  // no reflection: a zero column of Y
   else if (row == j + 1) v = vhead[j];
-  else if (row > j + 1) v = rowstore ? A[j + row * p] : A[row + j * p];
+  else if (row > j + 1) v = j < in_rows ? A[j + row * p] : A[row + j * p];
   Y[r + (int64_t)jj * n] = v;
 }
 
@@ -1139,61 +1486,90 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
     mirror_lower_kernel<<<dim3(cdiv(p, 256), (unsigned)p), 256, 0, s>>>(A, p);
     SHRK_CUDA(cudaGetLastError());
   }
-  // 1. tridiagonalisation (cooperative: all CTAs resident); one grid barrier
-  // per column (tridiag1_kernel, reflectors in the upper triangle) unless
-  // SHRK_EIGH_TRIDIAG=2 selects the two-barrier form
+  // 1. tridiagonalisation (cooperative: all CTAs resident): the last ~2 070
+  // columns by the resident kernel, those before them by tridiag1_kernel, which
+  // passes the trailing matrix through L2 once a column and leaves reflectors in
+  // the upper triangle's rows.  SHRK_EIGH_TRIDIAG=2 runs the two-barrier form on
+  // every column (reflectors in the lower triangle), SHRK_EIGH_TRI1_GLOBAL=1
+  // tridiag1_kernel with its vectors in global memory.
   const char* tri_env = std::getenv("SHRK_EIGH_TRIDIAG");
-  const int rowstore = (tri_env && std::strcmp(tri_env, "2") == 0) ? 0 : 1;
+  const bool rowstore = !(tri_env && std::strcmp(tri_env, "2") == 0);
+  int64_t in_rows = 0;  // reflectors that tridiag1_kernel left in rows
   {
     int dev = 0, sms = 0, per_sm = 0;
     SHRK_CUDA(cudaGetDevice(&dev));
     SHRK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    // one-barrier form: the per-CTA vectors in shared memory when they fit
-    // (SHRK_EIGH_TRI1_GLOBAL=1 keeps them in global memory at any size)
-    const size_t sh_bytes = sizeof(double) * 3 * (size_t)p;
+    const int blocks = std::min(sms, TRI_NT);  // tridiag1_kernel sums a share a thread
     const char* glob_env = std::getenv("SHRK_EIGH_TRI1_GLOBAL");
-    const bool sh = sh_bytes <= TRI1_SMEM_MAX && !(glob_env && std::strcmp(glob_env, "1") == 0);
-    // rows per lane per step of the trailing update: SHRK_EIGH_TRI1_ROWS (8,
-    // 16 or 32) or by size (measured: 8 best at p = 2 048, 18.8 ms; 16 at
-    // 4 096, 87.3 ms; 32 slower at both)
-    const char* rows_env = std::getenv("SHRK_EIGH_TRI1_ROWS");
-    const int rows = rows_env ? std::atoi(rows_env) : (p >= 3072 ? 16 : 8);
-    const void* tri1 = !sh          ? (const void*)tridiag1_kernel<false>
-                       : rows == 32 ? (const void*)tridiag1_kernel<true, 32>
-                       : rows == 8  ? (const void*)tridiag1_kernel<true, 8>
-                                    : (const void*)tridiag1_kernel<true, 16>;
-    const size_t dyn = rowstore && sh ? sh_bytes : 0;
-    if (dyn > 0)
-      SHRK_CUDA(cudaFuncSetAttribute(tri1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    SHRK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, rowstore ? tri1 : (const void*)tridiag_kernel, TRI_NT, dyn));
-    if (per_sm < 1) {
-      set_error("eigensolver: the tridiagonalisation kernel cannot be resident");
-      return SHRK_ECUDA;
-    }
-    const int blocks = std::min(sms, 2048);
-    if (rowstore) {
-      // p_j [2][p] and the partial sums [2][blocks]; the per-CTA vectors
-      // [blocks][3][p] only when they are not in shared memory
-      const size_t per_cta = sh ? 0 : (size_t)blocks * 3 * (size_t)p;
-      void* vbuf = nullptr;
-      SHRK_TRY(scratch_get(SLOT_VB, sizeof(double) * (per_cta + 2 * (size_t)p + 2 * (size_t)blocks),
-                           &vbuf));
-      double* vbd = (double*)vbuf;
-      Tri1Args ta{A,          p,
-                  d,          e,
-                  vhead,      beta,
-                  vbd + per_cta, vbd + per_cta + 2 * p,
-                  sh ? nullptr : vbd, sh ? nullptr : vbd + (size_t)blocks * 2 * p};
-      void* args[] = {&ta};
-      LaunchScope ls("eigh_tridiag", s);
-      SHRK_CUDA(cudaLaunchCooperativeKernel(tri1, dim3(blocks), dim3(TRI_NT), args, dyn, s));
-    } else {
+    const bool glob = glob_env && std::strcmp(glob_env, "1") == 0;
+    const bool resident = rowstore && !glob && p >= 3;
+    const int64_t held = resident ? resident_rows(blocks) : 0;
+    // phases before the resident kernel (p - 2: all of them)
+    const int64_t stop = resident ? (p - 1 <= held ? 0 : std::max<int64_t>(1, p - 2 - held)) : p - 2;
+    if (rowstore) in_rows = stop;
+    // p_j [2][p], (p, pivot) pairs [2][p], the partial sums [2][blocks] and the
+    // counter; tridiag1_kernel's per-CTA vectors [blocks][3][p] only when they
+    // are not in shared memory
+    const size_t sh_bytes = sizeof(double) * 3 * (size_t)p;
+    const bool sh = sh_bytes <= TRI1_SMEM_MAX && !glob;
+    const size_t per_cta = sh ? 0 : (size_t)blocks * 3 * (size_t)p;
+    void* vbuf = nullptr;
+    SHRK_TRY(scratch_get(SLOT_VB, sizeof(double) * (6 * (size_t)p + 2 * (size_t)blocks + 2 + per_cta),
+                         &vbuf));
+    double2* pairs = (double2*)vbuf;
+    double* pvec = (double*)(pairs + 2 * p);
+    double* sums = pvec + 2 * p;
+    unsigned* arrived = (unsigned*)(sums + 2 * blocks);
+    double* vbd = sums + 2 * blocks + 2;
+    if (!rowstore) {
+      SHRK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)tridiag_kernel,
+                                                              TRI_NT, 0));
+      if (per_sm < 1) {
+        set_error("eigensolver: the tridiagonalisation kernel cannot be resident");
+        return SHRK_ECUDA;
+      }
       TriArgs ta{A, p, d, e, vhead, beta, pv, part, scal};
       void* args[] = {&ta};
       LaunchScope ls("eigh_tridiag", s);
       SHRK_CUDA(cudaLaunchCooperativeKernel((const void*)tridiag_kernel, dim3(blocks),
                                             dim3(TRI_NT), args, 0, s));
+    } else if (stop > 0 || !resident) {
+      // rows per lane per step of the trailing update (measured: 8 best at p =
+      // 2 048; 16 at 4 096; 32 slower at both)
+      const void* tri1 = !sh         ? (const void*)tridiag1_kernel<false>
+                         : p >= 3072 ? (const void*)tridiag1_kernel<true, 16>
+                                     : (const void*)tridiag1_kernel<true, 8>;
+      const size_t dyn = sh ? sh_bytes : 0;
+      if (dyn > 0)
+        SHRK_CUDA(cudaFuncSetAttribute(tri1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+      SHRK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tri1, TRI_NT, dyn));
+      if (per_sm < 1) {
+        set_error("eigensolver: the tridiagonalisation kernel cannot be resident");
+        return SHRK_ECUDA;
+      }
+      Tri1Args ta{A,    p,    d, e, vhead, beta, pvec, sums, sh ? nullptr : vbd,
+                  sh ? nullptr : vbd + (size_t)blocks * 2 * p, stop};
+      void* args[] = {&ta};
+      LaunchScope ls("eigh_tridiag", s);
+      SHRK_CUDA(cudaLaunchCooperativeKernel(tri1, dim3(blocks), dim3(TRI_NT), args, dyn, s));
+    }
+    if (resident) {
+      ResArgs ra;
+      ra.A = A;
+      ra.p = p;
+      ra.resume = stop > 0;
+      ra.r0 = stop > 0 ? (int)stop + 2 : 1;
+      ra.d = d;
+      ra.e = e;
+      ra.vhead = vhead;
+      ra.beta = beta;
+      ra.pv = pvec;
+      ra.px = pairs;
+      ra.arrived = arrived;
+      ra.err = device_error_word();
+      ra.wait_cycles = wait_cycles();
+      LaunchScope ls("eigh_tridiag", s);
+      SHRK_TRY(tridiag_resident(ra, blocks, s));
     }
   }
   // 2. split T, Gershgorin bounds per block, eigenvalue slots (host; O(p))
@@ -1201,7 +1577,10 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   SHRK_CUDA(cudaMemcpyAsync(hd.data(), d, sizeof(double) * p, cudaMemcpyDeviceToHost, s));
   if (p > 1)
     SHRK_CUDA(cudaMemcpyAsync(he.data(), e, sizeof(double) * (p - 1), cudaMemcpyDeviceToHost, s));
+  int timed_out = 0;
+  SHRK_CUDA(cudaMemcpyAsync(&timed_out, device_error_word(), sizeof(int), cudaMemcpyDeviceToHost, s));
   SHRK_CUDA(cudaStreamSynchronize(s));
+  if (timed_out) return check_device_error(s);
   const double eps = 2.220446049250313e-16;
   double tnorm = 0.0;
   for (int64_t i = 0; i < p; ++i) {
@@ -1352,7 +1731,7 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
       {
         LaunchScope ls("eigh_wy_y", s);
         build_y_kernel<<<dim3(cdiv(n, 256), (unsigned)nb), 256, 0, s>>>(A, vhead, beta, p, j0,
-                                                                        nb, rowstore, Y);
+                                                                        nb, in_rows, Y);
         SHRK_CUDA(cudaGetLastError());
       }
       SHRK_TRY(dgemm(true, false, nb, nb, n, 1.0, Y, n, Y, n, 0.0, S, nb, s, "dgemm_wy_yty"));
