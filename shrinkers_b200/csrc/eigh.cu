@@ -145,25 +145,20 @@ __device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double
                : "d"(a), "d"(b));
 }
 
+// One 128 x 128 tile of op(A) op(B) at (i0, j0) over k in [kb, ke).
+struct GemmStage {
+  double As[2][GK2][GP2];  // As[kk][i] = op(A)[i0 + i, k0 + kk]
+  double Bs[2][GK2][GP2];  // Bs[kk][j] = op(B)[k0 + kk, j0 + j]
+};
+
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(256, 1) dgemm_big_kernel(int m, int n, int k, int kz,
-                                                           double alpha,
-                                                           const double* __restrict__ A,
-                                                           int64_t lda,
-                                                           const double* __restrict__ B,
-                                                           int64_t ldb, double beta,
-                                                           double* __restrict__ C,
-                                                           int64_t ldc, int lower) {
-  if (lower && blockIdx.y > blockIdx.x) return;  // a tile wholly above the diagonal
-  __shared__ double As[2][GK2][GP2];  // As[kk][i] = op(A)[i0 + i, k0 + kk]
-  __shared__ double Bs[2][GK2][GP2];  // Bs[kk][j] = op(B)[k0 + kk, j0 + j]
-  const int kb = blockIdx.z * kz, ke = min(k, kb + kz);
-  if (gridDim.z > 1) C += (int64_t)blockIdx.z * m * n;
+__device__ __forceinline__ void gemm_tile(GemmStage& st, int m, int n, int kb, int ke, int i0,
+                                          int j0, const double* __restrict__ A, int64_t lda,
+                                          const double* __restrict__ B, int64_t ldb,
+                                          double (&acc)[4][8][2]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wi = (warp & 3) * 32, wj = (warp >> 2) * 64;  // the warp's block
   const int fr = lane >> 2, fk = lane & 3;                 // fragment row / k
-  const int i0 = blockIdx.x * GT2, j0 = blockIdx.y * GT2;
-  double acc[4][8][2];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -195,10 +190,10 @@ __global__ void __launch_bounds__(256, 1) dgemm_big_kernel(int m, int n, int k, 
 #pragma unroll
     for (int it = 0; it < 4; ++it) {
       const int t = threadIdx.x + it * 256;
-      if (!TA) As[buf][t >> 7][t & 127] = ra[it];
-      else As[buf][t & 7][t >> 3] = ra[it];
-      if (!TB) Bs[buf][t & 7][t >> 3] = rb[it];
-      else Bs[buf][t >> 7][t & 127] = rb[it];
+      if (!TA) st.As[buf][t >> 7][t & 127] = ra[it];
+      else st.As[buf][t & 7][t >> 3] = ra[it];
+      if (!TB) st.Bs[buf][t & 7][t >> 3] = rb[it];
+      else st.Bs[buf][t >> 7][t & 127] = rb[it];
     }
   };
   fetch(kb);
@@ -212,9 +207,9 @@ __global__ void __launch_bounds__(256, 1) dgemm_big_kernel(int m, int n, int k, 
     for (int k4 = 0; k4 < GK2; k4 += 4) {
       double a[4], b[8];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = As[buf][k4 + fk][wi + 8 * r + fr];
+      for (int r = 0; r < 4; ++r) a[r] = st.As[buf][k4 + fk][wi + 8 * r + fr];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) b[c] = Bs[buf][k4 + fk][wj + 8 * c + fr];
+      for (int c = 0; c < 8; ++c) b[c] = st.Bs[buf][k4 + fk][wj + 8 * c + fr];
 #pragma unroll
       for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -226,20 +221,124 @@ __global__ void __launch_bounds__(256, 1) dgemm_big_kernel(int m, int n, int k, 
       buf ^= 1;
     }
   }
+}
+
+// C(i, j) = alpha * tile + beta C (beta = 0: C is not read).  C's entries are
+// read sixteen at a time before any is written (one after the other, as the
+// compiler must keep them, they were 64 L2 round trips: 25 us a tile).
+__device__ __forceinline__ void gemm_store(int m, int n, int i0, int j0, double alpha,
+                                           const double (&acc)[4][8][2], double beta, double* C,
+                                           int64_t ldc) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wi = (warp & 3) * 32, wj = (warp >> 2) * 64, fr = lane >> 2, fk = lane & 3;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c0 = 0; c0 < 8; c0 += 2) {
+    double old[2][2][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int gj = j0 + wj + 8 * c + 2 * fk + h;
-      if (gj >= n) continue;
+    for (int c = 0; c < 2; ++c)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int gi = i0 + wi + 8 * r + fr;
-        if (gi >= m) continue;
-        double* cp = C + gi + (int64_t)gj * ldc;
-        *cp = beta == 0.0 ? alpha * acc[r][c][h] : fma(alpha, acc[r][c][h], beta * *cp);
-      }
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int gj = j0 + wj + 8 * (c0 + c) + 2 * fk + h, gi = i0 + wi + 8 * r + fr;
+          old[c][h][r] = beta != 0.0 && gi < m && gj < n ? C[gi + (int64_t)gj * ldc] : 0.0;
+        }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int gj = j0 + wj + 8 * (c0 + c) + 2 * fk + h, gi = i0 + wi + 8 * r + fr;
+          if (gi >= m || gj >= n) continue;
+          const double v = acc[r][c0 + c][h];
+          C[gi + (int64_t)gj * ldc] =
+              beta == 0.0 ? alpha * v : fma(alpha, v, beta * old[c][h][r]);
+        }
+  }
+}
+
+// The tiles' k steps (GK2 each) numbered tile after tile, CTA c taking the
+// c-th of gridDim.x equal runs, so that every SM works to the end whatever the
+// number of tiles (2048^3 is 256 tiles: two waves of 148, the second a third
+// empty).  A run crosses whole tiles, written straight to C, and at most one
+// tile's tail and one tile's head, kept in slots 2 c and 2 c + 1 of the
+// workspace; dgemm_fixup_kernel adds a divided tile's parts in CTA order.
+struct GemmRuns {
+  int tm, tn;      // tiles along m and n
+  int lower;       // only the tiles on or below the diagonal (tm = tn)
+  int ksteps;      // steps a tile
+  int64_t total;   // steps in all
+  int64_t per;     // CTA c: [c per + min(c, rem), ...): the first rem have one more
+  int rem;
+
+  __host__ __device__ int64_t first(int64_t c) const { return c * per + (c < rem ? c : rem); }
+  __host__ __device__ int cta_of(int64_t step) const {
+    const int64_t head = (int64_t)rem * (per + 1);
+    return (int)(step < head ? step / (per + 1) : rem + (step - head) / per);
+  }
+  // tile t -> (ti, tj), column by column
+  __host__ __device__ void place(int t, int& ti, int& tj) const {
+    if (!lower) {
+      ti = t % tm;
+      tj = t / tm;
+      return;
     }
+    tj = 0;
+    while (t >= tm - tj) t -= tm - tj++;
+    ti = tj + t;
+  }
+};
+
+constexpr int GEMM_SLOT = GT2 * GT2;  // doubles of a partial tile, column-major
+
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(256, 1) dgemm_big_kernel(GemmRuns g, int m, int n, int k,
+                                                           double alpha,
+                                                           const double* __restrict__ A,
+                                                           int64_t lda,
+                                                           const double* __restrict__ B,
+                                                           int64_t ldb, double beta, double* C,
+                                                           int64_t ldc, double* ws) {
+  __shared__ GemmStage st;
+  const int64_t s0 = g.first(blockIdx.x), s1 = g.first((int64_t)blockIdx.x + 1);
+  for (int64_t s = s0; s < s1;) {
+    const int t = (int)(s / g.ksteps), ks = (int)(s - (int64_t)t * g.ksteps);
+    const int ke = (int)min((int64_t)g.ksteps, ks + (s1 - s));
+    int ti, tj;
+    g.place(t, ti, tj);
+    double acc[4][8][2];
+    __syncthreads();  // the last tile's readers are done with the stage
+    gemm_tile<TA, TB>(st, m, n, ks * GK2, min(k, ke * GK2), ti * GT2, tj * GT2, A, lda, B, ldb,
+                      acc);
+    if (ks == 0 && ke == g.ksteps)
+      gemm_store(m, n, ti * GT2, tj * GT2, alpha, acc, beta, C, ldc);
+    else
+      gemm_store(GT2, GT2, 0, 0, 1.0, acc, 0.0,
+                 ws + (int64_t)(2 * blockIdx.x + (s == s0 ? 0 : 1)) * GEMM_SLOT, GT2);
+    s += ke - ks;
+  }
+}
+
+// The divided tiles: a CTA adds 2 048 entries of one tile.
+__global__ void __launch_bounds__(256) dgemm_fixup_kernel(GemmRuns g, int m, int n, double alpha,
+                                                          double beta, double* __restrict__ C,
+                                                          int64_t ldc,
+                                                          const double* __restrict__ ws) {
+  const int t = blockIdx.x;
+  const int64_t a = (int64_t)t * g.ksteps;
+  const int c0 = g.cta_of(a), c1 = g.cta_of(a + g.ksteps - 1);
+  if (c0 == c1) return;
+  int ti, tj;
+  g.place(t, ti, tj);
+  const double* p0 = ws + (int64_t)(2 * c0 + (g.first(c0) == a ? 0 : 1)) * GEMM_SLOT;
+  for (int e = blockIdx.y * 2048 + threadIdx.x; e < blockIdx.y * 2048 + 2048; e += 256) {
+    const int gi = ti * GT2 + (e & (GT2 - 1)), gj = tj * GT2 + e / GT2;
+    if (gi >= m || gj >= n) continue;
+    double v = p0[e];
+    for (int c = c0 + 1; c <= c1; ++c) v += ws[(int64_t)2 * c * GEMM_SLOT + e];
+    double* cp = C + gi + (int64_t)gj * ldc;
+    *cp = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *cp);
   }
 }
 
@@ -967,52 +1066,54 @@ struct EigSlot {
   double lo, hi;
 };
 
-// Number of eigenvalues of T[b0:b1) below x: the negative pivots of the
-// LDL^T factorisation of T - x I, q_i = (d_i - x) - e_{i-1}^2 / q_{i-1}, a
-// pivot smaller than pivmin counting as -pivmin.  q_i is carried as a
-// fraction num / den, num_i = (d_i - x) num_{i-1} - e_{i-1}^2 den_{i-1},
-// den_i = num_{i-1}, so the chain through the block is one FMA a row
-// instead of one division (the count of a 2 048-row block is a chain of
-// 2 048 of them); the pair is rescaled by exact powers of two to stay in
-// range, and reset to (-pivmin, 1) when |q| falls below pivmin.
-__device__ __forceinline__ int sturm(const double* __restrict__ d, const double* __restrict__ e2,
-                                     int b0, int b1, double x, double pivmin) {
-  double num = d[b0] - x, den = 1.0;
-  if (fabs(num) < pivmin) num = -pivmin;
-  int cnt = num < 0.0;
-  for (int i = b0 + 1; i < b1; ++i) {
-    const double nn = fma(d[i] - x, num, -e2[i - 1] * den);
+// Number of eigenvalues of T[b0:b1) below x: the sign changes along the
+// leading minors of T - x I, n_i = (d_i - x) n_{i-1} - e_{i-1}^2 n_{i-2} (the
+// ratios n_i / n_{i-1} are the pivots of its LDL^T factorisation).  A zero minor
+// needs no care: its neighbours have opposite signs, so one change is counted
+// whichever sign the zero carries.  te[i] = (d_i, e_{i-1}^2) of T scaled by a
+// power of two to norm in (1/2, 1], so a minor grows at most threefold a row
+// and, with e^2 above eps^2, two rows lose at most 2^-104: rescaling the pair
+// by its exponent every eight rows keeps it in range.  Three FP64 operations,
+// two integer ones and a load a row (with a range test, a clamp and a select
+// on every row it was 43 instructions).
+__device__ __forceinline__ int sturm(const double2* __restrict__ te, int b0, int b1, double x) {
+  double num = te[b0].x - x, den = 1.0;
+  unsigned cnt = (unsigned)__double2hiint(num) >> 31;
+  auto row = [&](double2 t) {
+    const double nn = fma(t.x - x, num, -(t.y * den));
+    cnt += (unsigned)(__double2hiint(nn) ^ __double2hiint(num)) >> 31;
     den = num;
     num = nn;
-    const double an = fabs(num), ad = fabs(den);
-    if (an < pivmin * ad) {
-      num = -pivmin;
-      den = 1.0;
-    } else {
-      const double mx = fmax(an, ad);
-      if (mx > 0x1p+256 || mx < 0x1p-256) {
-        const double sc = mx > 1.0 ? 0x1p-256 : 0x1p+256;
-        num *= sc;
-        den *= sc;
-      }
-    }
-    cnt += (num < 0.0) != (den < 0.0);
+  };
+  int i = b0 + 1;
+  for (; i + 8 <= b1; i += 8) {
+    double2 t[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) t[u] = te[i + u];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) row(t[u]);
+    // 2^-k of the larger magnitude's exponent, exactly
+    const int hx = max(__double2hiint(num) & 0x7ff00000, __double2hiint(den) & 0x7ff00000);
+    const double sc = __hiloint2double(0x7fe00000 - hx, 0);
+    num *= sc;
+    den *= sc;
   }
-  return cnt;
+  for (; i < b1; ++i) row(te[i]);
+  return (int)cnt;
 }
 
 // G-way multisection, G lanes per eigenvalue (32 / G eigenvalues a warp):
 // each step probes G evenly spaced points of the bracket and keeps the
 // sub-interval where the Sturm count crosses kloc (log2(G + 1) bits a step).
-// A wide G takes fewer steps (latency); a narrow one fewer Sturm counts in
-// all (each is a chain of divisions over the block), which is what bounds
-// large matrices.  Every lane stays in the loop until its warp is done (the
-// shuffles span the warp).
+// A wide G takes fewer steps (each is a chain of one FMA a row), a narrow one
+// fewer counts in all.  Every lane stays in the loop until its warp is done
+// (the shuffles span the warp).  back = the power of two that undoes T's
+// scaling.
 template <int G>
-__global__ void __launch_bounds__(256) bisect_kernel(const double* __restrict__ d,
-                                                     const double* __restrict__ e2,
+__global__ void __launch_bounds__(128) bisect_kernel(const double2* __restrict__ te,
                                                      const EigSlot* __restrict__ slots, int n,
-                                                     double pivmin, double* __restrict__ lam) {
+                                                     double tiny, double back,
+                                                     double* __restrict__ lam) {
   const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = (int)(gt / G);
   const int wl = threadIdx.x & 31, lane = wl % G, g0 = wl - lane;
@@ -1023,10 +1124,10 @@ __global__ void __launch_bounds__(256) bisect_kernel(const double* __restrict__ 
   double lo = sl.lo, hi = sl.hi;
   const double eps = 2.220446049250313e-16;
   for (int it = 0; it < 64; ++it) {
-    if (!done && hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + pivmin) done = true;
+    if (!done && hi - lo <= 2.0 * eps * fmax(fabs(lo), fabs(hi)) + tiny) done = true;
     if (__ballot_sync(0xffffffffu, !done) == 0u) break;
     const double x = lo + (hi - lo) * (double)(lane + 1) / (double)(G + 1);
-    const bool above = !done && sturm(d, e2, sl.b0, sl.b1, x, pivmin) > sl.kloc;
+    const bool above = !done && sturm(te, sl.b0, sl.b1, x) > sl.kloc;
     const unsigned m = (__ballot_sync(0xffffffffu, above) & gmask) >> g0;
     const int f = __ffs(m);  // first probe above kloc, 1-based (0: none)
     const double xl = __shfl_sync(0xffffffffu, x, g0 + (f == 0 ? G - 1 : (f >= 2 ? f - 2 : 0)));
@@ -1041,7 +1142,7 @@ __global__ void __launch_bounds__(256) bisect_kernel(const double* __restrict__ 
       }
     }
   }
-  if (lane == 0 && k < n) lam[k] = 0.5 * (lo + hi);
+  if (lane == 0 && k < n) lam[k] = 0.5 * (lo + hi) * back;
 }
 
 // ------------------------------------------------------ inverse iteration --
@@ -1274,24 +1375,48 @@ __global__ void ns_matrix_kernel(double* __restrict__ g, int64_t p) {
   g[j + i * p] = mv;
 }
 
-// Y[r, jj] = v_{j0+jj}[j0+1+r] (rows of the block's reach, zero above the
-// reflector's first entry), n = p - j0 - 1 rows, nb columns.  Reflector j
-// sits right of the diagonal in row j (j < in_rows) or below it in column j,
-// its head in vhead[j].
+// The reflectors in blocks of WY_NB, block t from column j0 = t WY_NB: Y_t has
+// n_t = p - j0 - 1 rows (its reach) and its own leading dimension n_t; the
+// blocks lie one after the other.  Everything that does not depend on Z -- Y_t,
+// S_t = Y_t^T Y_t, T_t, Y_t T_t -- is formed for all blocks at once before the
+// first product with Z: block by block these were four launches of a few CTAs
+// each, 150 us of latency a block.
+constexpr int WY_NB = 128;
+__host__ __device__ inline int64_t wy_offset(int64_t p, int t) {  // entries of Y before block t
+  return (int64_t)WY_NB * ((int64_t)t * (p - 1) - (int64_t)WY_NB * ((int64_t)t * (t - 1) / 2));
+}
+
+// Y_t[r, jj] = v_{j0+jj}[j0+1+r] (zero above the reflector's first entry, and a
+// zero column past the last reflector or where beta = 0).  Reflector j sits
+// right of the diagonal in row j (j < in_rows) or below it in column j, its
+// head in vhead[j].
 __global__ void build_y_kernel(const double* __restrict__ A, const double* __restrict__ vhead,
-                               const double* __restrict__ beta, int64_t p, int64_t j0, int nb,
-                               int64_t in_rows, double* __restrict__ Y) {
+                               const double* __restrict__ beta, int64_t p, int64_t in_rows,
+                               double* __restrict__ Yall) {
+  const int t = blockIdx.z, jj = blockIdx.y;
+  const int64_t j0 = (int64_t)t * WY_NB, n = p - j0 - 1, j = j0 + jj;
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int jj = blockIdx.y;
-  const int64_t n = p - j0 - 1;
   if (r >= n) return;
-  const int64_t j = j0 + jj;
   const int64_t row = j0 + 1 + r;
   double v = 0.0;
-  if (beta[j] == 0.0) v = 0.0;  // no reflection: a zero column of Y
+  if (j >= p - 2 || beta[j] == 0.0) v = 0.0;
   else if (row == j + 1) v = vhead[j];
   else if (row > j + 1) v = j < in_rows ? A[j + row * p] : A[row + j * p];
-  Y[r + (int64_t)jj * n] = v;
+  Yall[wy_offset(p, t) + r + (int64_t)jj * n] = v;
+}
+
+// S_t = Y_t^T Y_t, k split over gridDim.y slabs [t][slab][WY_NB][WY_NB].
+__global__ void __launch_bounds__(256, 1) wy_gram_kernel(const double* __restrict__ Yall,
+                                                         int64_t p, double* __restrict__ S) {
+  __shared__ GemmStage st;
+  const int t = blockIdx.x, n = (int)(p - (int64_t)t * WY_NB - 1);
+  const int kz = ((n + (int)gridDim.y - 1) / (int)gridDim.y + GK2 - 1) / GK2 * GK2;
+  const int kb = min(n, (int)blockIdx.y * kz), ke = min(n, kb + kz);
+  const double* Y = Yall + wy_offset(p, t);
+  double acc[4][8][2];
+  gemm_tile<true, false>(st, WY_NB, WY_NB, kb, ke, 0, 0, Y, n, Y, n, acc);
+  gemm_store(WY_NB, WY_NB, 0, 0, 1.0, acc, 0.0,
+             S + ((int64_t)t * gridDim.y + blockIdx.y) * WY_NB * WY_NB, WY_NB);
 }
 
 // T of the compact WY form, H_{j0} ... H_{j0+nb-1} = I - Y T Y^T (forward),
@@ -1303,28 +1428,40 @@ __global__ void build_y_kernel(const double* __restrict__ A, const double* __res
 // owner of row i forms x_i = r_i beta_i (1 / U_ii = beta_i exactly) and
 // every lane removes x_i's share from its rows above.  Each step is a
 // shuffle and a few FMAs, so the 128-step chain of a column takes a few
-// microseconds, all columns at once.  U lives in dynamic shared memory.
-constexpr int WY_NB = 128;
+// microseconds, all columns and blocks at once.  U lives in dynamic shared
+// memory.
 constexpr int WY_T_WARPS = 32;  // columns per CTA
 constexpr size_t wy_t_smem() { return sizeof(double) * (WY_NB * (WY_NB + 1) + WY_NB); }
 
 __global__ void __launch_bounds__(WY_T_WARPS * 32) wy_t_kernel(const double* __restrict__ S,
+                                                              int slabs,
                                                               const double* __restrict__ beta,
-                                                              int64_t j0, int nb,
-                                                              double* __restrict__ T) {
+                                                              int64_t p, double* __restrict__ T) {
   extern __shared__ double u[];  // u[i LD + k] = U[i][k], i < k
-  constexpr int LD = WY_NB + 1, QN = WY_NB / 32;
+  constexpr int LD = WY_NB + 1, QN = WY_NB / 32, NN = WY_NB * WY_NB;
   double* rd = u + WY_NB * LD;   // 1 / U_ii
-  for (int idx = threadIdx.x; idx < nb * nb; idx += blockDim.x) {
-    const int i = idx % nb, k = idx / nb;
-    if (i < k) u[i * LD + k] = S[i + k * nb];
+  const int t = blockIdx.y;
+  const int64_t j0 = (int64_t)t * WY_NB;
+  S += (int64_t)t * slabs * NN;
+  T += (int64_t)t * NN;
+  for (int idx = threadIdx.x; idx < NN; idx += blockDim.x) {
+    const int i = idx % WY_NB, k = idx / WY_NB;
+    if (i >= k) continue;
+    double v = 0.0;
+    for (int z = 0; z < slabs; ++z) v += S[(int64_t)z * NN + idx];
+    u[i * LD + k] = v;
   }
-  for (int i = threadIdx.x; i < nb; i += blockDim.x)
-    rd[i] = beta[j0 + i] != 0.0 ? beta[j0 + i] : 1.0;
+  for (int i = threadIdx.x; i < WY_NB; i += blockDim.x) {
+    const double bi = j0 + i < p - 2 ? beta[j0 + i] : 0.0;
+    rd[i] = bi != 0.0 ? bi : 1.0;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int j = blockIdx.x * WY_T_WARPS + (threadIdx.x >> 5);
-  if (j >= nb) return;  // no barrier follows
+  if (j0 + j >= p - 2) {  // past the last reflector
+    for (int i = lane; i < WY_NB; i += 32) T[i + (int64_t)j * WY_NB] = 0.0;
+    return;
+  }
   double r[QN];
 #pragma unroll
   for (int q = 0; q < QN; ++q) r[q] = lane + 32 * q == j ? 1.0 : 0.0;
@@ -1347,8 +1484,23 @@ __global__ void __launch_bounds__(WY_T_WARPS * 32) wy_t_kernel(const double* __r
 #pragma unroll
   for (int q = 0; q < QN; ++q) {
     const int row = lane + 32 * q;
-    if (row < nb) T[row + (int64_t)j * nb] = row <= j ? r[q] : 0.0;
+    T[row + (int64_t)j * WY_NB] = row <= j ? r[q] : 0.0;
   }
+}
+
+// YT_t = Y_t T_t, a CTA per 128 rows of a block.
+__global__ void __launch_bounds__(256, 1) wy_yt_kernel(const double* __restrict__ Yall, int64_t p,
+                                                       const double* __restrict__ T,
+                                                       double* __restrict__ YT) {
+  __shared__ GemmStage st;
+  const int t = blockIdx.y, n = (int)(p - (int64_t)t * WY_NB - 1), i0 = blockIdx.x * GT2;
+  if (i0 >= n) return;
+  const int64_t off = wy_offset(p, t);
+  const int nb = min(WY_NB, n - 1);  // reflectors of the block
+  double acc[4][8][2];
+  gemm_tile<false, false>(st, n, WY_NB, 0, nb, i0, 0, Yall + off, n,
+                          T + (int64_t)t * WY_NB * WY_NB, WY_NB, acc);
+  gemm_store(n, WY_NB, i0, 0, 1.0, acc, 0.0, YT + off, n);
 }
 
 // out[:, k] = U[:, perm[k]]
@@ -1384,7 +1536,6 @@ __global__ void mirror_lower_kernel(double* __restrict__ A, int64_t p) {
 
 unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
-constexpr int NB = WY_NB;              // reflectors per WY block
 // Eigenvalues closer than CLUSTER_TOL ||T|| (numerically equal) share one
 // thread and are orthogonalised by Gram-Schmidt during inverse iteration;
 // every other pair is left to inverse iteration, whose vectors then overlap
@@ -1399,32 +1550,38 @@ constexpr int SLOT_U = 46, SLOT_Z = 47, SLOT_G = 48, SLOT_SMALL = 49, SLOT_WS = 
 }  // namespace
 
 template <bool TA, bool TB>
-static void launch_gemm(bool big, dim3 grid, int m, int n, int k, int kz, double alpha,
-                        const double* A, int64_t lda, const double* B, int64_t ldb, double beta,
-                        double* C, int64_t ldc, int lower, cudaStream_t s) {
-  if (big)
-    dgemm_big_kernel<TA, TB><<<grid, 256, 0, s>>>(m, n, k, kz, alpha, A, lda, B, ldb, beta, C,
-                                                  ldc, lower);
-  else
-    dgemm_kernel<TA, TB><<<grid, 256, 0, s>>>(m, n, k, kz, alpha, A, lda, B, ldb, beta, C, ldc,
-                                              lower);
-}
-
-shrk_status dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
-                  int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
-                  cudaStream_t s, const char* family, bool lower) {
-  if (m <= 0 || n <= 0) return SHRK_OK;
-  if (lower && m != n) {
-    set_error("dgemm: a lower-triangle product must be square");
-    return SHRK_EINVAL;
+static shrk_status gemm_form(int m, int n, int k, double alpha, const double* A, int64_t lda,
+                             const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
+                             int lower, const char* family, cudaStream_t s) {
+  if (m >= GT2 && n >= GT2 && k >= 64) {
+    GemmRuns g;
+    g.tm = (int)cdiv(m, GT2);
+    g.tn = (int)cdiv(n, GT2);
+    g.lower = lower;
+    g.ksteps = (int)cdiv(k, GK2);
+    const int64_t tiles = lower ? (int64_t)g.tm * (g.tm + 1) / 2 : (int64_t)g.tm * g.tn;
+    g.total = tiles * g.ksteps;
+    // at least eight steps a CTA: a part costs a slot written and read
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(sm_count(), g.total / 8));
+    g.per = g.total / grid;
+    g.rem = (int)(g.total % grid);
+    void* ws = nullptr;
+    SHRK_TRY(scratch_get(SLOT_SPLITK, sizeof(double) * 2 * (size_t)grid * GEMM_SLOT, &ws));
+    {
+      LaunchScope ls(family, s);
+      dgemm_big_kernel<TA, TB><<<grid, 256, 0, s>>>(g, m, n, k, alpha, A, lda, B, ldb, beta, C,
+                                                    ldc, (double*)ws);
+      SHRK_CUDA(cudaGetLastError());
+    }
+    // no tile is divided when the runs are whole tiles
+    if (g.rem == 0 && g.per % g.ksteps == 0) return SHRK_OK;
+    LaunchScope ls(family, s);
+    dgemm_fixup_kernel<<<dim3((unsigned)tiles, GEMM_SLOT / 2048), 256, 0, s>>>(
+        g, m, n, alpha, beta, C, ldc, (const double*)ws);
+    SHRK_CUDA(cudaGetLastError());
+    return SHRK_OK;
   }
-  if (m > INT32_MAX || n > INT32_MAX || k > INT32_MAX) {
-    set_error("dgemm: dimensions must be below 2^31");
-    return SHRK_EINVAL;
-  }
-  const bool big = m >= GT2 && n >= GT2 && k >= 64;
-  const int tile = big ? GT2 : GT;
-  const int64_t tiles = (int64_t)cdiv(m, tile) * cdiv(n, tile);
+  const int64_t tiles = (int64_t)cdiv(m, GT) * cdiv(n, GT);
   // too few output tiles to fill the GPU and a long k: split k
   const int64_t want = 2LL * sm_count();
   int splits = 1;
@@ -1440,22 +1597,38 @@ shrk_status dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alph
     ldo = m;
     b = 0.0;
   }
-  const int kz = (int)((k + splits - 1) / splits);
-  const dim3 grid(cdiv(m, tile), cdiv(n, tile), (unsigned)splits);
+  const int kz = (k + splits - 1) / splits;
   {
     LaunchScope ls(family, s);
-    if (!ta && !tb) launch_gemm<false, false>(big, grid, (int)m, (int)n, (int)k, kz, alpha, A, lda, B, ldb, b, out, ldo, lower ? 1 : 0, s);
-    else if (!ta && tb) launch_gemm<false, true>(big, grid, (int)m, (int)n, (int)k, kz, alpha, A, lda, B, ldb, b, out, ldo, lower ? 1 : 0, s);
-    else if (ta && !tb) launch_gemm<true, false>(big, grid, (int)m, (int)n, (int)k, kz, alpha, A, lda, B, ldb, b, out, ldo, lower ? 1 : 0, s);
-    else launch_gemm<true, true>(big, grid, (int)m, (int)n, (int)k, kz, alpha, A, lda, B, ldb, b, out, ldo, lower ? 1 : 0, s);
+    dgemm_kernel<TA, TB><<<dim3(cdiv(m, GT), cdiv(n, GT), (unsigned)splits), 256, 0, s>>>(
+        m, n, k, kz, alpha, A, lda, B, ldb, b, out, ldo, lower);
     SHRK_CUDA(cudaGetLastError());
   }
   if (splits > 1) {
     LaunchScope ls(family, s);
-    dgemm_reduce_kernel<<<cdiv(m * n, 256), 256, 0, s>>>(out, splits, (int)m, (int)n, beta, C, ldc);
+    dgemm_reduce_kernel<<<cdiv((int64_t)m * n, 256), 256, 0, s>>>(out, splits, m, n, beta, C, ldc);
     SHRK_CUDA(cudaGetLastError());
   }
   return SHRK_OK;
+}
+
+shrk_status dgemm(bool ta, bool tb, int64_t m, int64_t n, int64_t k, double alpha, const double* A,
+                  int64_t lda, const double* B, int64_t ldb, double beta, double* C, int64_t ldc,
+                  cudaStream_t s, const char* family, bool lower) {
+  if (m <= 0 || n <= 0) return SHRK_OK;
+  if (lower && m != n) {
+    set_error("dgemm: a lower-triangle product must be square");
+    return SHRK_EINVAL;
+  }
+  if (m > INT32_MAX || n > INT32_MAX || k > INT32_MAX) {
+    set_error("dgemm: dimensions must be below 2^31");
+    return SHRK_EINVAL;
+  }
+  const auto form = !ta && !tb  ? gemm_form<false, false>
+                    : !ta && tb ? gemm_form<false, true>
+                    : ta && !tb ? gemm_form<true, false>
+                                : gemm_form<true, true>;
+  return form((int)m, (int)n, (int)k, alpha, A, lda, B, ldb, beta, C, ldc, lower ? 1 : 0, family, s);
 }
 
 shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaStream_t s) {
@@ -1463,12 +1636,11 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   if (p <= 0) return SHRK_OK;
   const int64_t P2 = p * p;
   void *small = nullptr, *zt = nullptr, *u = nullptr;
-  // small: d, e, e2, vhead, beta, pv, scal (+2), part (<= 4096), lam, perm
+  // small: d, e, vhead, beta, pv, scal (+2), part (<= 4096), lam, perm
   SHRK_TRY(scratch_get(SLOT_SMALL, sizeof(double) * (8 * (size_t)p + 4096 + 16), &small));
   double* d = (double*)small;
   double* e = d + p;
-  double* e2 = e + p;
-  double* vhead = e2 + p;
+  double* vhead = e + p;
   double* beta = vhead + p;
   double* pv = beta + p;
   double* lam = pv + p;
@@ -1597,7 +1769,6 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   // eigenvalue by more than the tridiagonalisation's own backward error;
   // without it a block of rounding noise -- the null space of a low-rank
   // matrix -- would stay one huge cluster)
-  std::vector<double> he2(std::max<int64_t>(p - 1, 1), 0.0);
   std::vector<int> bstart{0};
   for (int64_t i = 0; i + 1 < p; ++i) {
     const double t2 = he[i] * he[i];
@@ -1606,10 +1777,17 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
       he[i] = 0.0;
       bstart.push_back((int)(i + 1));
     }
-    he2[i] = he[i] * he[i];
   }
   bstart.push_back((int)p);
-  const double pivmin = 1e-300 * std::max(1.0, tnorm * tnorm);
+  // T scaled exactly to norm in (1/2, 1] for the counts
+  int te_exp = 0;
+  (void)std::frexp(tnorm, &te_exp);
+  std::vector<double2> hte(p);
+  for (int64_t i = 0; i < p; ++i)
+    hte[i] = make_double2(std::ldexp(hd[i], -te_exp),
+                          i > 0 ? std::ldexp(he[i - 1], -te_exp) * std::ldexp(he[i - 1], -te_exp)
+                                : 0.0);
+  const double tiny = 1e-290;  // far below eps times any entry that is not zero
   std::vector<EigSlot> hslots(p);
   for (size_t b = 0; b + 1 < bstart.size(); ++b) {
     const int b0 = bstart[b], b1 = bstart[b + 1];
@@ -1619,41 +1797,33 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
       lo = std::min(lo, hd[i] - r);
       hi = std::max(hi, hd[i] + r);
     }
-    const double pad = 2.0 * eps * tnorm + 2.0 * pivmin;
-    for (int i = b0; i < b1; ++i) hslots[i] = EigSlot{b0, b1, i - b0, 0, lo - pad, hi + pad};
+    const double pad = 2.0 * eps;
+    lo = std::ldexp(lo, -te_exp) - pad;
+    hi = std::ldexp(hi, -te_exp) + pad;
+    for (int i = b0; i < b1; ++i) hslots[i] = EigSlot{b0, b1, i - b0, 0, lo, hi};
   }
   void* meta = nullptr;
-  SHRK_TRY(scratch_get(SLOT_META, sizeof(EigSlot) * (size_t)p + sizeof(Cluster) * (size_t)p + 256,
-                       &meta));
-  EigSlot* dslots = (EigSlot*)meta;
+  SHRK_TRY(scratch_get(SLOT_META, sizeof(EigSlot) * (size_t)p + sizeof(double2) * (size_t)p +
+                                      sizeof(Cluster) * (size_t)p + 256, &meta));
+  double2* dte = (double2*)meta;
+  EigSlot* dslots = (EigSlot*)(dte + p);
   Cluster* dcl = (Cluster*)(dslots + p);
   SHRK_CUDA(cudaMemcpyAsync(e, he.data(), sizeof(double) * std::max<int64_t>(p - 1, 0),
                             cudaMemcpyHostToDevice, s));
-  SHRK_CUDA(cudaMemcpyAsync(e2, he2.data(), sizeof(double) * std::max<int64_t>(p - 1, 0),
-                            cudaMemcpyHostToDevice, s));
+  SHRK_CUDA(cudaMemcpyAsync(dte, hte.data(), sizeof(double2) * p, cudaMemcpyHostToDevice, s));
   SHRK_CUDA(cudaMemcpyAsync(dslots, hslots.data(), sizeof(EigSlot) * p, cudaMemcpyHostToDevice, s));
   {
     LaunchScope ls("eigh_bisect", s);
-    // probes per eigenvalue: SHRK_EIGH_PROBES (4, 8, 16 or 32) or by size
-    // (measured: 16 best at p = 2 048, 3.1 ms; 8 at 4 096, 7.9 ms)
-    int probes = p >= 3072 ? 8 : (p >= 1024 ? 16 : 32);
-    if (const char* pe = std::getenv("SHRK_EIGH_PROBES")) {
-      const int v = std::atoi(pe);
-      if (v == 4 || v == 8 || v == 16 || v == 32) probes = v;
-    }
-    switch (probes) {
-      case 4:
-        bisect_kernel<4><<<cdiv(p * 4, 256), 256, 0, s>>>(d, e2, dslots, (int)p, pivmin, lam);
-        break;
-      case 8:
-        bisect_kernel<8><<<cdiv(p * 8, 256), 256, 0, s>>>(d, e2, dslots, (int)p, pivmin, lam);
-        break;
-      case 16:
-        bisect_kernel<16><<<cdiv(p * 16, 256), 256, 0, s>>>(d, e2, dslots, (int)p, pivmin, lam);
-        break;
-      default:
-        bisect_kernel<32><<<cdiv(p * 32, 256), 256, 0, s>>>(d, e2, dslots, (int)p, pivmin, lam);
-    }
+    const double back = std::ldexp(1.0, te_exp);
+    // probes per eigenvalue, measured (ms for G = 8 / 16 / 32): p = 501 0.23 /
+    // 0.18 / 0.16, 1 024 0.45 / 0.36 / 0.36, 2 048 0.88 / 0.81 / 1.09, 3 100 1.58 /
+    // 1.57 / 2.31
+    if (p > 4096)
+      bisect_kernel<8><<<cdiv(p * 8, 128), 128, 0, s>>>(dte, dslots, (int)p, tiny, back, lam);
+    else if (p >= 1024)
+      bisect_kernel<16><<<cdiv(p * 16, 128), 128, 0, s>>>(dte, dslots, (int)p, tiny, back, lam);
+    else
+      bisect_kernel<32><<<cdiv(p * 32, 128), 128, 0, s>>>(dte, dslots, (int)p, tiny, back, lam);
     SHRK_CUDA(cudaGetLastError());
   }
   // 3. clusters of close eigenvalues inside each block (host), inverse iteration
@@ -1718,44 +1888,49 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   // 4. back-transformation Zc <- H_0 ... H_{p-3} Zc, blocks from the last
   const int64_t nref = std::max<int64_t>(p - 2, 0);
   if (nref > 0) {
+    const int nblk = (int)((nref + WY_NB - 1) / WY_NB);
+    const int slabs = (int)std::min<int64_t>(8, (p + 255) / 256);
+    const int64_t y_len = wy_offset(p, nblk), NN = (int64_t)WY_NB * WY_NB;
     void* wy = nullptr;
-    SHRK_TRY(scratch_get(SLOT_WY, sizeof(double) * ((size_t)p * NB * 3 + 2 * NB * NB), &wy));
+    SHRK_TRY(scratch_get(SLOT_WY, sizeof(double) * (size_t)(2 * y_len + nblk * NN * (slabs + 1) +
+                                                            (int64_t)WY_NB * p), &wy));
     double* Y = (double*)wy;
-    double* W = Y + (size_t)p * NB;
-    double* W2 = W + (size_t)p * NB;
-    double* S = W2 + (size_t)p * NB;
-    double* T = S + NB * NB;
-    for (int64_t j0 = ((nref - 1) / NB) * NB; j0 >= 0; j0 -= NB) {
-      const int nb = (int)std::min<int64_t>(NB, nref - j0);
-      const int64_t n = p - j0 - 1;
-      {
-        LaunchScope ls("eigh_wy_y", s);
-        build_y_kernel<<<dim3(cdiv(n, 256), (unsigned)nb), 256, 0, s>>>(A, vhead, beta, p, j0,
-                                                                        nb, in_rows, Y);
-        SHRK_CUDA(cudaGetLastError());
-      }
-      SHRK_TRY(dgemm(true, false, nb, nb, n, 1.0, Y, n, Y, n, 0.0, S, nb, s, "dgemm_wy_yty"));
-      {
-        LaunchScope ls("eigh_wy_t", s);
-        static std::atomic<bool> opted[64];
-        int dv = 0;
-        SHRK_CUDA(cudaGetDevice(&dv));
-        if (dv < 0 || dv >= 64 || !opted[dv].load()) {
-          SHRK_CUDA(cudaFuncSetAttribute(wy_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)wy_t_smem()));
-          if (dv >= 0 && dv < 64) opted[dv] = true;
-        }
-        wy_t_kernel<<<(unsigned)cdiv(nb, WY_T_WARPS), WY_T_WARPS * 32, wy_t_smem(), s>>>(
-            S, beta, j0, nb, T);
-        SHRK_CUDA(cudaGetLastError());
-      }
+    double* YT = Y + y_len;
+    double* S = YT + y_len;
+    double* T = S + nblk * NN * slabs;
+    double* W = T + nblk * NN;
+    {
+      LaunchScope ls("eigh_wy_y", s);
+      build_y_kernel<<<dim3(cdiv(p - 1, 256), WY_NB, (unsigned)nblk), 256, 0, s>>>(
+          A, vhead, beta, p, in_rows, Y);
+      SHRK_CUDA(cudaGetLastError());
+    }
+    {
+      LaunchScope ls("dgemm_wy_yty", s);
+      wy_gram_kernel<<<dim3((unsigned)nblk, (unsigned)slabs), 256, 0, s>>>(Y, p, S);
+      SHRK_CUDA(cudaGetLastError());
+    }
+    {
+      LaunchScope ls("eigh_wy_t", s);
+      SHRK_CUDA(cudaFuncSetAttribute(wy_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wy_t_smem()));
+      wy_t_kernel<<<dim3(WY_NB / WY_T_WARPS, (unsigned)nblk), WY_T_WARPS * 32, wy_t_smem(), s>>>(
+          S, slabs, beta, p, T);
+      SHRK_CUDA(cudaGetLastError());
+    }
+    {
+      LaunchScope ls("dgemm_wy_yt", s);
+      wy_yt_kernel<<<dim3(cdiv(p - 1, GT2), (unsigned)nblk), 256, 0, s>>>(Y, p, T, YT);
+      SHRK_CUDA(cudaGetLastError());
+    }
+    for (int t = nblk - 1; t >= 0; --t) {
+      const int64_t j0 = (int64_t)t * WY_NB, n = p - j0 - 1, off = wy_offset(p, t);
+      const int64_t nb = std::min<int64_t>(WY_NB, nref - j0);
       double* Zs = Zc + (j0 + 1);  // rows j0+1 .. p-1 of Zc (leading dimension p)
-      SHRK_TRY(dgemm(true, false, nb, p, n, 1.0, Y, n, Zs, p, 0.0, W, nb, s,
+      SHRK_TRY(dgemm(true, false, nb, p, n, 1.0, Y + off, n, Zs, p, 0.0, W, WY_NB, s,
                      "dgemm_wy_ytz"));  // W = Y^T Zs
-      SHRK_TRY(dgemm(false, false, nb, p, nb, 1.0, T, nb, W, nb, 0.0, W2, nb, s,
-                     "dgemm_wy_tw"));  // W2 = T W
-      SHRK_TRY(dgemm(false, false, n, p, nb, -1.0, Y, n, W2, nb, 1.0, Zs, p, s,
-                     "dgemm_wy_update"));  // Zs -= Y W2
+      SHRK_TRY(dgemm(false, false, n, p, nb, -1.0, YT + off, n, W, WY_NB, 1.0, Zs, p, s,
+                     "dgemm_wy_update"));  // Zs -= (Y T) W
     }
   }
   // ascending eigenvalues; eigenvector columns in that order, into A

@@ -75,3 +75,34 @@ def test_wait_budget_of_zero_times_out():
     assert old > 0
     assert L.shrk_symmetric_eigh(*args) == _native.SHRK_OK
     assert np.max(np.abs(w - np.linalg.eigvalsh(a))) <= 1e-13 * np.max(np.abs(w))
+
+
+@pytest.mark.parametrize("m,n,k", [(128, 128, 64), (129, 128, 65), (128, 131, 71), (256, 384, 64),
+                                   (1200, 1111, 64), (1280, 1920, 72), (2048, 130, 600),
+                                   (130, 2048, 2047)])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1)])
+def test_gemm_in_equal_runs(m, n, k, ta, tb):
+    """The large FP64 product whose k steps are dealt out in equal runs: one
+    run a tile, tiles divided among two and many CTAs, whole tiles only, ragged
+    edges; with C read (beta) and not, beside a guard band that must stay.
+    Each entry is a sum of k products: 4 k eps of their magnitudes."""
+    import torch
+
+    L = _native.load()
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    rnd = lambda r, c: torch.randn(r, c, generator=g, device="cuda", dtype=torch.float64)
+    a = rnd(m, k) if ta else rnd(k, m)  # column-major op(A) m x k
+    b = rnd(k, n) if tb else rnd(n, k)
+    ldc = m + 3
+    opa, opb = (a if ta else a.T), (b if tb else b.T)
+    for beta in (0.0, -0.75):
+        c = rnd(n, ldc)
+        before = c.clone()
+        st = L.shrk_diag_dgemm(ta, tb, m, n, k, 1.25, a.data_ptr(), a.shape[1], b.data_ptr(),
+                               b.shape[1], beta, c.data_ptr(), ldc, None)
+        _native.check(st, "dgemm")
+        torch.cuda.synchronize()
+        ref = 1.25 * (opa @ opb) + beta * before[:, :m].T
+        bound = 4 * k * np.finfo(float).eps * (1.25 * (opa.abs() @ opb.abs()) + before[:, :m].T.abs())
+        assert bool(((c[:, :m].T - ref).abs() <= bound).all())
+        assert torch.equal(c[:, m:], before[:, m:])
