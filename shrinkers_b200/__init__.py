@@ -49,8 +49,9 @@ def _lib():
 
 def _dp(a: np.ndarray):
     """double* to a's data; the caller keeps `a` alive for the call (every
-    call site passes a named array)."""
-    return C.cast(a.ctypes.data, _D)
+    call site passes a named array).  (a.ctypes and C.cast build objects that
+    take a microsecond each.)"""
+    return C.byref(C.c_double.from_address(a.__array_interface__["data"][0]))
 
 
 # ------------------------------------------------------------ parsing --
@@ -103,8 +104,8 @@ def _owned_f64_vec(array, what: str = "eigenvalues") -> np.ndarray:
 
 
 def _require_finite(ev: np.ndarray, what: str) -> None:
-    """python.rs:135-144."""
-    if not np.all(np.isfinite(ev)):
+    """python.rs:135-144.  A finite sum means that every entry is finite."""
+    if not math.isfinite(float(ev.sum())) and not np.all(np.isfinite(ev)):
         raise ValueError(f"{what} must be finite (found NaN or infinity)")
 
 

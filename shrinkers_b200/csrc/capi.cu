@@ -96,6 +96,14 @@ static shrk_status init_context(Context* c, int dev, bool host) {
   c->host = host;
   SHRK_CUDA(cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, dev));
   if (host) SHRK_CUDA(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
+  if (host) {
+    // The error word of host-pointer calls is host memory the device writes
+    // to (never, in a good call), so that reading it costs no copy.
+    SHRK_CUDA(cudaHostAlloc((void**)&c->err, sizeof(int),
+                            cudaHostAllocMapped | cudaHostAllocPortable));
+    *c->err = DEV_ERR_NONE;
+    return SHRK_OK;
+  }
   SHRK_CUDA(cudaMalloc(&c->err, sizeof(int)));
   SHRK_CUDA(cudaMemset(c->err, 0, sizeof(int)));
   return SHRK_OK;
@@ -240,19 +248,23 @@ cudaStream_t library_stream() { return t_cur->stream; }
 
 static shrk_status check_error_word(Context* c, cudaStream_t s) {
   int h = 0;
-  char* st = (c->host && s == c->stream && c->stage && c->stage_used + 256 <= c->stage_bytes)
-                 ? c->stage + c->stage_used
-                 : nullptr;
-  SHRK_CUDA(cudaMemcpyAsync(st ? (void*)st : (void*)&h, c->err, sizeof(int),
-                            cudaMemcpyDeviceToHost, s));
-  SHRK_CUDA(cudaStreamSynchronize(s));
+  if (c->host) {
+    SHRK_CUDA(cudaStreamSynchronize(s));
+    h = *(volatile int*)c->err;
+  } else {
+    SHRK_CUDA(cudaMemcpyAsync(&h, c->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SHRK_CUDA(cudaStreamSynchronize(s));
+  }
   c->stage_busy = false;
-  if (st) std::memcpy(&h, st, sizeof(int));
   for (const auto& q : c->pending) std::memcpy(q.dst, c->stage + q.off, q.bytes);
   c->pending.clear();
   if (h != DEV_ERR_NONE) {
-    SHRK_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), s));
-    SHRK_CUDA(cudaStreamSynchronize(s));
+    if (c->host) {
+      *(volatile int*)c->err = DEV_ERR_NONE;
+    } else {
+      SHRK_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), s));
+      SHRK_CUDA(cudaStreamSynchronize(s));
+    }
     if (h == DEV_ERR_TIMEOUT) {
       set_error("a bounded device-side wait gave up (timeout)");
       return SHRK_ETIMEOUT;
@@ -264,6 +276,13 @@ static shrk_status check_error_word(Context* c, cudaStream_t s) {
 }
 
 shrk_status check_device_error(cudaStream_t s) { return check_error_word(t_cur, s); }
+
+// After a synchronisation of s in a host-pointer call: the error so far,
+// without another wait (other contexts are read by shrk_stream_check).
+shrk_status poll_device_error(cudaStream_t s) {
+  if (!t_cur->host || *(volatile int*)t_cur->err == DEV_ERR_NONE) return SHRK_OK;
+  return check_error_word(t_cur, s);
+}
 
 // ------------------------------------------------------------ timing --
 static std::atomic<int64_t> g_launches{0};
@@ -373,6 +392,54 @@ static shrk_status d2h(void* dst, const void* src, size_t bytes, cudaStream_t s)
   }
   return SHRK_OK;
 }
+
+// Uploads two arrays into adjacent device memory with one copy where the
+// stage has room; *dst2 (256-byte aligned) gets the second.
+static shrk_status h2d_pair(void* dst, const void* a, size_t na, const void* b, size_t nb,
+                            void** dst2, cudaStream_t s) {
+  const size_t pad = (na + 255) & ~(size_t)255;
+  *dst2 = (char*)dst + pad;
+  Context* c = t_cur;
+  size_t off = 0;
+  char* st = (c && c->host && s == c->stream) ? stage_take(c, pad + nb, &off) : nullptr;
+  if (!st) {
+    SHRK_TRY(h2d(dst, a, na, s));
+    return h2d(*dst2, b, nb, s);
+  }
+  std::memcpy(st, a, na);
+  std::memcpy(st + pad, b, nb);
+  SHRK_CUDA(cudaMemcpyAsync(dst, st, pad + nb, cudaMemcpyHostToDevice, s));
+  return SHRK_OK;
+}
+
+// Where the kernels of a host-pointer call write an output of `bytes` bytes:
+// small ones go straight to the pinned stage (each value is written once, by
+// the last kernel's epilogue, so the stores cross the bus as they come and no
+// copy follows), others to scratch.  take() gives the address, give() queues
+// what is left to do after the kernels; check_device_error completes both.
+struct HostOut {
+  static constexpr size_t kDirectMax = (size_t)256 << 10;
+  void* dev = nullptr;
+  void* dst = nullptr;
+  size_t bytes = 0;
+  bool direct = false;
+
+  shrk_status take(int slot, void* user, size_t n, cudaStream_t s) {
+    dst = user;
+    bytes = n;
+    Context* c = t_cur;
+    size_t off = 0;
+    char* st = n <= kDirectMax && c->host && s == c->stream ? stage_take(c, n, &off) : nullptr;
+    if (st) {
+      dev = st;
+      direct = true;
+      c->pending.push_back({user, off, n});
+      return SHRK_OK;
+    }
+    return scratch_get(slot, n, &dev);
+  }
+  shrk_status give(cudaStream_t s) { return direct ? SHRK_OK : d2h(dst, dev, bytes, s); }
+};
 
 // At the entry of a host-pointer call: settle what an earlier call that
 // returned early may have left in flight, and size the stage.
@@ -608,18 +675,18 @@ static shrk_status lw_device(const double* ev, size_t p, double c, int method, i
   if (std::isnan(eta)) eta = 0.4 / std::sqrt((double)p);  // mod.rs:150-153
   void* dev = nullptr;
   SHRK_TRY(scratch_get(3, sizeof(double) * p, &dev));
-  void* out = nullptr;
-  SHRK_TRY(scratch_get(4, sizeof(double) * p, &out));
+  HostOut out;
+  SHRK_TRY(out.take(4, xi, sizeof(double) * p, s));
   SHRK_TRY(h2d(dev, ev, sizeof(double) * p, s));
   set_source_hint((const double*)dev, ev, (int64_t)p);
   Epilogue epi;
   epi.mode = EPI_LW;
   epi.scale = 1.0 / (double)p;
   epi.c = c;
-  epi.out_re = (double*)out;
+  epi.out_re = (double*)out.dev;
   SHRK_TRY(sums_dispatch((const double*)dev, (int64_t)p, (const double*)dev, (int64_t)p, eta,
                          m, precision, NAN, epi, s, true));
-  SHRK_TRY(d2h(xi, out, sizeof(double) * p, s));
+  SHRK_TRY(out.give(s));
   return check_device_error(s);
 }
 
@@ -646,24 +713,21 @@ static shrk_status deconv_device(const double* ev, size_t p, double c, size_t n_
   const bool par = parallelism == SHRK_PAR_PARALLEL;
   int m = method;
   if (is_auto(m)) m = shrk_grid_appropriate(shrk_resolve_auto_method(m, par, p), p, n_points);
-  void* dev = nullptr;
-  SHRK_TRY(scratch_get(3, sizeof(double) * p, &dev));
-  void* dq = nullptr;
-  SHRK_TRY(scratch_get(6, sizeof(double) * n_points, &dq));
-  void* out = nullptr;
-  SHRK_TRY(scratch_get(4, sizeof(double) * 6 * n_points, &out));
-  SHRK_TRY(h2d(dev, ev, sizeof(double) * p, s));
+  void *dev = nullptr, *dq = nullptr;
+  SHRK_TRY(scratch_get(3, sizeof(double) * (p + n_points) + 256, &dev));
+  HostOut out;
+  SHRK_TRY(out.take(4, out7 + n_points, sizeof(double) * 6 * n_points, s));
+  SHRK_TRY(h2d_pair(dev, ev, sizeof(double) * p, grid, sizeof(double) * n_points, &dq, s));
   set_source_hint((const double*)dev, ev, (int64_t)p);
-  SHRK_TRY(h2d(dq, grid, sizeof(double) * n_points, s));
   Epilogue epi;
   epi.mode = EPI_MP;
   epi.scale = 1.0 / (double)p;
   epi.c = c;
   epi.eta = eta_val;
-  for (int i = 0; i < 6; ++i) epi.out[i] = (double*)out + i * n_points;
+  for (int i = 0; i < 6; ++i) epi.out[i] = (double*)out.dev + i * n_points;
   SHRK_TRY(sums_dispatch((const double*)dq, (int64_t)n_points, (const double*)dev, (int64_t)p,
                          eta_val, m, precision, cutoff, epi, s, false));
-  SHRK_TRY(d2h(out7 + n_points, out, sizeof(double) * 6 * n_points, s));
+  SHRK_TRY(out.give(s));
   return check_device_error(s);
 }
 
@@ -886,19 +950,20 @@ shrk_status shrk_stieltjes_all(const double* ev, size_t p, double eta, int metho
   int m = resolve(method, parallelism, p);
   void* dev = nullptr;
   SHRK_TRY(scratch_get(3, sizeof(double) * p, &dev));
-  void* out = nullptr;
-  SHRK_TRY(scratch_get(4, sizeof(double) * 2 * p, &out));
+  HostOut re, im;
+  SHRK_TRY(re.take(4, out_re, sizeof(double) * p, s));
+  SHRK_TRY(im.take(5, out_im, sizeof(double) * p, s));
   SHRK_TRY(h2d(dev, ev, sizeof(double) * p, s));
   set_source_hint((const double*)dev, ev, (int64_t)p);
   Epilogue epi;
   epi.mode = EPI_SUMS;
   epi.scale = 1.0 / (double)p;
-  epi.out_re = (double*)out;
-  epi.out_im = (double*)out + p;
+  epi.out_re = (double*)re.dev;
+  epi.out_im = (double*)im.dev;
   SHRK_TRY(sums_dispatch((const double*)dev, (int64_t)p, (const double*)dev, (int64_t)p, eta,
                          m, precision, cutoff, epi, s, true));
-  SHRK_TRY(d2h(out_re, out, sizeof(double) * p, s));
-  SHRK_TRY(d2h(out_im, (double*)out + p, sizeof(double) * p, s));
+  SHRK_TRY(re.give(s));
+  SHRK_TRY(im.give(s));
   return check_device_error(s);
 }
 
@@ -969,24 +1034,22 @@ shrk_status shrk_stieltjes_at_points(const double* q, size_t nq, const double* e
   const bool par = parallelism == SHRK_PAR_PARALLEL;
   int m = method;
   if (is_auto(m)) m = shrk_grid_appropriate(shrk_resolve_auto_method(m, par, p), p, nq);
-  void* dev = nullptr;
-  SHRK_TRY(scratch_get(3, sizeof(double) * p, &dev));
-  void* dq = nullptr;
-  SHRK_TRY(scratch_get(6, sizeof(double) * nq, &dq));
-  void* out = nullptr;
-  SHRK_TRY(scratch_get(4, sizeof(double) * 2 * nq, &out));
-  SHRK_TRY(h2d(dev, ev, sizeof(double) * p, s));
+  void *dev = nullptr, *dq = nullptr;
+  SHRK_TRY(scratch_get(3, sizeof(double) * (p + nq) + 256, &dev));
+  HostOut re, im;
+  SHRK_TRY(re.take(4, raw_re, sizeof(double) * nq, s));
+  SHRK_TRY(im.take(5, raw_im, sizeof(double) * nq, s));
+  SHRK_TRY(h2d_pair(dev, ev, sizeof(double) * p, q, sizeof(double) * nq, &dq, s));
   set_source_hint((const double*)dev, ev, (int64_t)p);
-  SHRK_TRY(h2d(dq, q, sizeof(double) * nq, s));
   Epilogue epi;
   epi.mode = EPI_SUMS;
   epi.scale = 1.0;
-  epi.out_re = (double*)out;
-  epi.out_im = (double*)out + nq;
+  epi.out_re = (double*)re.dev;
+  epi.out_im = (double*)im.dev;
   SHRK_TRY(sums_dispatch((const double*)dq, (int64_t)nq, (const double*)dev, (int64_t)p, eta,
                          m, precision, cutoff, epi, s, false));
-  SHRK_TRY(d2h(raw_re, out, sizeof(double) * nq, s));
-  SHRK_TRY(d2h(raw_im, (double*)out + nq, sizeof(double) * nq, s));
+  SHRK_TRY(re.give(s));
+  SHRK_TRY(im.give(s));
   return check_device_error(s);
 }
 

@@ -1749,10 +1749,8 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   SHRK_CUDA(cudaMemcpyAsync(hd.data(), d, sizeof(double) * p, cudaMemcpyDeviceToHost, s));
   if (p > 1)
     SHRK_CUDA(cudaMemcpyAsync(he.data(), e, sizeof(double) * (p - 1), cudaMemcpyDeviceToHost, s));
-  int timed_out = 0;
-  SHRK_CUDA(cudaMemcpyAsync(&timed_out, device_error_word(), sizeof(int), cudaMemcpyDeviceToHost, s));
   SHRK_CUDA(cudaStreamSynchronize(s));
-  if (timed_out) return check_device_error(s);
+  SHRK_TRY(poll_device_error(s));  // a wait of the reduction gave up
   const double eps = 2.220446049250313e-16;
   double tnorm = 0.0;
   for (int64_t i = 0; i < p; ++i) {
