@@ -644,9 +644,9 @@ def run_path(args, world, rank, local):
             roof = {"bound": "hbm", "achieved": ach, "peak": _measured_hbm(), "unit": "GB/s",
                     "frac": ach / _measured_hbm(), "traffic": tr, "kernel": "nufft_splat",
                     "kernel_ms": k_s * 1e3, "grid_cells": m,
-                    "basis": "splat family (keys + short-run sums, long-run sums, pack: three "
-                             "launches) per step: " + basis + "; traffic = DRAM bytes of those "
-                             "launches per step (ncu at p = 2^24, scaled by the source count)",
+                    "basis": "splat family (splat and pack, two launches) per step: " + basis +
+                             "; traffic = DRAM bytes of those launches per step "
+                             "(ncu at p = 2^24, scaled by the source count)",
                     "families_ms": {k_: v[1] / max(1, args.steps) for k_, v in fams.items()},
                     "call_algorithmic_bytes": total_alg,
                     "call_gbs": total_alg / (ms * 1e-3) / 1e9}
@@ -654,7 +654,7 @@ def run_path(args, world, rank, local):
             m = O.fft5_grid_size(ev_h, eta)
             fam = family.decode()
             alg_step, basis = {
-                "fft5_splat": (8 * p + 16 * m, "splat (cell, key, run-sum and pack launches): 8 B per "
+                "fft5_splat": (8 * p + 16 * m, "splat and pack launches: 8 B per "
                                "source read + 16 B per grid cell written, per step"),
                 "fft5_fft": (128 * m, "two transforms of two four-step passes: 16 B per cell "
                              "read + 16 B written per pass, per step"),

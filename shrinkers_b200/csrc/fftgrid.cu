@@ -10,12 +10,10 @@
 // Pipeline (all FP64), stencil width N = 2/4/6/8 a template parameter:
 //
 //   1. runs         a source's stencil cell is i0 = floor((v-lo)/dx); the
-//                   sources are sorted, so the cells are too, and one thread
-//                   per cell key bisects for first[key] = the first source
-//                   with cell >= key (on an integer cell array for large
-//                   grids); each run of equal cells gets the sums of its N
-//                   stencil weights, from the key's thread, a warp or CTAs
-//                   by the run's length.
+//                   sources are sorted, so the cells are too: one thread per
+//                   source finds its cell and its N Lagrange weights, the
+//                   sources at which the cell changes mark the runs of equal
+//                   cells, and each run gets the sums of its weights.
 //   2. pack         one thread per grid cell adds the weights of its sources
 //                   (at most 32) run by run in ascending source order -- the
 //                   order of the reference's sequential splat, so these
@@ -24,24 +22,24 @@
 //                   t = pos - i0 are recomputed where they are added
 //                   (sources come from L2; no weight array).
 //                   packed[c] = density[c] + i x_c/(x_c^2 + eta^2).
-//   4. fft          four-step FFT m = m1*m2 (m1, m2 <= 2048): column FFTs of
-//                   length m1 in shared memory with the inter-pass twiddle,
-//                   then row FFTs of length m2.  Twiddles and the analytic
-//                   even-kernel spectrum are device tables cached per grid.
-//   5. spectral     unpack the two real spectra (conjugate symmetry), form
-//                   Im_hat + i Re_hat = D*K_even + i D*K_odd.
-//   6. fft          inverse transform.
-//   7. interp       N-point interpolation at the query points, 1/m scale,
+//   3. fft          four-step FFT m = m1*m2 (m1, m2 <= 2048): column FFTs of
+//                   length m1 with the inter-pass twiddle, then row FFTs of
+//                   length m2, in registers with exchanges through shared
+//                   memory.  Twiddles and the analytic even-kernel spectrum
+//                   are device tables cached per grid.
+//   4. fft          inverse transform, whose column pass forms the spectral
+//                   product on the way in: unpack the two real spectra
+//                   (conjugate symmetry), Im_hat + i Re_hat = D*K_even +
+//                   i D*K_odd.
+//   5. interp       N-point interpolation at the query points, 1/m scale,
 //                   fused FP64 epilogue.
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "internal.h"
 
 #include <algorithm>
-#include <atomic>
+#include <climits>
 #include <cmath>
-#include <cstdlib>
-#include <map>
 #include <string>
 
 namespace shrk {
@@ -74,6 +72,17 @@ size_t sat_usize(double v) {
   return (size_t)v;
 }
 
+// x / den for a constant integer |den| < 2^13, correctly rounded without a
+// division: q = x rc (rc the rounded reciprocal) is within 1.5 ulp and one
+// residual step leaves q + r rc within 1.5 2^-53 ulp of x / den, while a
+// quotient by den that is not itself a midpoint is at least ulp / (2 |den|)
+// from the nearest one.  (The stencil divides by N constants a source and a
+// query; the divisions were two thirds of the weights' time.)
+__device__ __forceinline__ double div_const(double x, double den, double rc) {
+  const double q = x * rc;
+  return fma(fma(-q, den, x), rc, q);
+}
+
 // fft5.rs:136-164 lagrange_weights<N>, operation order preserved.
 template <int N>
 __device__ __forceinline__ void lagrange(double t, double w[N]) {
@@ -96,16 +105,39 @@ __device__ __forceinline__ void lagrange(double t, double w[N]) {
 #pragma unroll
     for (int l = 0; l < N; ++l)
       if (l != j) den *= (double)(j - l);
-    w[j] = pref[j] * suf[j] / den;
+    w[j] = div_const(pref[j] * suf[j], den, 1.0 / den);
   }
+}
+
+// A grid's spacing with its rounded reciprocal (0 outside the range in which
+// the quotients below are exact, so that they take the division).
+struct Spacing {
+  double dx, rdx;
+};
+
+Spacing spacing(double dx) {
+  const double ax = std::fabs(dx);
+  return {dx, ax > 1e-100 && ax < 1e100 ? 1.0 / dx : 0.0};
+}
+
+// a / dx, correctly rounded: two residual steps on a rdx (Markstein: a
+// faithful quotient corrected once with the rounded reciprocal is the rounded
+// quotient); anything outside the plain range, NaN included, divides.
+__device__ __forceinline__ double grid_pos(double a, const Spacing& h) {
+  double q = a * h.rdx;
+  const double aq = fabs(q);
+  if (!(aq > 1e-100 && aq < 1e100)) return a / h.dx;
+  q = fma(fma(-q, h.dx, a), h.rdx, q);
+  return fma(fma(-q, h.dx, a), h.rdx, q);
 }
 
 // floor((v - lo)/dx) as a cell index clamped to [-N - 1, m + N] (every slot
 // of a source beyond that range lands on the same edge cell), and the
 // fraction t = pos - floor(pos) of the unclamped position.
 template <int N>
-__device__ __forceinline__ int64_t cell_of(double v, double lo, double dx, int64_t m, double* t) {
-  const double pos = (v - lo) / dx;
+__device__ __forceinline__ int64_t cell_of(double v, double lo, const Spacing& h, int64_t m,
+                                           double* t) {
+  const double pos = grid_pos(v - lo, h);
   const double fl = floor(pos);
   *t = pos - fl;
   const double c = fmin(fmax(fl, -(double)N - 1.0), (double)(m + N));
@@ -116,257 +148,149 @@ struct GridArgs {
   const double* src;  // ascending
   int64_t ns;
   int rev;            // 1: visit the sources in descending order (dx < 0)
-  double lo, dx, eta;
+  double lo;
+  Spacing h;
+  double eta;
   int64_t m;
   double2* packed;
   double* dens;       // non-null: write the density alone (the splat stage)
 };
 
+__device__ __forceinline__ double visited(const GridArgs& a, int64_t j) {
+  return a.rev ? a.src[a.ns - 1 - j] : a.src[j];
+}
+
 template <int N>
-__device__ __forceinline__ int clamped_cell(const GridArgs& a, int64_t j, double* t) {
-  const double v = a.rev ? a.src[a.ns - 1 - j] : a.src[j];
-  const int64_t i0 = cell_of<N>(v, a.lo, a.dx, a.m, t);
+__device__ __forceinline__ int clamped_cell(const GridArgs& a, double v, double* t) {
+  const int64_t i0 = cell_of<N>(v, a.lo, a.h, a.m, t);
   return (int)(i0 < -N ? -N : (i0 > a.m + N ? a.m + N : i0));
 }
 
-// Stencil weight k of visited source j (fft5.rs:136-164, 175-185): the same
-// arithmetic as the k-th entry of lagrange<N>, recomputed where it is summed
-// (k is a compile-time constant at every call, so only that weight's
-// operations remain).  Sources are read through L2; no weight array.
-template <int N, int K>
-__device__ __forceinline__ double weight_of(const GridArgs& a, int64_t j) {
-  double t;
-  (void)clamped_cell<N>(a, j, &t);
-  double w[N];
-  lagrange<N>(t, w);
-  return w[K];
-}
+constexpr int DENSE_MIN = 32;  // cells with more sources take their density from run sums
 
-// first[key + N + 1] for every key in [-N - 1, m + N + 1]: the number of
-// visited sources whose clamped stencil cell is below key.  Visiting order
-// makes the cells non-decreasing, so this is a lower bound found by
-// bisection (the same cell computation as everywhere else, so the same runs).
-// With `cells` (the clamped cell of every visited source, cells_kernel) the
-// probes compare integers instead of each dividing, and start on `coarse`
-// (every COARSE-th entry of cells, small enough to stay in L1): the first
-// coarse entry at least key brackets the answer within COARSE sources.
-constexpr int COARSE = 64;
+// The runs of equal stencil cells and their weight sums.  run[cell + N + 1] =
+// the visited sources [x, y) of that cell, {0, 0} for an empty one (zero on
+// entry).  The sources are cut in chunks of SPLAT_CHUNK, a CTA each: a run
+// inside one chunk has its sums in sum[(cell + N + 1) N + k]; one that spans
+// chunks has tail[] of the chunk it starts in plus head[] of the later ones,
+// in that order.
+struct Runs {
+  int2* run;
+  double* sum;
+  double* head;  // [chunks][N]
+  double* tail;
+};
 
+constexpr int SPLAT_CHUNK = 512;
+constexpr int SPLAT_NT = 256;
+constexpr int SPLAT_LONG = 32;  // longer pieces of a run are summed by a warp
+
+// One chunk of sources: each source's cell and weights once, by a thread each
+// (coalesced), into shared memory; the places where the cell changes cut the
+// chunk in pieces; each piece's N sums in source order by a thread each, or by
+// a warp for a long piece (lanes strided, a fixed butterfly).  Work follows
+// the sources, whatever their spread: a thread per cell that bisected for its
+// run's start spent 51 us on the 2^20 cells of 200 003 sources (mostly empty
+// ones), and a warp a run 14 us more on runs of ten sources; this takes 8, and
+// 14 us for 10^6 sources on 65 536 cells, where those took 41.  FP64-bound:
+// about 60 operations a source at N = 4, 90 at N = 8.
 template <int N>
-__device__ __forceinline__ int64_t lower_key(const GridArgs& a, const int* __restrict__ cells,
-                                             const int* __restrict__ coarse, int key, int64_t lo,
-                                             int64_t hi) {
-  if (cells) {
-    int64_t blo = 0, bhi = (a.ns + COARSE - 1) / COARSE;
-    while (blo < bhi) {
-      const int64_t mid = (blo + bhi) >> 1;
-      if (__ldg(coarse + mid) < key) blo = mid + 1;
-      else bhi = mid;
+__global__ void __launch_bounds__(SPLAT_NT) splat_kernel(const GridArgs a, const Runs R) {
+  constexpr int W = SPLAT_CHUNK + 1;
+  constexpr int PER = SPLAT_CHUNK / SPLAT_NT;
+  extern __shared__ double wsm[];       // [N][W]
+  __shared__ int cell_sh[SPLAT_CHUNK + 2];  // of the sources j0 - 1 .. j0 + SPLAT_CHUNK
+  __shared__ int start[SPLAT_CHUNK + 1];    // pieces, in source order
+  __shared__ int longs[SPLAT_CHUNK / SPLAT_LONG];
+  __shared__ int base[PER * SPLAT_NT / 32 + 1];
+  __shared__ int n_long;
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+  const int64_t j0 = (int64_t)blockIdx.x * SPLAT_CHUNK;
+  const int n = (int)(a.ns - j0 < SPLAT_CHUNK ? a.ns - j0 : SPLAT_CHUNK);
+  if (tid == 0) n_long = 0;
+#pragma unroll
+  for (int it = 0; it < PER; ++it) {
+    const int i = tid + it * SPLAT_NT;
+    if (i < n) {
+      double t, w[N];
+      cell_sh[i + 1] = clamped_cell<N>(a, visited(a, j0 + i), &t);
+      lagrange<N>(t, w);
+#pragma unroll
+      for (int k = 0; k < N; ++k) wsm[k * W + i] = w[k];
     }
-    // cells[COARSE (blo - 1)] < key <= cells[COARSE blo] (or blo = the end)
-    if (blo == 0) return 0;
-    lo = COARSE * (blo - 1) + 1;
-    hi = COARSE * blo < a.ns ? COARSE * blo : a.ns;
   }
-  while (lo < hi) {
-    const int64_t mid = (lo + hi) >> 1;
+  if (tid == 0 || tid == 32) {  // the neighbours; INT_MIN is no cell
+    const int64_t j = tid ? j0 + n : j0 - 1;
     double t;
-    const int c = cells ? __ldg(cells + mid) : clamped_cell<N>(a, mid, &t);
-    if (c < key) lo = mid + 1;
-    else hi = mid;
+    cell_sh[tid ? n + 1 : 0] = j >= 0 && j < a.ns ? clamped_cell<N>(a, visited(a, j), &t) : INT_MIN;
   }
-  return lo;
-}
-
-// cells[j] = the clamped stencil cell of visited source j: one division per
-// source, for grids with many keys, whose searches would otherwise divide at
-// every probe.
-template <int N>
-__global__ void cells_kernel(const GridArgs a, int* __restrict__ cells, int* __restrict__ coarse) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < a.ns; j += stride) {
-    double t;
-    const int c = clamped_cell<N>(a, j, &t);
-    cells[j] = c;
-    if (j % COARSE == 0) coarse[j / COARSE] = c;
-  }
-}
-
-constexpr int DENSE_MIN = 32;   // cells with more sources take their density from run sums
-constexpr int RUN_CHUNK = 4096; // long runs are summed in chunks of this many sources, a CTA each
-
-// Run lengths that decide who sums a run: at most `thread_max` sources, the
-// key's own thread; up to `warp_max`, a warp; longer runs, CTAs in chunks of
-// RUN_CHUNK.  Each run's sum depends only on its length, so it is the same
-// from call to call.
-struct RunSplit {
-  int thread_max;
-  int warp_max;
-};
-
-// The long runs and their chunks (keys_kernel fills them, long_runs_kernel
-// sums them): run r is key idx[r] with nch[r] chunks from the chunk list's
-// base[r]; cnt[r] counts its finished chunks; partial[g][k] holds chunk g's
-// sums; widx[] lists the keys of the warp-summed runs.  counters[0] / [1] /
-// [2] = runs / chunks / warp runs listed (zero on entry).
-struct LongRuns {
-  int* idx;
-  int* base;
-  int* nch;
-  int* cnt;
-  int* chunk_run;  // chunk g -> its run r
-  int* widx;
-  int* counters;
-  double* partial;
-};
-
-// Keys and run sums.  A CTA of KEYS_CTA threads serves KEYS_CTA - 1
-// consecutive keys: each thread finds first[] of its key, and the end of a
-// key's run, first[] of the next key, comes from the next thread through
-// shared memory (the last thread of a CTA searches only for that, the next
-// CTA's first key), so every thread makes one search.  Then
-// S[(e + N + 1) N + k], the sum of stencil weight k over the run, computing
-// each source's N weights once in ascending source order -- or, for a longer
-// run (RunSplit), lists it for long_runs_kernel: as a warp run, or with its
-// chunks of RUN_CHUNK sources.
-constexpr int KEYS_CTA = 256;
-
-template <int N>
-__global__ void __launch_bounds__(KEYS_CTA) keys_kernel(const GridArgs a, int* __restrict__ first,
-                                                        int64_t n_keys, double* __restrict__ S,
-                                                        LongRuns L, const int* __restrict__ cells,
-                                                        const int* __restrict__ coarse,
-                                                        RunSplit rs) {
-  __shared__ int first_sh[KEYS_CTA];
-  const int64_t idx = (int64_t)blockIdx.x * (KEYS_CTA - 1) + threadIdx.x;
-  const int key = (int)(idx - N - 1);
-  int64_t j0 = a.ns;
-  if (idx <= n_keys) j0 = lower_key<N>(a, cells, coarse, key, 0, a.ns);
-  first_sh[threadIdx.x] = (int)j0;
   __syncthreads();
-  if (idx > n_keys || threadIdx.x == KEYS_CTA - 1) return;
-  first[idx] = (int)j0;
-  if (idx == n_keys) return;  // the closing entry (= ns)
-  // end of the run: the first source whose cell is at least key + 1 (the
-  // next thread's key; idx < n_keys, so that thread searched)
-  const int64_t j1 = first_sh[threadIdx.x + 1];
-  double t;
-  if (j1 - j0 > rs.thread_max && j1 - j0 <= rs.warp_max) {
-    L.widx[atomicAdd(L.counters + 2, 1)] = (int)idx;
-    return;
+  // pieces: a source whose cell differs from the one before it, and source 0
+  unsigned flags[PER];
+#pragma unroll
+  for (int it = 0; it < PER; ++it) {
+    const int i = tid + it * SPLAT_NT;
+    const bool f = i < n && (i == 0 || cell_sh[i + 1] != cell_sh[i]);
+    flags[it] = __ballot_sync(0xffffffffu, f);
+    if (lane == 0) base[it * (SPLAT_NT / 32) + wib + 1] = __popc(flags[it]);
   }
-  if (j1 - j0 > rs.thread_max) {
-    const int nch = (int)((j1 - j0 + RUN_CHUNK - 1) / RUN_CHUNK);
-    const int r = atomicAdd(L.counters, 1);
-    const int base = atomicAdd(L.counters + 1, nch);
-    L.idx[r] = (int)idx;
-    L.base[r] = base;
-    L.nch[r] = nch;
-    L.cnt[r] = 0;
-    for (int c = 0; c < nch; ++c) L.chunk_run[base + c] = r;
-    return;
+  if (tid == 0) base[0] = 0;
+  __syncthreads();
+  if (wib == 0) {  // inclusive scan of the PER * SPLAT_NT / 32 <= 32 counts
+    constexpr int NB = PER * SPLAT_NT / 32;
+    static_assert(NB <= 32, "one warp scans the counts");
+    int v = lane < NB ? base[lane + 1] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane < NB) base[lane + 1] = v;
   }
-  double acc[N];
+  __syncthreads();
+  const int pieces = base[PER * SPLAT_NT / 32];
 #pragma unroll
-  for (int k = 0; k < N; ++k) acc[k] = 0.0;
-  for (int64_t j = j0; j < j1; ++j) {
-    double w[N];
-    (void)clamped_cell<N>(a, j, &t);
-    lagrange<N>(t, w);
-#pragma unroll
-    for (int k = 0; k < N; ++k) acc[k] += w[k];
-  }
-#pragma unroll
-  for (int k = 0; k < N; ++k) S[idx * N + k] = acc[k];
-}
-
-// Run sums of the longer runs.  Runs listed with chunks: a CTA per chunk of
-// RUN_CHUNK sources (threads stride the chunk, partials added in a fixed
-// order); a run of one chunk writes its sums directly, otherwise the CTA that
-// finishes a run's last chunk (a ticket taken after a fence) adds the run's
-// chunk partials in chunk order.  Then the warp runs, a warp each.  The
-// lists' order varies from call to call; each run's sum does not.
-template <int N>
-__global__ void __launch_bounds__(256) long_runs_kernel(const GridArgs a,
-                                                        const int* __restrict__ first,
-                                                        const LongRuns L,
-                                                        double* __restrict__ S) {
-  __shared__ double red[8][N];
-  __shared__ int last;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int n_chunks = L.counters[1];
-  for (int g = blockIdx.x; g < n_chunks; g += gridDim.x) {
-    const int r = L.chunk_run[g];
-    const int64_t idx = L.idx[r];
-    const int nch = L.nch[r], c = g - L.base[r];
-    const int64_t r0 = first[idx], r1 = first[idx + 1];
-    const int64_t j0 = r0 + (int64_t)c * RUN_CHUNK;
-    const int64_t j1 = j0 + RUN_CHUNK < r1 ? j0 + RUN_CHUNK : r1;
-    double acc[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) acc[k] = 0.0;
-    for (int64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-      double t, w[N];
-      (void)clamped_cell<N>(a, j, &t);
-      lagrange<N>(t, w);
-#pragma unroll
-      for (int k = 0; k < N; ++k) acc[k] += w[k];
-    }
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) red[wib][k] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < N) {
-      double tt = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tt += red[w][threadIdx.x];
-      if (nch == 1) S[idx * N + threadIdx.x] = tt;
-      else L.partial[(int64_t)g * N + threadIdx.x] = tt;
-    }
-    if (nch > 1) {
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        __threadfence();  // this chunk's partials before its ticket
-        last = atomicAdd(L.cnt + r, 1) == nch - 1;
-      }
-      __syncthreads();
-      if (last && threadIdx.x < N) {
-        __threadfence();
-        const int b0 = L.base[r];
-        double tt = 0.0;
-        for (int q = 0; q < nch; ++q) tt += __ldcg(L.partial + (int64_t)(b0 + q) * N + threadIdx.x);
-        S[idx * N + threadIdx.x] = tt;
+  for (int it = 0; it < PER; ++it) {
+    const int i = tid + it * SPLAT_NT;
+    if ((flags[it] >> lane) & 1u) {
+      start[base[it * (SPLAT_NT / 32) + wib] + __popc(flags[it] & ((1u << lane) - 1u))] = i;
+      // the run's ends, each written once
+      const int c = cell_sh[i + 1], before = cell_sh[i];
+      if (c != before) {
+        R.run[c + N + 1].x = (int)(j0 + i);
+        if (before != INT_MIN) R.run[before + N + 1].y = (int)(j0 + i);
       }
     }
-    __syncthreads();
   }
-  // Warp runs: a warp per run, lanes striding it, the lanes' partials added
-  // by a fixed butterfly.
-  const int n_warp_runs = L.counters[2];
-  const int warps = (int)(blockDim.x >> 5);
-  for (int r = blockIdx.x * warps + wib; r < n_warp_runs; r += gridDim.x * warps) {
-    const int64_t idx = L.widx[r];
-    const int64_t j1 = first[idx + 1];
-    double acc[N];
-#pragma unroll
-    for (int k = 0; k < N; ++k) acc[k] = 0.0;
-    for (int64_t j = first[idx] + lane; j < j1; j += 32) {
-      double t, w[N];
-      (void)clamped_cell<N>(a, j, &t);
-      lagrange<N>(t, w);
-#pragma unroll
-      for (int k = 0; k < N; ++k) acc[k] += w[k];
+  if (tid == 0) {
+    start[pieces] = n;
+    if (j0 + n == a.ns) R.run[cell_sh[n] + N + 1].y = (int)a.ns;
+  }
+  __syncthreads();
+  const auto out = [&](int p, int p0, int p1) -> double* {
+    const int c = cell_sh[p0 + 1];
+    if (p == 0 && cell_sh[0] == c) return R.head + (int64_t)blockIdx.x * N;
+    if (p1 == n && cell_sh[n + 1] == c) return R.tail + (int64_t)blockIdx.x * N;
+    return R.sum + (int64_t)(c + N + 1) * N;
+  };
+  for (int u = tid; u < pieces * N; u += SPLAT_NT) {
+    const int p = u / N, k = u % N, p0 = start[p], p1 = start[p + 1];
+    if (p1 - p0 > SPLAT_LONG) {
+      if (k == 0) longs[atomicAdd(&n_long, 1)] = p;
+      continue;
     }
+    double s = 0.0;
+    for (int i = p0; i < p1; ++i) s += wsm[k * W + i];
+    out(p, p0, p1)[k] = s;
+  }
+  __syncthreads();
+  for (int u = wib; u < n_long * N; u += SPLAT_NT / 32) {
+    const int p = longs[u / N], k = u % N, p0 = start[p], p1 = start[p + 1];
+    double s = 0.0;
+    for (int i = p0 + lane; i < p1; i += 32) s += wsm[k * W + i];
 #pragma unroll
-    for (int k = 0; k < N; ++k) {
-      double v = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == k) S[idx * N + k] = v;
-    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out(p, p0, p1)[k] = s;
   }
 }
 
@@ -378,91 +302,170 @@ __global__ void __launch_bounds__(256) long_runs_kernel(const GridArgs a,
 // a denser cell adds the N run sums in that run order (deterministic, not the
 // sequential order).  The two edge cells also collect every clamped slot.
 // packed[c] = density[c] + i x_c/(x_c^2 + eta^2) (fft5.rs:364-376).
-__device__ __forceinline__ void pack_cell(const GridArgs& a, int64_t c, double dens) {
-  if (a.dens) {
-    a.dens[c] = dens;
-    return;
-  }
+// The odd kernel's sample x_c/(x_c^2 + eta^2).
+__device__ __forceinline__ double odd_kernel(const GridArgs& a, int64_t c) {
   const int64_t half = a.m / 2;
   const double sd = (c <= half) ? (double)c : (double)c - (double)a.m;
-  const double x = sd * a.dx;
-  const double denom = x * x + a.eta * a.eta;
-  a.packed[c] = make_double2(dens, x / denom);
+  const double x = sd * a.h.dx;
+  return x / (x * x + a.eta * a.eta);
 }
 
-// dens += weight K of every source of the run of cell c + N/2 - 1 - K, for
-// K = KK .. 0 in that order.
-template <int N, int KK>
-__device__ __forceinline__ void run_sums(const GridArgs& a, const int* first, int64_t c,
-                                         double& dens) {
-  if constexpr (KK >= 0) {
-    const int64_t e = c + N / 2 - 1 - KK;
-    for (int64_t j = first[e], j1 = first[e + 1]; j < j1; ++j) dens += weight_of<N, KK>(a, j);
-    run_sums<N, KK - 1>(a, first, c, dens);
-  }
-}
-
+// A cell's sources are one stretch [A, B) of the sorted sources.  The sparse
+// cells of a warp share theirs 32 sources at a time: a lane per source finds
+// its cell and weights into shared memory, then every lane adds its own cell's
+// in source order.  (Each lane walking its own sources was a serial chain of
+// up to 32 loads and stencils; a lot of 32 sources takes 2 700 clk, and the
+// kernel on 2^20 cells 14 us where it took 18.)
+// Most cells of a large grid are empty: a warp whose window has no run stores
+// its odd kernel and ends.
 template <int N>
-__global__ void __launch_bounds__(256) pack_kernel(const GridArgs a, const int* __restrict__ first_all,
-                                                   const double* __restrict__ S) {
+__global__ void __launch_bounds__(256, 6) pack_kernel(const GridArgs a, const Runs R) {
   constexpr int H = N / 2;
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int NP = N == 6 ? 8 : N;
+  __shared__ double wsm[8][32 * NP];
+  __shared__ int off_sh[8][32];
+  __shared__ int2 run_sh[8][32 + N];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, cw = c - lane;
   const int64_t m = a.m;
-  if (c >= m) return;
-  const int* first = first_all + N + 1;  // first[key] for key >= -N - 1
+  const int2* run = R.run + N + 1;  // run[cell] for -N - 1 <= cell <= m + N
+  // the warp's window: the runs of the cells cw - H .. cw + 31 + H
+  const int64_t e0 = cw - H + lane, e1 = e0 + 32;
+  const int2 w0 = e0 <= m + N ? __ldg(run + e0) : make_int2(0, 0);
+  const int2 w1 = lane < N && e1 <= m + N ? __ldg(run + e1) : make_int2(0, 0);
+  const double odd = a.dens || c >= m ? 0.0 : odd_kernel(a, c);
   double dens = 0.0;
-  if (c > 0 && c < m - 1) {
-    const int cnt = first[c + H] - first[c - H];
-    if (cnt > DENSE_MIN) {
+  const bool edge = cw == 0 || cw + 32 >= m;
+  if (edge || __any_sync(0xffffffffu, w0.y > w0.x || w1.y > w1.x)) {
+    run_sh[wib][lane] = w0;
+    if (lane < N) run_sh[wib][32 + lane] = w1;
+    __syncwarp();
+    const int2* r = run_sh[wib] + lane;  // r[i]: the run of cell c - H + i
+    unsigned A = UINT_MAX, B = 0;
+    if (c > 0 && c < m - 1) {
 #pragma unroll
-      for (int k = N - 1; k >= 0; --k) dens += S[(c + H - 1 - k + N + 1) * N + k];
-    } else {
-      run_sums<N, N - 1>(a, first, c, dens);
+      for (int i = 0; i < N; ++i)
+        if (r[i].y > r[i].x) {
+          A = min(A, (unsigned)r[i].x);
+          B = (unsigned)r[i].y;
+        }
     }
-  } else {
-    // edge cell: every slot whose clamped index lands here, sources then slots
-    const int64_t j0 = (c == 0) ? 0 : first[m - 1 - H];
-    const int64_t j1 = (c == 0) ? first[H] : a.ns;
-    for (int64_t j = j0; j < j1; ++j) {
-      double t;
-      const int i0 = clamped_cell<N>(a, j, &t);
-      double w[N];
-      lagrange<N>(t, w);
+    const bool any = B > A;
+    const bool sparse = any && B - A <= DENSE_MIN;
+    int64_t ahead = -1;
+    double v_ahead = 0.0;
+    for (unsigned pos = 0;;) {
+      unsigned next = sparse && B > pos ? max(A, pos) : UINT_MAX;
+      next = __reduce_min_sync(0xffffffffu, next);
+      if (next == UINT_MAX) break;
+      const int64_t j = (int64_t)next + lane;
+      const double v = ahead == j ? v_ahead : j < a.ns ? visited(a, j) : 0.0;
+      ahead = j + 32;  // mostly the next lot's
+      if (ahead < a.ns) v_ahead = visited(a, ahead);
+      if (j < a.ns) {
+        double t, w[N];
+        // the weight of cell c is entry off + 32 (c - cw), k = c + H - 1 - cell
+        off_sh[wib][lane] = lane + 32 * (int)(cw + H - 1 - clamped_cell<N>(a, v, &t));
+        lagrange<N>(t, w);
 #pragma unroll
-      for (int k = 0; k < N; ++k) {
-        int64_t cell = (int64_t)i0 - H + 1 + k;
-        cell = cell < 0 ? 0 : (cell > m - 1 ? m - 1 : cell);
-        if (cell == c) dens += w[k];
+        for (int k = 0; k < N; ++k) wsm[wib][k * 32 + lane] = w[k];
+      }
+      __syncwarp();
+      pos = next + 32;
+      if (sparse) {
+        const int i1 = (int)(min(B, pos) - next);
+#pragma unroll 8
+        for (int i = (int)(max(A, next) - next); i < i1; ++i)  // k < N; masked for cells
+          dens += wsm[wib][(off_sh[wib][i] + 32 * lane) & (32 * NP - 1)];  // out of order (NaN)
+      }
+      __syncwarp();
+    }
+    if (c > 0 && c < m - 1) {
+      if (any && !sparse) {
+        double s[N];  // the run's sum, or its tail: N loads in flight (9 000 clk one by one)
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const int k = N - 1 - i, c0 = r[i].x / SPLAT_CHUNK;
+          const double* at = R.sum + (c - H + i + N + 1) * N + k;
+          if (c0 < (r[i].y - 1) / SPLAT_CHUNK) at = R.tail + (int64_t)c0 * N + k;
+          s[i] = r[i].y > r[i].x ? __ldg(at) : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const int c1 = (r[i].y - 1) / SPLAT_CHUNK;
+          if (r[i].y > r[i].x)
+            for (int h = r[i].x / SPLAT_CHUNK + 1; h <= c1; ++h)
+              s[i] += R.head[(int64_t)h * N + N - 1 - i];
+          dens += s[i];
+        }
+      }
+    } else if (c < m) {
+      // edge cell: every slot whose clamped index lands here, sources then slots
+      int j0 = c == 0 ? 0 : (int)a.ns, j1 = c == 0 ? 0 : (int)a.ns;
+      if (c == 0)
+        for (int64_t e = -N; e < H; ++e) j1 = max(j1, run[e].y);
+      else
+        for (int64_t e = m - 1 - H; e <= m + N; ++e) {
+          const int2 r = run[e];
+          if (r.y > r.x) j0 = min(j0, r.x);
+        }
+      for (int j = j0; j < j1; ++j) {
+        double t;
+        const int i0 = clamped_cell<N>(a, visited(a, j), &t);
+        double w[N];
+        lagrange<N>(t, w);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          int64_t cell = (int64_t)i0 - H + 1 + k;
+          cell = cell < 0 ? 0 : (cell > m - 1 ? m - 1 : cell);
+          if (cell == c) dens += w[k];
+        }
       }
     }
   }
-  pack_cell(a, c, dens);
+  if (c >= m) return;
+  if (a.dens) a.dens[c] = dens;
+  else a.packed[c] = make_double2(dens, odd);
 }
 
 // The evaluation stage's input: packed[c] from a given density (the sum of
 // the splat stages of several source sets).
 __global__ void pack_density_kernel(const GridArgs a, const double* __restrict__ density) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < a.m) pack_cell(a, c, density[c]);
+  if (c < a.m) a.packed[c] = make_double2(density[c], odd_kernel(a, c));
 }
 
 // ---------------------------------------------------------------- FFT --
 // Unnormalised DFT, forward sign e^{-2 pi i jk/m}, inverse e^{+2 pi i jk/m}
 // (the contract of the reference's transform, rustfft).  m = m1*m2 by the
-// four-step method; each row transform of length L (8 <= L <= 2048) runs in
-// shared memory as a mixed-radix Stockham FFT (radix 8, then one radix-4 or
-// radix-2 stage): every thread owns 8 elements per stage, the stage twiddles
-// come from a per-CTA table, and rows are stored with one pad slot per 8
-// elements (and one more per row) so that strided accesses spread over the
-// shared-memory banks.
+// four-step method; each row transform of length L = 2^LOG (8 <= L <= 2048) is
+// a mixed-radix Stockham FFT (radix 8, then one radix-4 or radix-2 stage) by
+// L/8 threads of eight elements each.  Thread q loads the elements q + r L/8,
+// which are its first butterfly, and ends with the outputs q + r L/8, so the
+// first stage takes its inputs, and the last leaves its outputs, in registers;
+// only the exchanges between stages go through shared memory (one pad slot per
+// 8 elements).  A butterfly's twiddles are the powers of one table entry.  With
+// the loads, the stores and every twiddle staged in shared memory a pass over
+// 2^20 points took 36 (columns) and 21 us (rows), now 18 and 12 (16 + 16 MB
+// each way through L2); bound by the latency of a CTA's chain of load, four
+// butterflies with three exchanges, and store, 4 CTAs an SM overlapping.
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+// The transform's products, fused (two operations fewer, one rounding less).
+__device__ __forceinline__ double2 cmulf(double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
 }
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) {
   return make_double2(a.x + b.x, a.y + b.y);
 }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) {
   return make_double2(a.x - b.x, a.y - b.y);
+}
+// v e^{i pi/4 sign}
+__device__ __forceinline__ double2 mul_w8(double2 v, double sign) {
+  const double h = 0.70710678118654752440;  // sqrt(1/2)
+  return make_double2(h * (v.x - sign * v.y), h * (v.y + sign * v.x));
 }
 // v * (sign * i)
 __device__ __forceinline__ double2 mul_si(double2 v, double sign) {
@@ -471,11 +474,6 @@ __device__ __forceinline__ double2 mul_si(double2 v, double sign) {
 __device__ __forceinline__ int padi(int i) { return i + (i >> 3); }
 
 // R-point DFTs in registers, W_R = e^{sign 2 pi i/R}.
-__device__ __forceinline__ void dft2(double2* v) {
-  const double2 a = v[0], b = v[1];
-  v[0] = cadd(a, b);
-  v[1] = csub(a, b);
-}
 __device__ __forceinline__ void dft4(double2& v0, double2& v1, double2& v2, double2& v3,
                                      double sign) {
   const double2 t0 = cadd(v0, v2), t1 = csub(v0, v2), t2 = cadd(v1, v3);
@@ -486,14 +484,13 @@ __device__ __forceinline__ void dft4(double2& v0, double2& v1, double2& v2, doub
   v3 = csub(t1, t3);
 }
 __device__ __forceinline__ void dft8(double2* v, double sign) {
-  const double h = 0.70710678118654752440;  // sqrt(1/2)
   double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
   double2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
   dft4(e0, e1, e2, e3, sign);
   dft4(o0, o1, o2, o3, sign);
-  o1 = cmul(o1, make_double2(h, sign * h));
+  o1 = mul_w8(o1, sign);
   o2 = mul_si(o2, sign);
-  o3 = cmul(o3, make_double2(-h, sign * h));
+  o3 = mul_si(mul_w8(o3, sign), sign);
   v[0] = cadd(e0, o0);
   v[1] = cadd(e1, o1);
   v[2] = cadd(e2, o2);
@@ -504,167 +501,172 @@ __device__ __forceinline__ void dft8(double2* v, double sign) {
   v[7] = csub(e3, o3);
 }
 
-// One radix-R Stockham stage over a row of length L (sub-transform length Ns
-// so far): thread q of the row does the 8/R butterflies j = q + b*L/8.
-template <int R>
-__device__ __forceinline__ void fft_stage(double2* row, const double2* tws, int L, int Ns, int q,
-                                          double sign) {
-  // tws: this stage's twiddles W_{Ns R}^{k r} at [(r - 1) * Ns + k]
-  constexpr int B = 8 / R;
-  const int tpr = L >> 3;
-  double2 v[8];
-#pragma unroll
-  for (int b = 0; b < B; ++b) {
-    const int j = q + b * tpr;
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[b * R + r] = row[padi(j + r * (L / R))];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int b = 0; b < B; ++b) {
-    const int j = q + b * tpr;
-    const int k = j & (Ns - 1);
-    if (Ns > 1) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[b * R + r] = cmul(v[b * R + r], tws[(r - 1) * Ns + k]);
-    }
-    if (R == 8) dft8(&v[b * R], sign);
-    else if (R == 4) dft4(v[b * R], v[b * R + 1], v[b * R + 2], v[b * R + 3], sign);
-    else dft2(&v[b * R]);
-    const int base = (j - k) * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) row[padi(base + r * Ns)] = v[b * R + r];
-  }
-  __syncthreads();
+// v[r] *= w^r, r = 1..7, the powers at most three products deep.
+__device__ __forceinline__ void twist8(double2* v, double2 w) {
+  const double2 w2 = cmulf(w, w), w4 = cmulf(w2, w2), w3 = cmulf(w, w2);
+  v[1] = cmulf(v[1], w);
+  v[2] = cmulf(v[2], w2);
+  v[3] = cmulf(v[3], w3);
+  v[4] = cmulf(v[4], w4);
+  v[5] = cmulf(v[5], cmulf(w4, w));
+  v[6] = cmulf(v[6], cmulf(w4, w2));
+  v[7] = cmulf(v[7], cmulf(w4, w3));
 }
 
-// In-place FFT of a padded row of length L >= 8; every thread of the CTA
-// calls it (the stages hold barriers).
-__device__ void row_fft(double2* row, const double2* tws, int L, int q, double sign) {
-  int Ns = 1, rem = L, off = 0;
-  while (rem >= 8) {
-    fft_stage<8>(row, tws + off, L, Ns, q, sign);
-    if (Ns > 1) off += 7 * Ns;
-    Ns *= 8;
-    rem >>= 3;
-  }
-  if (rem == 4) fft_stage<4>(row, tws + off, L, Ns, q, sign);
-  else if (rem == 2) fft_stage<2>(row, tws + off, L, Ns, q, sign);
+// Stage s >= 1 of a row transform combines Ns = 8^s points; its table holds
+// W_{Ns R}^k, k < Ns, from entry stage_off(s) (8 + 64 + 512 entries at most).
+constexpr int STAGE_TAB = 584;
+__host__ __device__ constexpr int stage_off(int s) { return s <= 1 ? 0 : s == 2 ? 8 : 72; }
+
+__global__ void stage_twiddle_kernel(double2* __restrict__ out, const double2* __restrict__ tw,
+                                     int L, int64_t m) {
+  const int idx = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int s = idx < 8 ? 1 : idx < 72 ? 2 : 3, Ns = 1 << (3 * s);
+  if (idx >= STAGE_TAB || Ns >= L) return;
+  const int R = L / Ns < 8 ? L / Ns : 8;
+  out[idx] = tw[(int64_t)(idx - stage_off(s)) * (m / ((int64_t)Ns * R))];
 }
 
-// Per-stage twiddles for row_fft: for every stage after the first (Ns > 1,
-// radix R), W_{Ns R}^{k r} = W_m^{k r m/(Ns R)} for r = 1..R-1, k < Ns, laid
-// out [r - 1][k] so that consecutive lanes read consecutive entries; L - 8
-// entries in all.  Taken from the length-m table, sign applied.
-__device__ __forceinline__ void load_stage_twiddles(double2* tws, const double2* __restrict__ tw,
-                                                    int L, int64_t m, double sign) {
-  const int total = L - 8;  // <= 8 * blockDim
-  double2 w[8];
+// The stages S .. of a row: v holds stage S's inputs for S = 0 (the elements
+// q + r L/8 in v[r]), otherwise they are in `row`; the outputs q + r L/8 end in
+// v[r].  Every thread of the CTA calls it (the stages hold barriers).
+template <int LOG, int S>
+__device__ __forceinline__ void row_stages(double2 (&v)[8], double2* row,
+                                           const double2* __restrict__ st, int q, double sign) {
+  constexpr int L = 1 << LOG, TPR = L / 8, Ns = 1 << (3 * S);
+  constexpr int R = L / Ns >= 8 ? 8 : L / Ns, B = 8 / R;
+  const int k = q & (Ns - 1);
+  double2 w = make_double2(1.0, 0.0);
+  if (S > 0) {
+    w = __ldg(st + stage_off(S) + k);
+    w.y *= sign;
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int idx = threadIdx.x + it * blockDim.x;
-    w[it] = make_double2(1.0, 0.0);
-    if (idx < total) {
-      int off = 0, Ns = 8, rem = L >> 3, R = rem >= 8 ? 8 : rem;
-      while (idx >= off + (R - 1) * Ns) {
-        off += (R - 1) * Ns;
-        Ns *= R;
-        rem /= R;
-        R = rem >= 8 ? 8 : rem;
-      }
-      const int r = (idx - off) / Ns + 1, k = (idx - off) & (Ns - 1);
-      w[it] = tw[(int64_t)k * r * (m / ((int64_t)Ns * R))];
+    for (int r = 0; r < 8; ++r) v[r] = row[padi(q + r * TPR)];
+  }
+  if constexpr (R == 8) {
+    if (S > 0) twist8(v, w);
+    dft8(v, sign);
+  } else if constexpr (R == 4) {  // butterflies q and q + L/8
+    const double2 u = mul_w8(w, sign);
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const double2 x = b ? u : w, x2 = cmulf(x, x);
+      v[b + 2] = cmulf(v[b + 2], x);
+      v[b + 4] = cmulf(v[b + 4], x2);
+      v[b + 6] = cmulf(v[b + 6], cmulf(x, x2));
+      dft4(v[b], v[b + 2], v[b + 4], v[b + 6], sign);
+    }
+  } else {  // butterflies q + b L/8, b < 4
+    const double2 u = mul_w8(w, sign);
+    v[4] = cmulf(v[4], w);
+    v[5] = cmulf(v[5], u);
+    v[6] = cmulf(v[6], mul_si(w, sign));
+    v[7] = cmulf(v[7], mul_si(u, sign));
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const double2 x = v[b], y = v[b + 4];
+      v[b] = cadd(x, y);
+      v[b + 4] = csub(x, y);
     }
   }
+  if constexpr (Ns * R < L) {
+    if (S > 0) __syncthreads();  // the row was read
+    const int base = (q - k) * 8 + k;
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int idx = threadIdx.x + it * blockDim.x;
-    if (idx < total) tws[idx] = make_double2(w[it].x, sign * w[it].y);
+    for (int r = 0; r < 8; ++r) row[padi(base + r * Ns)] = v[r];
+    __syncthreads();
   }
+}
+
+template <int LOG, int S>
+__device__ __forceinline__ void row_rest(double2 (&v)[8], double2* row,
+                                         const double2* __restrict__ st, int q, double sign) {
+  if constexpr ((1 << (3 * S)) < (1 << LOG)) {
+    row_stages<LOG, S>(v, row, st, q, sign);
+    row_rest<LOG, S + 1>(v, row, st, q, sign);
+  }
+}
+
+// Row pitch for G rows side by side: lanes hold G rows of 8/G elements in a
+// 128-byte wavefront, so the rows start 8/G slots apart modulo 8.
+__host__ __device__ constexpr int row_pitch(int L, int G) {
+  return L + (L >> 3) + (G >= 8 ? 1 : 8 / G);
+}
+
+// fftplan.rs:43-76: unpack D (density) and K (odd kernel) from the packed
+// forward transform's entries k and m - k, multiply, repack as
+// Im_hat + i Re_hat.
+__device__ __forceinline__ double2 spectral(double2 ck, double2 cn, double ke) {
+  const double2 cnc = make_double2(cn.x, -cn.y);
+  const double2 s = make_double2(ck.x + cnc.x, ck.y + cnc.y);
+  const double2 df = make_double2(ck.x - cnc.x, ck.y - cnc.y);
+  const double2 D = make_double2(0.5 * s.x, 0.5 * s.y);
+  const double2 K = make_double2(0.5 * df.y, -0.5 * df.x);  // (-0.5 i) * df
+  const double2 rh = cmul(D, K);
+  return make_double2(D.x * ke - rh.y, D.y * ke + rh.x);
 }
 
 // Pass 1: Y[k1*m2 + n2] = W_m^{n2 k1} * sum_n1 x[m2 n1 + n2] W_m1^{n1 k1}, for
-// G columns n2 per CTA (G*m1/8 threads).
+// G columns n2 per CTA (G*m1/8 threads), lanes side by side in the columns.
+// With ke the input is the spectral product of x, formed on the way in (a
+// kernel of its own took 8 us at 2^20).
+template <int LOG>
 __global__ void __launch_bounds__(256, 4) fft_pass1(const double2* __restrict__ x,
-                                                 double2* __restrict__ y, int m1, int m2,
-                                                 int64_t m, const double2* __restrict__ tw,
-                                                 double sign) {
+                                                    double2* __restrict__ y, int m2, int64_t m,
+                                                    const double2* __restrict__ tw,
+                                                    const double2* __restrict__ st, double sign,
+                                                    const double* __restrict__ ke) {
   extern __shared__ double2 fsm[];
-  const int L = m1, Lp = L + (L >> 3) + 1, tpr = L >> 3;
-  const int G = blockDim.x / tpr, gl = __ffs(G) - 1;
-  double2* tws = fsm + G * Lp;
-  load_stage_twiddles(tws, tw, L, m, sign);
-  const int n2_0 = blockIdx.x * G;
-  // G*L = 8*blockDim: every thread moves exactly 8 elements each way
+  constexpr int L = 1 << LOG, TPR = L / 8;
+  const int G = blockDim.x / TPR, gl = __ffs(G) - 1;
+  const int g = threadIdx.x & (G - 1), q = threadIdx.x >> gl;
+  const int n2 = blockIdx.x * G + g;
   double2 v[8];
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int e = threadIdx.x + it * blockDim.x;
-    const int n1 = e >> gl, g = e & (G - 1);
-    v[it] = n2_0 + g < m2 ? x[(int64_t)m2 * n1 + n2_0 + g] : make_double2(0.0, 0.0);
+  for (int r = 0; r < 8; ++r) {
+    v[r] = make_double2(0.0, 0.0);
+    const int64_t k = (int64_t)m2 * (q + r * TPR) + n2;
+    if (n2 < m2) v[r] = ke ? spectral(x[k], x[(m - k) & (m - 1)], ke[k]) : x[k];
   }
+  row_rest<LOG, 0>(v, fsm + g * row_pitch(L, G), st, q, sign);
+  if (n2 >= m2) return;
+  // The outputs are column n2 at k1 = q + r L/8, their twiddles W_m^{n2 k1} =
+  // W^{n2 q} times the powers of W^{n2 L/8}: four table entries
+  // (W^a = W^{a - a mod 1024} W^{a mod 1024}) and products at most three deep.
+  const int64_t a0 = ((int64_t)n2 * q) & (m - 1), a1 = ((int64_t)n2 * TPR) & (m - 1);
+  double2 base = cmulf(__ldg(tw + (a0 & ~(int64_t)1023)), __ldg(tw + (a0 & 1023)));
+  double2 w = cmulf(__ldg(tw + (a1 & ~(int64_t)1023)), __ldg(tw + (a1 & 1023)));
+  base.y *= sign;
+  w.y *= sign;
+  twist8(v, w);
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int e = threadIdx.x + it * blockDim.x;
-    fsm[(e & (G - 1)) * Lp + padi(e >> gl)] = v[it];
-  }
-  __syncthreads();
-  row_fft(fsm + (threadIdx.x / tpr) * Lp, tws, L, threadIdx.x % tpr, sign);
-  // W_m^a = W_m^{a - a mod 1024} * W_m^{a mod 1024}, both from the table;
-  // two batches of 4 elements keep the loads in flight within 64 registers
-#pragma unroll
-  for (int h = 0; h < 8; h += 4) {
-    double2 wh[4], wl[4];
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int e = threadIdx.x + (h + it) * blockDim.x;
-      const int64_t a = ((int64_t)(n2_0 + (e & (G - 1))) * (e >> gl)) & (m - 1);
-      wh[it] = tw[a & ~(int64_t)1023];
-      wl[it] = tw[a & 1023];
-    }
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-      const int e = threadIdx.x + (h + it) * blockDim.x;
-      const int k1 = e >> gl, g = e & (G - 1);
-      const int n2 = n2_0 + g;
-      const double2 w = cmul(wh[it], wl[it]);
-      if (n2 < m2)
-        y[(int64_t)k1 * m2 + n2] = cmul(fsm[g * Lp + padi(k1)], make_double2(w.x, sign * w.y));
-    }
-  }
+  for (int r = 0; r < 8; ++r) y[(int64_t)(q + r * TPR) * m2 + n2] = cmulf(v[r], base);
 }
 
-// Pass 2: X[k1 + m1 k2] = sum_n2 Y[k1*m2 + n2] W_m2^{n2 k2}, G rows per CTA.
+// Pass 2: X[k1 + m1 k2] = sum_n2 Y[k1*m2 + n2] W_m2^{n2 k2}, G rows per CTA:
+// lanes along the row for the loads and the first stage, side by side in the
+// rows for the others and the stores.
+template <int LOG>
 __global__ void __launch_bounds__(256, 4) fft_pass2(const double2* __restrict__ y,
-                                                 double2* __restrict__ x, int m1, int m2,
-                                                 int64_t m, const double2* __restrict__ tw,
-                                                 double sign) {
+                                                    double2* __restrict__ x, int m1,
+                                                    const double2* __restrict__ st, double sign) {
   extern __shared__ double2 fsm[];
-  const int L = m2, Lp = L + (L >> 3) + 1, tpr = L >> 3;
-  const int G = blockDim.x / tpr, gl = __ffs(G) - 1, ll = __ffs(L) - 1;
-  double2* tws = fsm + G * Lp;
-  load_stage_twiddles(tws, tw, L, m, sign);
+  constexpr int L = 1 << LOG, TPR = L / 8;
+  const int G = blockDim.x / TPR, gl = __ffs(G) - 1, Lp = row_pitch(L, G);
   const int k1_0 = blockIdx.x * G;
   double2 v[8];
+  {
+    const int g = threadIdx.x / TPR, q = threadIdx.x % TPR;
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int e = threadIdx.x + it * blockDim.x;
-    const int g = e >> ll, n2 = e & (L - 1);
-    v[it] = k1_0 + g < m1 ? y[(int64_t)(k1_0 + g) * m2 + n2] : make_double2(0.0, 0.0);
+    for (int r = 0; r < 8; ++r)
+      v[r] = k1_0 + g < m1 ? y[(int64_t)(k1_0 + g) * L + q + r * TPR] : make_double2(0.0, 0.0);
+    row_stages<LOG, 0>(v, fsm + g * Lp, st, q, sign);
   }
+  const int g = threadIdx.x & (G - 1), q = threadIdx.x >> gl;  // the same for L = 8
+  row_rest<LOG, 1>(v, fsm + g * Lp, st, q, sign);
+  if (k1_0 + g >= m1) return;
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int e = threadIdx.x + it * blockDim.x;
-    fsm[(e >> ll) * Lp + padi(e & (L - 1))] = v[it];
-  }
-  __syncthreads();
-  row_fft(fsm + (threadIdx.x / tpr) * Lp, tws, L, threadIdx.x % tpr, sign);
-#pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int e = threadIdx.x + it * blockDim.x;
-    const int k2 = e >> gl, g = e & (G - 1);
-    if (k1_0 + g < m1) x[(int64_t)(k1_0 + g) + (int64_t)m1 * k2] = fsm[g * Lp + padi(k2)];
-  }
+  for (int r = 0; r < 8; ++r) x[(int64_t)(k1_0 + g) + (int64_t)m1 * (q + r * TPR)] = v[r];
 }
 
 // Transforms shorter than 64 points: direct DFT, one thread per output.
@@ -680,22 +682,12 @@ __global__ void dft_small(const double2* __restrict__ x, double2* __restrict__ y
   y[k] = acc;
 }
 
-// fftplan.rs:43-76: unpack D (density) and K (odd kernel) from the packed
-// forward transform, multiply, repack as Im_hat + i Re_hat.
+// The spectral product as a pass of its own, where the inverse transform does
+// not read the grid itself (Bluestein's form, fewer than 64 points).
 __global__ void spectral_kernel(const double2* __restrict__ C, const double* __restrict__ ke,
                                 double2* __restrict__ out, int64_t m) {
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= m) return;
-  const double2 ck = C[k];
-  const double2 cn = C[(m - k) % m];
-  const double2 cnc = make_double2(cn.x, -cn.y);
-  const double2 s = make_double2(ck.x + cnc.x, ck.y + cnc.y);
-  const double2 df = make_double2(ck.x - cnc.x, ck.y - cnc.y);
-  const double2 D = make_double2(0.5 * s.x, 0.5 * s.y);
-  const double2 K = make_double2(0.5 * df.y, -0.5 * df.x);  // (-0.5 i) * df
-  const double ih_re = D.x * ke[k], ih_im = D.y * ke[k];
-  const double2 rh = cmul(D, K);
-  out[k] = make_double2(ih_re - rh.y, ih_im + rh.x);
+  if (k < m) out[k] = spectral(C[k], C[(m - k) % m], ke[k]);
 }
 
 struct InterpArgs {
@@ -703,7 +695,9 @@ struct InterpArgs {
   int64_t nq;
   const double2* grid;
   int64_t m;
-  double lo, dx, inv_m;
+  double lo;
+  Spacing h;
+  double inv_m;
   Epilogue epi;
 };
 
@@ -714,7 +708,7 @@ __global__ void interp_kernel(const InterpArgs a) {
   if (t >= a.nq) return;
   const double qv = a.q[t];
   double tt;
-  const int64_t i0 = cell_of<N>(qv, a.lo, a.dx, a.m, &tt);
+  const int64_t i0 = cell_of<N>(qv, a.lo, a.h, a.m, &tt);
   double w[N];
   lagrange<N>(tt, w);
   double ra = 0.0, ia = 0.0;
@@ -819,8 +813,8 @@ int64_t transform_len(int64_t m) {
 // Constant tables, cached per call context for the last transform length,
 // m and (m, dx, eta); written and read on the context's stream.
 struct Tables {
-  double2* tw = nullptr;     // twiddles of the transform length
-  int64_t tw_m = 0;
+  double2* tw = nullptr;     // twiddles of the transform length, then the
+  int64_t tw_m = 0;          // stage twiddles of its two passes [STAGE_TAB] each
   double2* chirp = nullptr;  // Bluestein: c_j (m) and the filter's transform (M)
   double2* bhat = nullptr;
   int64_t bs_m = 0, bs_cap = 0, bhat_cap = 0;
@@ -838,6 +832,14 @@ struct Tables {
 
 unsigned blocks_for(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
+// m = m1 m2, the lengths of the two passes.
+void fft_split(int64_t m, int* m1, int* m2) {
+  int bits = 0;
+  while ((int64_t(1) << bits) < m) ++bits;
+  *m1 = 1 << ((bits + 1) / 2);
+  *m2 = 1 << (bits / 2);
+}
+
 shrk_status fft(double2* buf, double2* tmp, int64_t m, const double2* tw, double sign,
                 const char* family, cudaStream_t s);
 
@@ -849,9 +851,18 @@ shrk_status ensure_tables(int64_t m, double dx, double eta, const char* family, 
     if (T.tw) SHRK_CUDA(cudaFree(T.tw));
     T.tw = nullptr;
     T.tw_m = 0;
-    SHRK_CUDA(cudaMalloc(&T.tw, sizeof(double2) * L));
+    SHRK_CUDA(cudaMalloc(&T.tw, sizeof(double2) * (L + 2 * STAGE_TAB)));
     twiddle_kernel<<<blocks_for(L, 256), 256, 0, s>>>(T.tw, L);
     SHRK_CUDA(cudaGetLastError());
+    if (L >= 64) {
+      int m1 = 0, m2 = 0;
+      fft_split(L, &m1, &m2);
+      stage_twiddle_kernel<<<blocks_for(STAGE_TAB, 256), 256, 0, s>>>(T.tw + L, T.tw, m1, L);
+      SHRK_CUDA(cudaGetLastError());
+      stage_twiddle_kernel<<<blocks_for(STAGE_TAB, 256), 256, 0, s>>>(T.tw + L + STAGE_TAB, T.tw, m2,
+                                                                     L);
+      SHRK_CUDA(cudaGetLastError());
+    }
     T.tw_m = L;
   }
   if (L != m && T.bs_m != m) {
@@ -896,23 +907,57 @@ shrk_status ensure_tables(int64_t m, double dx, double eta, const char* family, 
   return SHRK_OK;
 }
 
-int ilog2(int64_t v) {
-  int b = 0;
-  while ((int64_t(1) << b) < v) ++b;
-  return b;
-}
-
 // Rows per CTA for a pass over `rows` transforms of length L: as many as fit
-// 256 threads (8 elements each), but no more than keeps ~2 CTAs per SM.
+// 256 threads (8 elements each), but no more than keeps ~2 CTAs per SM, and at
+// least two where they fit, whose neighbouring 16-byte elements fill a sector.
 int rows_per_cta(int L, int rows) {
   const int cap = 2048 / L;
   int g = 1;
-  while (g * 2 <= cap && (int64_t)rows / (g * 2) >= 296) g *= 2;
+  while (g * 2 <= cap && (g == 1 || (int64_t)rows / (g * 2) >= 296)) g *= 2;
   return g;
 }
 
-size_t pass_smem(int L, int G) {
-  return sizeof(double2) * ((size_t)G * (L + (L >> 3) + 1) + L);
+struct PassKernels {
+  void (*p1)(const double2*, double2*, int, int64_t, const double2*, const double2*, double,
+             const double*);
+  void (*p2)(const double2*, double2*, int, const double2*, double);
+};
+
+PassKernels pass_kernels(int L) {
+  switch (L) {
+    case 8: return {fft_pass1<3>, fft_pass2<3>};
+    case 16: return {fft_pass1<4>, fft_pass2<4>};
+    case 32: return {fft_pass1<5>, fft_pass2<5>};
+    case 64: return {fft_pass1<6>, fft_pass2<6>};
+    case 128: return {fft_pass1<7>, fft_pass2<7>};
+    case 256: return {fft_pass1<8>, fft_pass2<8>};
+    case 512: return {fft_pass1<9>, fft_pass2<9>};
+    case 1024: return {fft_pass1<10>, fft_pass2<10>};
+    default: return {fft_pass1<11>, fft_pass2<11>};
+  }
+}
+
+// src -> dst (which may be src) through tmp, all of m >= 64 points; with ke the
+// transform of the spectral product of src, which is then not dst.
+shrk_status fft_from(const double2* src, double2* dst, double2* tmp, int64_t m, const double2* tw,
+                     double sign, const double* ke, const char* family, cudaStream_t s) {
+  int m1 = 0, m2 = 0;
+  fft_split(m, &m1, &m2);
+  {
+    const int G = rows_per_cta(m1, m2);
+    LaunchScope ls(family, s);
+    pass_kernels(m1).p1<<<blocks_for(m2, G), G * (m1 >> 3), sizeof(double2) * G * row_pitch(m1, G),
+                          s>>>(src, tmp, m2, m, tw, tw + m, sign, ke);
+    SHRK_CUDA(cudaGetLastError());
+  }
+  {
+    const int G = rows_per_cta(m2, m1);
+    LaunchScope ls(family, s);
+    pass_kernels(m2).p2<<<blocks_for(m1, G), G * (m2 >> 3), sizeof(double2) * G * row_pitch(m2, G),
+                          s>>>(tmp, dst, m1, tw + m + STAGE_TAB, sign);
+    SHRK_CUDA(cudaGetLastError());
+  }
+  return SHRK_OK;
 }
 
 shrk_status fft(double2* buf, double2* tmp, int64_t m, const double2* tw, double sign,
@@ -924,32 +969,7 @@ shrk_status fft(double2* buf, double2* tmp, int64_t m, const double2* tw, double
     SHRK_CUDA(cudaMemcpyAsync(buf, tmp, sizeof(double2) * m, cudaMemcpyDeviceToDevice, s));
     return SHRK_OK;
   }
-  const int bits = ilog2(m);
-  const int m1 = 1 << ((bits + 1) / 2), m2 = 1 << (bits / 2);
-  static std::atomic<bool> opted[64];
-  int dev = 0;
-  SHRK_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64 || !opted[dev].load()) {
-    const int big = (int)pass_smem(FFT_MAXL, 1);
-    SHRK_CUDA(cudaFuncSetAttribute(fft_pass1, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    SHRK_CUDA(cudaFuncSetAttribute(fft_pass2, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    if (dev >= 0 && dev < 64) opted[dev] = true;
-  }
-  {
-    const int G = rows_per_cta(m1, m2);
-    LaunchScope ls(family, s);
-    fft_pass1<<<blocks_for(m2, G), G * (m1 >> 3), pass_smem(m1, G), s>>>(buf, tmp, m1, m2, m, tw,
-                                                                        sign);
-    SHRK_CUDA(cudaGetLastError());
-  }
-  {
-    const int G = rows_per_cta(m2, m1);
-    LaunchScope ls(family, s);
-    fft_pass2<<<blocks_for(m1, G), G * (m2 >> 3), pass_smem(m2, G), s>>>(tmp, buf, m1, m2, m, tw,
-                                                                        sign);
-    SHRK_CUDA(cudaGetLastError());
-  }
-  return SHRK_OK;
+  return fft_from(buf, buf, tmp, m, tw, sign, nullptr, family, s);
 }
 
 // Unnormalised DFT of the m-cell grid in buf (sign -1 forward, +1 inverse):
@@ -996,28 +1016,6 @@ shrk_status eval_grid(double2* A, double2* B, double2* Wa, double2* Wt, const Ta
                       const double* d_q, int64_t nq, const GridPlan& g, const Epilogue& epi,
                       cudaStream_t s);
 
-// Splat tuning, read once: SHRK_SPLAT_CELLS (0 / 1: the key searches on a
-// cell array off / on; default: on when the keys outnumber one wave of
-// resident threads), SHRK_SPLAT_THREAD_MAX and SHRK_SPLAT_WARP_MAX (the
-// RunSplit bounds; default 8 and 256, measured at p = 10^6 on the NUFFT's
-// 65 536-cell grid and the fft5 grid of 2^20 cells).
-struct SplatTuning {
-  int cells = -1;
-  RunSplit rs{8, 256};
-};
-
-const SplatTuning& splat_tuning() {
-  static const SplatTuning t = [] {
-    SplatTuning v;
-    if (const char* e = std::getenv("SHRK_SPLAT_CELLS")) v.cells = std::atoi(e) != 0 ? 1 : 0;
-    if (const char* e = std::getenv("SHRK_SPLAT_THREAD_MAX")) v.rs.thread_max = std::max(0, std::atoi(e));
-    if (const char* e = std::getenv("SHRK_SPLAT_WARP_MAX")) v.rs.warp_max = std::atoi(e);
-    v.rs.warp_max = std::max(v.rs.warp_max, v.rs.thread_max);
-    return v;
-  }();
-  return t;
-}
-
 // The whole grid convolution, or one of its two stages: with dens_out the
 // splat alone (the density of the sources into dens_out[m], nothing else);
 // with dens_in the evaluation alone from that density (no sources read).
@@ -1037,7 +1035,7 @@ shrk_status run_grid(const double* d_q, int64_t nq, const double* d_src, int64_t
   double2* B = A + m;
   double2* Wt = B + m;
   double2* Wa = Wt + L;
-  GridArgs ga{d_src, ns, g.dx < 0.0 ? 1 : 0, g.lo, g.dx, eta, m, A, dens_out};
+  GridArgs ga{d_src, ns, g.dx < 0.0 ? 1 : 0, g.lo, spacing(g.dx), eta, m, A, dens_out};
   if (dens_in) {
     LaunchScope ls(g.fam_splat, s);
     pack_density_kernel<<<blocks_for(m, 256), 256, 0, s>>>(ga, dens_in);
@@ -1048,60 +1046,28 @@ shrk_status run_grid(const double* d_q, int64_t nq, const double* d_src, int64_t
     if (dens_out) SHRK_CUDA(cudaMemsetAsync(dens_out, 0, sizeof(double) * m, s));
     return SHRK_OK;
   }
-  // slot 24: first [K + 1] | long runs: idx, base, nch, cnt, warp runs [K]
-  // each | three counters | chunk list [C] | source cells [ns] (when used) |
-  // run sums [K][N] | chunk partials [C][N], K = m + 2N + 2 keys from
-  // -N - 1, C = ns / RUN_CHUNK + K chunks at most (a chunked run of n sources
-  // has ceil(n / RUN_CHUNK)); the source cells are followed by their coarse
-  // table [ceil(ns / COARSE)]
+  // slot 24: runs [K], K = m + 2N + 2 keys from -N - 1 | run sums [K][N] |
+  // chunk heads and tails [C][N] each, C = ceil(ns / SPLAT_CHUNK)
   const int64_t n_keys = m + 2 * N + 2;
-  const int64_t max_chunks = ns / RUN_CHUNK + n_keys;
-  const SplatTuning& st = splat_tuning();
-  const bool use_cells =
-      st.cells >= 0 ? st.cells != 0 : (n_keys + 1) > (int64_t)sm_count() * 2048;
-  const size_t n_coarse = (size_t)((ns + COARSE - 1) / COARSE);
-  const size_t int_bytes =
-      ((sizeof(int) * (6 * (size_t)n_keys + 4 + (size_t)max_chunks +
-                       (use_cells ? (size_t)ns + n_coarse : 0))) +
-       255) & ~(size_t)255;
+  const int64_t chunks = (ns + SPLAT_CHUNK - 1) / SPLAT_CHUNK;
+  const size_t run_bytes = (sizeof(int2) * (size_t)n_keys + 255) & ~(size_t)255;
   void* sw = nullptr;
-  SHRK_TRY(scratch_get(24, int_bytes + sizeof(double) * N * ((size_t)n_keys + (size_t)max_chunks),
-                       &sw));
-  int* first = (int*)sw;
-  LongRuns lr;
-  lr.idx = first + n_keys + 1;
-  lr.base = lr.idx + n_keys;
-  lr.nch = lr.base + n_keys;
-  lr.cnt = lr.nch + n_keys;
-  lr.widx = lr.cnt + n_keys;
-  lr.counters = lr.widx + n_keys;
-  lr.chunk_run = lr.counters + 3;
-  int* cells = use_cells ? lr.chunk_run + max_chunks : nullptr;
-  int* coarse = use_cells ? cells + ns : nullptr;
-  double* runs = (double*)((char*)sw + int_bytes);
-  lr.partial = runs + (size_t)N * n_keys;
-  SHRK_CUDA(cudaMemsetAsync(lr.counters, 0, 3 * sizeof(int), s));
-  if (use_cells) {
+  SHRK_TRY(scratch_get(24, run_bytes + sizeof(double) * N * (size_t)(n_keys + 2 * chunks), &sw));
+  Runs runs;
+  runs.run = (int2*)sw;
+  runs.sum = (double*)((char*)sw + run_bytes);
+  runs.head = runs.sum + (size_t)N * n_keys;
+  runs.tail = runs.head + (size_t)N * chunks;
+  SHRK_CUDA(cudaMemsetAsync(runs.run, 0, sizeof(int2) * (size_t)n_keys, s));
+  {
     LaunchScope ls(g.fam_splat, s);
-    const int64_t blocks = std::min<int64_t>((ns + 255) / 256, (int64_t)sm_count() * 8);
-    cells_kernel<N><<<(unsigned)blocks, 256, 0, s>>>(ga, cells, coarse);
+    splat_kernel<N><<<(unsigned)chunks, SPLAT_NT, sizeof(double) * N * (SPLAT_CHUNK + 1), s>>>(
+        ga, runs);
     SHRK_CUDA(cudaGetLastError());
   }
   {
     LaunchScope ls(g.fam_splat, s);
-    keys_kernel<N><<<blocks_for(n_keys + 1, KEYS_CTA - 1), KEYS_CTA, 0, s>>>(ga, first, n_keys,
-                                                                             runs, lr, cells, coarse,
-                                                                             st.rs);
-    SHRK_CUDA(cudaGetLastError());
-  }
-  {
-    LaunchScope ls(g.fam_splat, s);
-    long_runs_kernel<N><<<sm_count() * 4, 256, 0, s>>>(ga, first, lr, runs);
-    SHRK_CUDA(cudaGetLastError());
-  }
-  {
-    LaunchScope ls(g.fam_splat, s);
-    pack_kernel<N><<<blocks_for(m, 256), 256, 0, s>>>(ga, first, runs);
+    pack_kernel<N><<<blocks_for(m, 256), 256, 0, s>>>(ga, runs);
     SHRK_CUDA(cudaGetLastError());
   }
   if (dens_out) return SHRK_OK;
@@ -1116,13 +1082,17 @@ shrk_status eval_grid(double2* A, double2* B, double2* Wa, double2* Wt, const Ta
                       cudaStream_t s) {
   const int64_t m = g.m;
   SHRK_TRY(dft(A, m, T, -1.0, Wa, Wt, g.fam_fft, s));
-  {
-    LaunchScope ls(g.fam_spectral, s);
-    spectral_kernel<<<blocks_for(m, 256), 256, 0, s>>>(A, T->ke, B, m);
-    SHRK_CUDA(cudaGetLastError());
+  if (m >= 64 && transform_len(m) == m) {
+    SHRK_TRY(fft_from(A, B, Wt, m, T->tw, +1.0, T->ke, g.fam_fft, s));
+  } else {
+    {
+      LaunchScope ls(g.fam_spectral, s);
+      spectral_kernel<<<blocks_for(m, 256), 256, 0, s>>>(A, T->ke, B, m);
+      SHRK_CUDA(cudaGetLastError());
+    }
+    SHRK_TRY(dft(B, m, T, +1.0, Wa, Wt, g.fam_fft, s));
   }
-  SHRK_TRY(dft(B, m, T, +1.0, Wa, Wt, g.fam_fft, s));
-  InterpArgs ia{d_q, nq, B, m, g.lo, g.dx, 1.0 / (double)m, epi};
+  InterpArgs ia{d_q, nq, B, m, g.lo, spacing(g.dx), 1.0 / (double)m, epi};
   {
     LaunchScope ls(g.fam_interp, s);
     interp_kernel<N><<<blocks_for(nq, 256), 256, 0, s>>>(ia);
