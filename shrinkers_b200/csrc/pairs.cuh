@@ -35,6 +35,25 @@ __device__ __forceinline__ void pair64(double x, double s, double eta2, double& 
   iv = iv + inv;
 }
 
+// Two FP64 pairs, x against s1 and s2 with |s1 - s2| <= eta, through one
+// reciprocal.  With N = 2x - (s1 + s2) and D = s1 - s2 (d1 d2 = (N^2 - D^2)/4):
+//   G = 4 (d1 d2 + eta^2) = N^2 + (4 eta^2 - D^2),
+//   16 e1 e2 = G^2 + 16 eta^2 D^2 = P,   e1 + e2 = (G + 2 D^2) / 2,
+//   d1/e1 + d2/e2 = 4 N G / P,           1/e1 + 1/e2 = 8 (G + 2 D^2) / P,
+// so C = 4 eta^2 - D^2, H = 16 eta^2 D^2 and W = 2 D^2 belong to the source
+// pair: ten operations for pair64's fourteen.  |D| <= eta keeps G at least
+// 3/5 of its terms' magnitudes.  N is formed from offsets to the block's
+// first source, so its rounding is that of the offsets.  re accumulates a
+// quarter and iv an eighth of the sums.
+__device__ __forceinline__ void pairs64x2(double X2, double2 sc, double2 hw, double& re,
+                                          double& iv) {
+  const double N = X2 - sc.x;
+  const double G = fma(N, N, sc.y);
+  const double r = rcp_f64(fma(G, G, hw.x));
+  re = fma(N, G * r, re);
+  iv = fma(G + hw.y, r, iv);
+}
+
 // ---------------------------------------------- FP32 separation scheme --
 // Targets and sources are split around a centre c: x - c = xh + xl and
 // s - c = mh + ml, with xh a multiple of a power of two u >= ulp(max|s-c|).

@@ -23,7 +23,8 @@
 // reciprocal per two sources (pairs32x4 in pairs.cuh), FP32 partials folded
 // into FP64 every 16 sources with the reciprocal's measured mean error taken
 // out at the fold.  Every other pair (the near field, where the
-// terms are large and d cancels) is summed in FP64, as are all reductions.
+// terms are large and d cancels) is summed in FP64 (pairs64x2 in pairs.cuh
+// where two adjacent sources are within eta), as are all reductions.
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "internal.h"
@@ -52,6 +53,13 @@ constexpr int R_MIXED = SHRK_R_MIXED;
 constexpr int R_SMALL_F64 = 1;    // targets per thread below one full tile
 constexpr int R_SMALL_MIXED = 2;  // the packed far field takes target pairs
 
+// MIXED sums over more sources take their near field pair by pair: it is then
+// a few per cent of the pairs, and the paired form costs the far field's loop
+// about 1 % in registers.  Full tiles, eta = 1/sqrt(p): 65 536 sources 1.11 ms
+// paired, 1.14 not; 262 144: 16.7 and 17.1; 400 000: 35.6 and 35.8; 10^6:
+// 214.1 and 212.3.
+constexpr int64_t PAIRED_MAX = 1 << 19;
+
 double g_near_k = SHRK_NEAR_K;
 // Budget of the pair kernels' bulk-copy waits (clock cycles); changed only by
 // shrk_diag_set_wait_limit to exercise the timeout path.
@@ -75,9 +83,9 @@ struct PairArgs {
   long long wait_cycles;   // budget of each bulk-copy wait
 };
 
-template <bool MIXED, int R>
+template <bool MIXED, int R, bool PAIRED = MIXED>
 __global__ void __launch_bounds__(NT, MIXED ? SHRK_MIXED_CTAS : 2) pair_sum_kernel(const PairArgs a) {
-  __shared__ PairStage st;
+  __shared__ PairStageOf<PAIRED> st;
   pair_stage_init(st);
   uint32_t phase = 0u;    // bit b: expected parity of st.bar[b]
   uint32_t pending = 0u;  // bit b: thread 0 has a copy in flight into st.sbuf[b]
@@ -100,7 +108,7 @@ __global__ void __launch_bounds__(NT, MIXED ? SHRK_MIXED_CTAS : 2) pair_sum_kern
     it.err = a.err;
     it.use_tma = a.use_tma != 0;
     it.wait_cycles = a.wait_cycles;
-    if (!pair_item<MIXED, R>(it, st, phase, pending)) return;
+    if (!pair_item<MIXED, R, PAIRED>(it, st, phase, pending)) return;
   }
 }
 
@@ -260,7 +268,8 @@ shrk_status exact_pair_sums(const double* d_tgt, int64_t nt, const double* d_src
   {
     LaunchScope ls(mixed ? "pair_sum_mixed" : "pair_sum_f64", s);
     if (mixed && small) pair_sum_kernel<true, R_SMALL_MIXED><<<pl.grid, NT, 0, s>>>(a);
-    else if (mixed) pair_sum_kernel<true, R_MIXED><<<pl.grid, NT, 0, s>>>(a);
+    else if (mixed && ns <= PAIRED_MAX) pair_sum_kernel<true, R_MIXED><<<pl.grid, NT, 0, s>>>(a);
+    else if (mixed) pair_sum_kernel<true, R_MIXED, false><<<pl.grid, NT, 0, s>>>(a);
     else if (small) pair_sum_kernel<false, R_SMALL_F64><<<pl.grid, NT, 0, s>>>(a);
     else pair_sum_kernel<false, R_F64><<<pl.grid, NT, 0, s>>>(a);
     SHRK_CUDA(cudaGetLastError());
@@ -367,7 +376,8 @@ shrk_status exact_pair_sums_fixed(const double* d_tgt, int64_t nt, const double*
   a.err = err;
   a.use_tma = ((uintptr_t)d_src % 16 == 0) ? 1 : 0;
   a.wait_cycles = g_wait_cycles.load();
-  if (mixed) pair_sum_kernel<true, R_MIXED><<<grid, NT, 0, s>>>(a);
+  if (mixed && ns <= PAIRED_MAX) pair_sum_kernel<true, R_MIXED><<<grid, NT, 0, s>>>(a);
+  else if (mixed) pair_sum_kernel<true, R_MIXED, false><<<grid, NT, 0, s>>>(a);
   else pair_sum_kernel<false, R_F64><<<grid, NT, 0, s>>>(a);
   SHRK_CUDA(cudaGetLastError());
   reduce_flagged_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(
