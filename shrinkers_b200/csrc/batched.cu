@@ -83,7 +83,7 @@ __global__ void batched_bounds_kernel(const double* __restrict__ ev,
 
 template <bool MIXED>
 __global__ void __launch_bounds__(PAIR_NT, B_CTAS) batched_kernel(const BatchArgs a) {
-  __shared__ PairStageOf<MIXED> st;
+  __shared__ PairStageOf<true> st;
   __shared__ int s_item;
   pair_stage_init(st);
   uint32_t phase = 0u, pending = 0u;

@@ -8,10 +8,16 @@
 // by plain loads.  F64 sums every pair in FP64.  MIXED sums a 256-source
 // block in FP32 on the packed f32x2 pipe (pairs32x4) when the block lies at
 // least near_dist from all of the warp's targets, and everything else in
-// FP64 -- PAIRED, two adjacent sources through one reciprocal wherever they
-// are within eta of each other (ten operations for fourteen; a batch of 1 024
-// spectra with 256 to 8 192 values, four tenths of its pairs in the near
-// field, 10.5 -> 9.1 ms) -- FP32 partials are folded into FP64 every PAIR_FOLD sources.
+// FP64; FP32 partials are folded into FP64 every PAIR_FOLD sources.
+//
+// PAIRED, the FP64 sums take two adjacent sources through one reciprocal
+// (pairs64x2) in every 64 sources whose neighbours are within eta, ten
+// operations for the pair form's fourteen; others, the rest of a block and
+// values outside the exponent range keep the pair form.  FP64-pipe-bound: a
+// batch of 1 024 FP64 spectra of 256 to 8 192 values 4.96 -> 3.80 ms (mixed,
+// to 16 384, 10.5 -> 9.1), 50 000 FP64 queries of as many sources 1.20 ->
+// 0.97 ms, with half as many additions an error against 64 bits of 4e-16
+// where it was 1.1e-15.
 #pragma once
 
 #include <type_traits>
@@ -32,7 +38,7 @@ struct __align__(16) PairStage {
   uint64_t bar[2];              // one mbarrier per buffer
 };
 
-// The same with the near field's source pairs (MIXED): {S, C}, {H, W} of
+// The same with the FP64 sums' source pairs: {S, C}, {H, W} of
 // pairs64x2, S = s1 + s2 relative to twice the SUB-block's first source, and
 // whether |s1 - s2| <= eta in all of 32 consecutive pairs.
 struct __align__(16) PairStageNear : PairStage {
@@ -71,8 +77,7 @@ __device__ __forceinline__ void pair_stage_init(PairStage& st) {
 // Sums one item.  phase / pending carry the mbarrier state across items.
 // Returns false (uniformly across the CTA, after recording DEV_ERR_TIMEOUT
 // and draining its own bulk copies) if a bulk copy never completed.
-// PAIRED: MIXED's near field two sources to a reciprocal (pairs64x2).
-template <bool MIXED, int R, bool PAIRED = MIXED>
+template <bool MIXED, int R, bool PAIRED = true>
 __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>& st,
                                           uint32_t& phase, uint32_t& pending) {
   constexpr int NT = PAIR_NT, CH = PAIR_CH, FOLD = PAIR_FOLD;
@@ -110,7 +115,7 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
     wlo = warp_min(mn);
     whi = warp_max(mx);
   }
-  if constexpr (PAIRED)  // (the first chunk's barrier follows)
+  if constexpr (MIXED && PAIRED)  // (the first chunk's barrier follows)
     if (lane == 0) st.range[warp] = make_double2(wlo, whi);
   double clo = 0.0, chi = 0.0;  // PAIRED: range of the CTA's targets
 
@@ -169,7 +174,7 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
       }
     }
     if constexpr (PAIRED) {
-      if (k == 0) {
+      if (MIXED && k == 0) {
         clo = st.range[0].x;
         chi = st.range[0].y;
 #pragma unroll
@@ -178,22 +183,26 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
           chi = fmax(chi, st.range[w].y);
         }
       }
-      // Adjacent sources of the full blocks that are near some target of the
-      // CTA, a flag to a warp's 32 pairs (the conditions are the warp's).
-      for (int i = tid; i < len / SUB * (SUB / 2); i += NT) {
-        const double2 bd = a.bounds[(cs + 2 * i) / SUB];
-        const double gap = fmax(bd.x - chi, clo - bd.y);
-        if (gap >= a.near_dist && fmax(bd.y - clo, chi - bd.x) <= 1e9) continue;
+      // Adjacent sources, a flag to a warp's 32 pairs (the conditions are the
+      // warp's); of MIXED the full blocks that are near some target of the CTA.
+      constexpr int GRP = MIXED ? SUB : 64;
+      for (int i = tid; i < len / GRP * (GRP / 2); i += NT) {
+        if constexpr (MIXED) {
+          const double2 bd = a.bounds[(cs + 2 * i) / SUB];
+          const double gap = fmax(bd.x - chi, clo - bd.y);
+          if (gap >= a.near_dist && fmax(bd.y - clo, chi - bd.x) <= 1e9) continue;
+        }
         const double cb = st.sbuf[b][2 * i / SUB * SUB];
         const double2 v = *reinterpret_cast<const double2*>(&st.sbuf[b][2 * i]);
         const double dd = v.x - v.y, d2 = dd * dd;
         st.sc[i] = make_double2((v.x - cb) + (v.y - cb), 4.0 * eta2 - d2);
         st.hw[i] = make_double2(16.0 * eta2 * d2, 2.0 * d2);
-        const bool tight = __all_sync(0xffffffffu, fabs(dd) <= eta);
+        const bool tight =
+            __all_sync(0xffffffffu, fabs(dd) <= eta && (MIXED || fabs(v.x - cb) <= 1e60));
         if (lane == 0) st.tight[i >> 5] = tight;
       }
     }
-    if (MIXED) __syncthreads();
+    if (MIXED || PAIRED) __syncthreads();
 
     for (int sub = 0; sub < len; sub += SUB) {
       const int slen = min(SUB, len - sub);
@@ -265,6 +274,12 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
           }
         };
         if constexpr (PAIRED) {
+          if (!MIXED) {  // no bounds: the targets themselves
+            bool in = eta >= 1e-60 && eta <= 1e60;
+#pragma unroll
+            for (int r = 0; r < R; ++r) in = in && fabs(x[r] - st.sbuf[b][sub]) <= 1e60;
+            pairs = __all_sync(0xffffffffu, in);
+          }
           if (pairs) {
             const double cb = st.sbuf[b][sub];
             double X2[R], rn[R], vn[R];
@@ -273,8 +288,9 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
               X2[r] = 2.0 * (x[r] - cb);
               rn[r] = vn[r] = 0.0;
             }
-            for (int h = 0; h < SUB; h += 64) {  // 32 pairs under one flag
-              if (st.tight[(sub + h) >> 6]) {
+            const int n = MIXED ? SUB : slen;
+            for (int h = 0; h < n; h += 64) {  // 32 pairs under one flag
+              if (h + 64 <= n && st.tight[(sub + h) >> 6]) {
                 const int i0 = (sub + h) >> 1;
 #pragma unroll 2
                 for (int i = i0; i < i0 + 32; ++i) {
@@ -283,7 +299,7 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
                   for (int r = 0; r < R; ++r) pairs64x2(X2[r], sc, hw, rn[r], vn[r]);
                 }
               } else {
-                plain(h, h + 64);
+                plain(h, min(h + 64, n));
               }
             }
 #pragma unroll

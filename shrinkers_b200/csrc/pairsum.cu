@@ -15,7 +15,8 @@
 // (deterministic) and applies the fused epilogue.
 //
 // F64 (R = 4): every pair in FP64, reciprocal = hardware seed + one
-// third-order Newton step.
+// third-order Newton step, for two adjacent sources at a time where they are
+// within eta of each other (pairs64x2 in pairs.cuh).
 //
 // MIXED (R = 4): a source block of 256 whose interval lies at least
 // max(K*eta, 1e-9) from all of the warp's targets is summed in FP32 on the
@@ -23,8 +24,8 @@
 // reciprocal per two sources (pairs32x4 in pairs.cuh), FP32 partials folded
 // into FP64 every 16 sources with the reciprocal's measured mean error taken
 // out at the fold.  Every other pair (the near field, where the
-// terms are large and d cancels) is summed in FP64 (pairs64x2 in pairs.cuh
-// where two adjacent sources are within eta), as are all reductions.
+// terms are large and d cancels) is summed in FP64 as above, as are all
+// reductions.
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "internal.h"
@@ -83,7 +84,7 @@ struct PairArgs {
   long long wait_cycles;   // budget of each bulk-copy wait
 };
 
-template <bool MIXED, int R, bool PAIRED = MIXED>
+template <bool MIXED, int R, bool PAIRED = true>
 __global__ void __launch_bounds__(NT, MIXED ? SHRK_MIXED_CTAS : 2) pair_sum_kernel(const PairArgs a) {
   __shared__ PairStageOf<PAIRED> st;
   pair_stage_init(st);

@@ -1,7 +1,7 @@
-"""The mixed kernel's paired FP64 near field against the FP64 sums.
+"""The paired FP64 sums: the mixed kernel's near field and the FP64 query sums.
 
 Every target's sum is near field here (all values within 32 eta), so the mixed
-result must be an FP64 result: each pair term carries a few roundings, and a
+result must be an FP64 result like the query one's: each pair term carries a few roundings, and a
 sum of n terms of one sign (the imaginary part) at most (n + 16) 2^-53 of
 itself; the real part the same against the sum of its terms' magnitudes, plus
 the rounding of the block offsets, at most 2^-52 of the spectrum's width over
@@ -30,6 +30,16 @@ def gpu_mixed(ev, eta):
     return re * ev.size, im * ev.size
 
 
+def gpu_points(q, ev, eta):
+    L = _native.load()
+    q, ev = np.ascontiguousarray(q), np.ascontiguousarray(ev)
+    re, im = np.empty(q.size), np.empty(q.size)
+    p = lambda a: a.ctypes.data_as(_D)
+    _native.check(L.shrk_stieltjes_at_points(p(q), q.size, p(ev), ev.size, eta, 2, 0, NAN, 0,
+                                             p(re), p(im)))
+    return re, im
+
+
 def spectrum(kind, p, eta):
     g = np.random.default_rng(p)
     if kind == "close":
@@ -46,23 +56,45 @@ def spectrum(kind, p, eta):
     return v
 
 
+def check(q, ev, eta, re, im):
+    n = ev.size
+    d = q.astype(np.longdouble)[:, None] - ev.astype(np.longdouble)[None, :]
+    e = d * d + np.longdouble(eta) ** 2
+    want_re, want_im, mag = (d / e).sum(1), (eta / e).sum(1), (np.abs(d) / e).sum(1)
+    eps = 2.0 ** -53
+    assert np.all(np.abs(im - want_im) <= (n + 16) * eps * want_im)
+    width = float(ev.max() - ev.min())
+    assert np.all(np.abs(re - want_re) <= (n + 16) * eps * mag + 2.0 * eps * (width / eta) * n / eta)
+
+
 @pytest.mark.parametrize("kind", ["close", "apart", "descending", "equal", "spike"])
 @pytest.mark.parametrize("p", [2, 255, 256, 257, 511, 512, 1300, 5000])
 @pytest.mark.parametrize("eta", [0.01, 3e-70])
 def test_near_field_is_fp64(kind, p, eta):
     ev = spectrum(kind, p, eta if eta > 1e-3 else 0.01)
-    n = ev.size
     re, im = gpu_mixed(ev, eta)
-    x = ev.astype(np.longdouble)
-    d = x[:, None] - x[None, :]
-    e = d * d + np.longdouble(eta) ** 2
     if eta < 1e-3:
         # outside the paired form's range: the same calls as ever, finite
         assert np.all(np.isfinite(re)) and np.all(np.isfinite(im))
         return
-    want_re, want_im = (d / e).sum(1), (eta / e).sum(1)
-    eps = 2.0 ** -53
-    assert np.all(np.abs(im - want_im) <= (n + 16) * eps * want_im)
-    mag = (np.abs(d) / e).sum(1)
-    width = float(ev.max() - ev.min())
-    assert np.all(np.abs(re - want_re) <= (n + 16) * eps * mag + 2.0 * eps * (width / eta) * n / eta)
+    check(ev, ev, eta, re, im)
+
+
+@pytest.mark.parametrize("kind", ["close", "apart", "descending", "equal", "spike"])
+@pytest.mark.parametrize("p", [1, 63, 64, 65, 257, 1300, 20001])
+def test_query_sums(kind, p):
+    """One target a thread and four, groups of 64 sources and the rest."""
+    ev = spectrum(kind, p, 0.01)
+    q = ev if p < 2000 else np.linspace(ev.min() - 0.1, ev.max() + 0.1, p)
+    re, im = gpu_points(q, ev, 0.01)
+    at = np.arange(q.size) if p < 2000 else np.random.default_rng(1).integers(0, q.size, 200)
+    check(q[at], ev, 0.01, re[at], im[at])
+
+
+def test_query_far_outside():
+    """Queries outside the paired form's range stay exact."""
+    ev = np.sort(np.random.default_rng(2).uniform(1.0, 2.0, 640))
+    q = np.concatenate([ev[:100], [1e70, -1e70]])
+    re, im = gpu_points(q, ev, 0.05)
+    assert np.all(np.isfinite(re)) and np.all(np.isfinite(im))
+    np.testing.assert_allclose(re[-2:], ev.size / q[-2:], rtol=1e-12)
