@@ -1163,20 +1163,24 @@ __device__ __forceinline__ double start_entry(int slot, int i) {
 // One thread per cluster, a warp per CTA.  Workspace: the factorisation of
 // T - lambda I (U's off-diagonals, reciprocal pivots, multipliers, row
 // swaps) and the right-hand side / solution x, rows relative to the block
-// start, stored per warp as [row][array][lane] so that a warp's rows are
-// one contiguous range (a chunk of rows is one span of memory, prefetched
-// into L2 a few chunks ahead of its use).  Each eigenvalue is factored once
-// and its three solves replay the elimination with multiplications only.
+// start, stored per warp as [row][array][lane].  Each eigenvalue is factored
+// once and its three solves replay the elimination with multiplications only.
 // Eigenvector of slot s goes to Zt[s + i p] (row s of Z^T) for i in [b0, b1).
+//
+// A lane's solve is one chain over the rows, a warp or less on an SM, so the
+// workspace reads must be far ahead of it: each lane copies its own values
+// into a ring of II_D chunks in shared memory, asynchronously.  (Chunks loaded
+// into registers when their turn came waited out the memory's latency each
+// time: 1.74 ms at p = 2 048, whose workspace of 200 MB does not stay in L2,
+// now 1.32.)
 constexpr int II_ARRAYS = 6;  // u1, u2, 1/pivot, multiplier, swap, x
-constexpr int II_CH = 16;     // rows whose loads are issued together
-constexpr int II_AHEAD = 6;   // chunks prefetched ahead
+constexpr int II_CH = 16;     // rows of a chunk
+constexpr int II_D = 5;       // chunks in flight
+constexpr int II_RING = II_D * II_CH * 4 * 32;  // doubles
 
-__device__ __forceinline__ void prefetch_rows(const double* base, int r0, int rows) {
-  // rows [r0, r0 + rows) of this warp's workspace, one bulk L2 prefetch
-  const unsigned bytes = (unsigned)rows * II_ARRAYS * 32 * sizeof(double);
-  const double* a = base + (int64_t)r0 * II_ARRAYS * 32;
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(bytes) : "memory");
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src)
+               : "memory");
 }
 
 constexpr int II_RS = II_ARRAYS * 32;  // doubles per workspace row of a warp
@@ -1192,14 +1196,15 @@ __device__ __forceinline__ void factor_row(double* r, double sub, double nd, dou
   const bool swp = fabs(diag) < fabs(sub);
   const double piv = swp ? sub : diag;
   const double num = swp ? diag : sub;
-  const double rinv = 1.0 / piv;
+  const double ap = fabs(piv);
+  const double rinv = ap > 0x1p-400 && ap < 0x1p400 ? rcp_rn_mid(piv) : 1.0 / piv;
   const double m = piv != 0.0 ? num * rinv : 0.0;
   r[II_U1 * 32] = swp ? nd : sup;
   r[II_U2 * 32] = swp ? ns : 0.0;
   r[II_MU * 32] = m;
   r[II_SW * 32] = swp ? 1.0 : 0.0;
   r[II_RP * 32] = fabs(piv) < small ? (piv < 0.0 ? -rsmall : rsmall) : rinv;
-  const double nd2 = swp ? sup - m * nd : nd - m * sup;
+  const double nd2 = swp ? fma(-m, nd, sup) : fma(-m, sup, nd);
   sup = swp ? -m * ns : ns;
   diag = nd2;
 }
@@ -1212,7 +1217,7 @@ __device__ __forceinline__ void forward_row(double* r, double rn, double m, doub
   const double keep = swp ? rn : rhs;
   const double other = swp ? rhs : rn;
   r[II_X * 32] = keep;
-  rhs = other - m * keep;
+  rhs = fma(-m, keep, other);
 }
 
 __global__ void __launch_bounds__(32) inverse_iteration_kernel(
@@ -1223,16 +1228,11 @@ __global__ void __launch_bounds__(32) inverse_iteration_kernel(
   const int t = blockIdx.x * 32 + lane;
   if (t >= ncl) return;
   const Cluster c = cl[t];
-  double* base = ws + (int64_t)blockIdx.x * p * II_RS;
-  double* const wl = base + lane;  // row 0 of this lane
+  double* const wl = ws + (int64_t)blockIdx.x * p * II_RS + lane;  // row 0 of this lane
 #define W(a, i) wl[(int64_t)(i) * II_RS + (a) * 32]
-  // lane 0 prefetches for the warp; rows past p are outside the region
-  const bool pf = lane == 0;
-  auto ahead = [&](int r0) {
-    if (!pf) return;
-    const int lo = max(r0, 0);
-    const int hi = (int)((int64_t)r0 + II_CH < p ? (int64_t)r0 + II_CH : p);
-    if (hi > lo) prefetch_rows(base, lo, hi - lo);
+  extern __shared__ double ring[];  // [II_D][II_CH][4][32]
+  const auto at = [&](int k, int u, int j) -> double* {
+    return ring + ((((k % II_D) * II_CH + u) * 4 + j) * 32 + lane);
   };
   const int n = c.b1 - c.b0;
   const double small = 2.220446049250313e-16 * tnorm + 1e-300;
@@ -1279,59 +1279,86 @@ __global__ void __launch_bounds__(32) inverse_iteration_kernel(
     double scale = 1.0;  // x in memory times scale is the current vector
     for (int iter = 0; iter < 3; ++iter) {
       // the factorisation's row operations on the right-hand side
-      for (int k = 0; k < II_AHEAD; ++k) ahead(k * CH);
+      __threadfence();  // the workspace before the copies of it
       double rhs = W(II_X, 0) * scale;
       {
-        int i0 = 0;
-        for (; i0 + CH < n; i0 += CH) {  // full chunks: rows i0 + u + 1 < n
-          ahead(i0 + II_AHEAD * CH);
-          double* r = &W(0, i0);
+        const int nch = (n - 1) / CH;  // full chunks: rows i0 + u + 1 < n
+        const auto fetch = [&](int k) {
+          if (k < nch) {
+            const double* r = &W(0, k * CH);
+#pragma unroll
+            for (int u = 0; u < CH; ++u) {
+              copy8(at(k, u, 0), r + (u + 1) * II_RS + II_X * 32);
+              copy8(at(k, u, 1), r + u * II_RS + II_MU * 32);
+              copy8(at(k, u, 2), r + u * II_RS + II_SW * 32);
+            }
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (int k = 0; k < II_D - 1; ++k) fetch(k);
+        for (int k = 0; k < nch; ++k) {
+          fetch(k + II_D - 1);
+          asm volatile("cp.async.wait_group %0;" ::"n"(II_D - 1) : "memory");
+          double* r = &W(0, k * CH);
           double rnv[CH], mv[CH], sv[CH];
 #pragma unroll
           for (int u = 0; u < CH; ++u) {
-            rnv[u] = r[(u + 1) * II_RS + II_X * 32] * scale;
-            mv[u] = r[u * II_RS + II_MU * 32];
-            sv[u] = r[u * II_RS + II_SW * 32];
+            rnv[u] = *at(k, u, 0) * scale;
+            mv[u] = *at(k, u, 1);
+            sv[u] = *at(k, u, 2);
           }
 #pragma unroll
           for (int u = 0; u < CH; ++u) forward_row(r + u * II_RS, rnv[u], mv[u], sv[u], rhs);
         }
-        for (int i = i0; i + 1 < n; ++i) {
+        for (int i = nch * CH; i + 1 < n; ++i) {
           const double rn = W(II_X, i + 1) * scale;
           forward_row(&W(0, i), rn, W(II_MU, i), W(II_SW, i), rhs);
         }
       }
       W(II_X, n - 1) = rhs;
+      __threadfence();
       // back substitution (the last row's U entries are zero), chunks of
-      // rows [i0 - CH + 1, i0]
-      for (int k = 0; k < II_AHEAD; ++k) ahead(n - (k + 1) * CH);
+      // rows from the last
       double nrm2 = 0.0, x1 = 0.0, x2 = 0.0;
       {
-        int i0 = n - 1;
-        for (; i0 - CH + 1 >= 0; i0 -= CH) {
-          ahead(i0 + 1 - (II_AHEAD + 1) * CH);
-          double* r = &W(0, i0);
-          double r0[CH], p1[CH], p2[CH], xv[CH];
+        const int nch = n / CH;
+        const auto fetch = [&](int k) {
+          if (k < nch) {
+            const double* r = &W(0, n - 1 - k * CH);
 #pragma unroll
-          for (int u = 0; u < CH; ++u) {
-            r0[u] = r[-u * II_RS + II_RP * 32];
-            p1[u] = r[-u * II_RS + II_U1 * 32];
-            p2[u] = r[-u * II_RS + II_U2 * 32];
-            xv[u] = r[-u * II_RS + II_X * 32];
+            for (int u = 0; u < CH; ++u) {
+              copy8(at(k, u, 0), r - u * II_RS + II_RP * 32);
+              copy8(at(k, u, 1), r - u * II_RS + II_U1 * 32);
+              copy8(at(k, u, 2), r - u * II_RS + II_U2 * 32);
+              copy8(at(k, u, 3), r - u * II_RS + II_X * 32);
+            }
           }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        for (int k = 0; k < II_D - 1; ++k) fetch(k);
+        for (int k = 0; k < nch; ++k) {
+          fetch(k + II_D - 1);
+          asm volatile("cp.async.wait_group %0;" ::"n"(II_D - 1) : "memory");
+          double* r = &W(0, n - 1 - k * CH);
 #pragma unroll
           for (int u = 0; u < CH; ++u) {
-            const double xi = (xv[u] - p1[u] * x1 - p2[u] * x2) * r0[u];
+            // the pivot multiplied in first: one FMA from x1 to xi
+            const double r0 = *at(k, u, 0);
+            const double xi = fma(-(*at(k, u, 1) * r0), x1,
+                                  fma(-(*at(k, u, 2) * r0), x2, *at(k, u, 3) * r0));
             r[-u * II_RS + II_X * 32] = xi;
-            nrm2 += xi * xi;
+            nrm2 = fma(xi, xi, nrm2);
             x2 = x1;
             x1 = xi;
           }
         }
+        const int i0 = n - 1 - nch * CH;
         for (int i = i0; i >= 0; --i) {
-          const double xi = (W(II_X, i) - W(II_U1, i) * x1 - W(II_U2, i) * x2) * W(II_RP, i);
+          const double r0 = W(II_RP, i);
+          const double xi =
+              fma(-(W(II_U1, i) * r0), x1, fma(-(W(II_U2, i) * r0), x2, W(II_X, i) * r0));
           W(II_X, i) = xi;
-          nrm2 += xi * xi;
+          nrm2 = fma(xi, xi, nrm2);
           x2 = x1;
           x1 = xi;
         }
@@ -1854,7 +1881,10 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   SHRK_CUDA(cudaMemsetAsync(Zt, 0, sizeof(double) * (size_t)P2, s));
   {
     LaunchScope ls("eigh_inverse_iteration", s);
-    inverse_iteration_kernel<<<cdiv(ncl, 32), 32, 0, s>>>(d, e, lam, dcl, ncl, p, tnorm,
+    constexpr int ring = II_RING * (int)sizeof(double);
+    SHRK_CUDA(cudaFuncSetAttribute(inverse_iteration_kernel,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, ring));
+    inverse_iteration_kernel<<<cdiv(ncl, 32), 32, ring, s>>>(d, e, lam, dcl, ncl, p, tnorm,
                                                             (double*)ws, Zt);
     SHRK_CUDA(cudaGetLastError());
   }
