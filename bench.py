@@ -310,8 +310,11 @@ def run_ours(args, world, rank, local):
         # ---- roofline of the dominant kernel (library CUDA-event timing)
         f32r, f64r = C.c_double(), C.c_double()
         _native.check(L.shrk_measure_pipe_rates(C.byref(f32r), C.byref(f64r)))
-        k_avg_s = kms.value / max(kn.value, 1) * 1e-3
-        ops_per_pair = 6.0 if prec == 1 else 7.0
+        # the family's time per step (the FP64 sums of a large spectrum are
+        # several launches)
+        k_avg_s = kms.value / max(args.steps, 1) * 1e-3
+        # FP64: 9 ops per unordered pair = 4.5 per ordered pair
+        ops_per_pair = 6.0 if prec == 1 else 4.5
         peak = f32r.value if prec == 1 else f64r.value
         achieved = p * p * ops_per_pair / k_avg_s
         traffic = None
@@ -608,8 +611,10 @@ def run_path(args, world, rank, local):
         if wl in ("adjoint", "batched") and kn.value:
             f32r, f64r = C.c_double(), C.c_double()
             _native.check(L.shrk_measure_pipe_rates(C.byref(f32r), C.byref(f64r)))
-            # adjoint: 15 ops per unordered pair = 7.5 per ordered pair
-            ops = (7.5 if wl == "adjoint" else (6.0 if prec == 1 else 7.0))
+            # adjoint: 12 (FP64) or 15 ops per unordered pair, half per ordered
+            # pair; FP64 batch: 10 ops per two pairs
+            ops = ((7.5 if prec == 1 else 6.0) if wl == "adjoint"
+                   else (6.0 if prec == 1 else 5.0))
             peak = f32r.value if prec == 1 else f64r.value
             ach = units * ops / k_s
             roof = {"bound": "fp32" if prec == 1 else "fp64", "achieved": ach / 1e12,
@@ -645,8 +650,7 @@ def run_path(args, world, rank, local):
                     "frac": ach / _measured_hbm(), "traffic": tr, "kernel": "nufft_splat",
                     "kernel_ms": k_s * 1e3, "grid_cells": m,
                     "basis": "splat family (splat and pack, two launches) per step: " + basis +
-                             "; traffic = DRAM bytes of those launches per step "
-                             "(ncu at p = 2^24, scaled by the source count)",
+                             "; traffic = DRAM bytes of those launches per step, where measured",
                     "families_ms": {k_: v[1] / max(1, args.steps) for k_, v in fams.items()},
                     "call_algorithmic_bytes": total_alg,
                     "call_gbs": total_alg / (ms * 1e-3) / 1e9}

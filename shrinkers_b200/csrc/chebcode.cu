@@ -2,8 +2,9 @@
 //
 // Replaces src/stieltjes/chebcode.rs: the flat pre-order tree of
 // FlatChebTree::build (242-572: midpoint split, barycentric leaf fill,
-// reverse-order parent merge, f32 mirrors) is built on the GPU, breadth
-// first, with every weight accumulated in the reference's order; the
+// reverse-order parent merge, f32 mirrors) is built on the GPU (in one CTA,
+// subtree by subtree, or level by level, by size), with every weight
+// accumulated in the reference's order; the
 // per-query evaluation (contribution_f64 607-711, contribution_fast32
 // 722-828) runs one thread per query, queries in their given order
 // (ascending queries keep a warp's traversals coherent).

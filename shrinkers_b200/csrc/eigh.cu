@@ -4,32 +4,31 @@
 // path).  Written for the GPU instead of restating Jacobi:
 //
 //   1. tridiagonalisation  Householder reflections H_j = I - beta_j v_j v_j^T,
-//                          one cooperative persistent kernel: every warp owns
-//                          columns of the (full, symmetric, column-major)
-//                          trailing matrix; per column j one grid barrier
-//                          after the symmetric product p = beta A22 v and one
-//                          after the rank-2 update A22 -= v w^T + w v^T,
-//                          w = p - (beta/2)(p^T v) v.  The reflectors stay in
-//                          the strict lower part of A (v_{j+1} and beta_j
-//                          aside), as in LAPACK's dsytrd.
+//                          one cooperative persistent kernel with the (full,
+//                          symmetric) trailing matrix in shared memory: per
+//                          column one walk applies the reflector and forms the
+//                          next product, one exchange of vectors through L2
+//                          and one grid barrier.  Above 2 048 rows a kernel
+//                          that walks the matrix in global memory runs first.
 //   2. eigenvalues         the tridiagonal T splits where an off-diagonal is
 //                          negligible; each eigenvalue of each unreduced block
-//                          by 32-way multisection on Sturm counts, one warp
-//                          per eigenvalue.
+//                          by multisection on Sturm counts (8 to 32 probes a
+//                          step), a warp serving several eigenvalues.
 //   3. eigenvectors of T   inverse iteration (LU with partial pivoting,
 //                          three solves from a fixed pseudo-random start),
 //                          one thread per cluster of eigenvalues closer than
 //                          CLUSTER_TOL ||T||, modified Gram-Schmidt inside a
-//                          cluster; then one Newton-Schulz step
-//                          Z <- Z (3I - Z^T Z)/2 on the whole basis, which
-//                          takes the remaining O(eps ||T|| / gap) overlaps
-//                          of close eigenvectors to rounding level.
+//                          cluster; then as many Newton-Schulz steps
+//                          Z <- Z (3I - Z^T Z)/2 on the whole basis as take
+//                          the remaining O(eps ||T|| / gap) overlaps of close
+//                          eigenvectors to rounding level.
 //   4. back-transformation U = H_0 ... H_{p-3} Z in blocks of NB reflectors,
-//                          each (I - Y T Y^T) in compact WY form (three
-//                          GEMMs).
+//                          each (I - Y T Y^T) in compact WY form, all blocks'
+//                          T formed at once, then two GEMMs a block.
 //
-// The GEMM (dgemm) is a plain FP64 tiled kernel: 64 x 64 outputs per CTA of
-// 256 threads, 4 x 4 per thread, k staged 16 at a time in shared memory.
+// The GEMM (dgemm): 128 x 128 tiles on the FP64 tensor instruction, the work
+// of a product cut in as many equal runs as there are SMs; a 64 x 64 SIMT form
+// for small products.
 #include "common.cuh"
 #include "internal.h"
 
