@@ -415,30 +415,32 @@ static shrk_status h2d_pair(void* dst, const void* a, size_t na, const void* b, 
 // Where the kernels of a host-pointer call write an output of `bytes` bytes:
 // small ones go straight to the pinned stage (each value is written once, by
 // the last kernel's epilogue, so the stores cross the bus as they come and no
-// copy follows), others to scratch.  take() gives the address, give() queues
-// what is left to do after the kernels; check_device_error completes both.
+// copy follows), others to scratch.  take() gives the address; give(), after
+// the kernels are launched, queues the copy to the caller that
+// check_device_error completes.  A call that fails in between has queued
+// nothing: its caller may free the array.
 struct HostOut {
   static constexpr size_t kDirectMax = (size_t)256 << 10;
   void* dev = nullptr;
   void* dst = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0, off = 0;  // off: of a direct output in the stage
   bool direct = false;
 
   shrk_status take(int slot, void* user, size_t n, cudaStream_t s) {
     dst = user;
     bytes = n;
     Context* c = t_cur;
-    size_t off = 0;
     char* st = n <= kDirectMax && c->host && s == c->stream ? stage_take(c, n, &off) : nullptr;
-    if (st) {
-      dev = st;
-      direct = true;
-      c->pending.push_back({user, off, n});
-      return SHRK_OK;
-    }
-    return scratch_get(slot, n, &dev);
+    if (!st) return scratch_get(slot, n, &dev);
+    dev = st;
+    direct = true;
+    return SHRK_OK;
   }
-  shrk_status give(cudaStream_t s) { return direct ? SHRK_OK : d2h(dst, dev, bytes, s); }
+  shrk_status give(cudaStream_t s) {
+    if (!direct) return d2h(dst, dev, bytes, s);
+    t_cur->pending.push_back({dst, off, bytes});
+    return SHRK_OK;
+  }
 };
 
 // At the entry of a host-pointer call: settle what an earlier call that
@@ -772,7 +774,8 @@ shrk_status lib_enter(cudaStream_t* stream) {
   c->mu.lock();
   t_cur = c;
   *stream = c->stream;
-  return SHRK_OK;
+  // the outermost call settles what an earlier one that failed left (as Guard)
+  return t_lib_stack.back().first != c ? stage_begin(c) : SHRK_OK;
 }
 
 void lib_exit() {
