@@ -11,9 +11,10 @@
 // FP64; FP32 partials are folded into FP64 every PAIR_FOLD sources.
 //
 // PAIRED, the FP64 sums take two adjacent sources through one reciprocal
-// (pairs64x2) in every 64 sources whose neighbours are within eta, ten
-// operations for the pair form's fourteen; others, the rest of a block and
-// values outside the exponent range keep the pair form.  FP64-pipe-bound: a
+// (pairs64x2) in every 64 sources whose neighbours are within eta and which lie
+// close together (PAIR_SPREAD), ten operations for the pair form's fourteen;
+// others, the rest of a block and values outside the exponent range keep the
+// pair form.  FP64-pipe-bound: a
 // batch of 1 024 FP64 spectra of 256 to 8 192 values 4.96 -> 3.80 ms (mixed,
 // to 16 384, 10.5 -> 9.1), 50 000 FP64 queries of as many sources 1.20 ->
 // 0.97 ms, with half as many additions an error against 64 bits of 4e-16
@@ -38,9 +39,10 @@ struct __align__(16) PairStage {
   uint64_t bar[2];              // one mbarrier per buffer
 };
 
-// The same with the FP64 sums' source pairs: {S, C}, {H, W} of
-// pairs64x2, S = s1 + s2 relative to twice the SUB-block's first source, and
-// whether |s1 - s2| <= eta in all of 32 consecutive pairs.
+// The same with the FP64 sums' source pairs: {S, C}, {H, W} of pairs64x2,
+// S = s1 + s2 relative to twice the middle source of their group of 64, and
+// whether the group may take that form: |s1 - s2| <= eta in all of its 32 pairs
+// and no source further than PAIR_SPREAD eta from the middle one.
 struct __align__(16) PairStageNear : PairStage {
   double2 sc[PAIR_CH / 2], hw[PAIR_CH / 2];
   unsigned char tight[PAIR_CH / 64];
@@ -48,6 +50,18 @@ struct __align__(16) PairStageNear : PairStage {
 };
 template <bool PAIRED>
 using PairStageOf = std::conditional_t<PAIRED, PairStageNear, PairStage>;
+
+// A group's separations are formed from offsets to its middle source, so each
+// carries the rounding of an offset: at most 2^-53 PAIR_SPREAD eta.  At 16 the
+// error against extended precision was the pair form's or less in every
+// spectrum tried (Marchenko-Pastur bulks with spikes of 256 to 16 384 values,
+// either order, eta = 0.1, 0.4 and 1 / sqrt(p): rms 3e-16 to 1.2e-15, pair form
+// 5e-16 to 4.9e-15; groups of two clusters 12 eta apart: 2e-16 to 4e-16, pair
+// form 2.5e-16 to 1.1e-15), and at 32 and 64 no more than a twentieth of the
+// sources would join (8 loses a third at eta = 0.1 / sqrt(p)).  Without a bound,
+// with offsets to the 256-source block's first source, one value of 1e3 in front
+// of a descending bulk cost three digits and one of 1e17 all of them.
+constexpr double PAIR_SPREAD = 16.0;
 
 struct PairItem {
   const double* tgt;        // targets
@@ -192,13 +206,14 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
           const double gap = fmax(bd.x - chi, clo - bd.y);
           if (gap >= a.near_dist && fmax(bd.y - clo, chi - bd.x) <= 1e9) continue;
         }
-        const double cb = st.sbuf[b][2 * i / SUB * SUB];
+        const double cg = st.sbuf[b][2 * i / 64 * 64 + 32];
         const double2 v = *reinterpret_cast<const double2*>(&st.sbuf[b][2 * i]);
-        const double dd = v.x - v.y, d2 = dd * dd;
-        st.sc[i] = make_double2((v.x - cb) + (v.y - cb), 4.0 * eta2 - d2);
+        const double o1 = v.x - cg, o2 = v.y - cg, dd = v.x - v.y, d2 = dd * dd;
+        st.sc[i] = make_double2(o1 + o2, 4.0 * eta2 - d2);
         st.hw[i] = make_double2(16.0 * eta2 * d2, 2.0 * d2);
-        const bool tight =
-            __all_sync(0xffffffffu, fabs(dd) <= eta && (MIXED || fabs(v.x - cb) <= 1e60));
+        const bool mine = fabs(dd) <= eta && fmax(fabs(o1), fabs(o2)) <= PAIR_SPREAD * eta &&
+                          (MIXED || fabs(v.x - st.sbuf[b][2 * i / SUB * SUB]) <= 1e60);
+        const bool tight = __all_sync(0xffffffffu, mine);
         if (lane == 0) st.tight[i >> 5] = tight;
       }
     }
@@ -281,17 +296,17 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
             pairs = __all_sync(0xffffffffu, in);
           }
           if (pairs) {
-            const double cb = st.sbuf[b][sub];
-            double X2[R], rn[R], vn[R];
+            double rn[R], vn[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
-              X2[r] = 2.0 * (x[r] - cb);
-              rn[r] = vn[r] = 0.0;
-            }
+            for (int r = 0; r < R; ++r) rn[r] = vn[r] = 0.0;
             const int n = MIXED ? SUB : slen;
             for (int h = 0; h < n; h += 64) {  // 32 pairs under one flag
               if (h + 64 <= n && st.tight[(sub + h) >> 6]) {
                 const int i0 = (sub + h) >> 1;
+                const double cg = st.sbuf[b][sub + h + 32];
+                double X2[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) X2[r] = 2.0 * (x[r] - cg);
 #pragma unroll 2
                 for (int i = i0; i < i0 + 32; ++i) {
                   const double2 sc = st.sc[i], hw = st.hw[i];

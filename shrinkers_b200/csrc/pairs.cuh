@@ -44,8 +44,9 @@ __device__ __forceinline__ void pair64(double x, double s, double eta2, double& 
 // pair: ten operations for pair64's fourteen.  |D| <= eta keeps G at least
 // 3/5 of its terms' magnitudes (at 2 eta, with more pairs inside, sums of
 // 1 000 sources at eta = 0.1/sqrt(p) were 1.4 times as far off as pair64's).
-// N is formed from offsets to the block's first source, so its rounding is
-// that of the offsets.  re accumulates a quarter and iv an eighth of the sums.
+// N is formed from offsets to a source of the group, so its rounding is that of
+// the offsets, which the caller bounds by a multiple of eta.  re accumulates a
+// quarter and iv an eighth of the sums.
 __device__ __forceinline__ void pairs64x2(double X2, double2 sc, double2 hw, double& re,
                                           double& iv) {
   const double N = X2 - sc.x;
