@@ -444,11 +444,14 @@ __global__ void pack_density_kernel(const GridArgs a, const double* __restrict__
 // which are its first butterfly, and ends with the outputs q + r L/8, so the
 // first stage takes its inputs, and the last leaves its outputs, in registers;
 // only the exchanges between stages go through shared memory (one pad slot per
-// 8 elements).  A butterfly's twiddles are the powers of one table entry.  With
-// the loads, the stores and every twiddle staged in shared memory a pass over
-// 2^20 points took 36 (columns) and 21 us (rows), now 18 and 12 (16 + 16 MB
-// each way through L2); bound by the latency of a CTA's chain of load, four
-// butterflies with three exchanges, and store, 4 CTAs an SM overlapping.
+// 8 elements).  Every twiddle is a table entry, those between the passes the
+// product of two, so the rounding is that of a transform with exact twiddles
+// (rms error 3.2e-16 at 2^20 points; with a butterfly's twiddles formed as
+// powers of one entry 5.8e-16, 3 us less for the two passes).  With the loads,
+// the stores and every twiddle staged in shared memory a pass over 2^20 points
+// took 36 (columns) and 21 us (rows), now 20 and 13 (16 + 16 MB each way
+// through L2); bound by the latency of a CTA's chain of load, four butterflies
+// with three exchanges, and store, 4 CTAs an SM overlapping.
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -501,30 +504,27 @@ __device__ __forceinline__ void dft8(double2* v, double sign) {
   v[7] = csub(e3, o3);
 }
 
-// v[r] *= w^r, r = 1..7, the powers at most three products deep.
-__device__ __forceinline__ void twist8(double2* v, double2 w) {
-  const double2 w2 = cmulf(w, w), w4 = cmulf(w2, w2), w3 = cmulf(w, w2);
-  v[1] = cmulf(v[1], w);
-  v[2] = cmulf(v[2], w2);
-  v[3] = cmulf(v[3], w3);
-  v[4] = cmulf(v[4], w4);
-  v[5] = cmulf(v[5], cmulf(w4, w));
-  v[6] = cmulf(v[6], cmulf(w4, w2));
-  v[7] = cmulf(v[7], cmulf(w4, w3));
+// w or its conjugate: a table entry for the transform's sign.
+__device__ __forceinline__ double2 signed_tw(double2 w, double sign) {
+  const int flip = __double2hiint(sign) & 0x80000000;
+  w.y = __hiloint2double(__double2hiint(w.y) ^ flip, __double2loint(w.y));
+  return w;
 }
 
-// Stage s >= 1 of a row transform combines Ns = 8^s points; its table holds
-// W_{Ns R}^k, k < Ns, from entry stage_off(s) (8 + 64 + 512 entries at most).
-constexpr int STAGE_TAB = 584;
-__host__ __device__ constexpr int stage_off(int s) { return s <= 1 ? 0 : s == 2 ? 8 : 72; }
+// Stage s >= 1 of a row transform combines Ns = 8^s points with radix R; its
+// table holds W_{Ns R}^{k r}, k < Ns, r = 1 .. R - 1, at [r - 1][k] from entry
+// stage_off(s) (7 x 8, 7 x 64 and 3 x 512 entries at most).
+constexpr int STAGE_TAB = 2040;
+__host__ __device__ constexpr int stage_off(int s) { return s <= 1 ? 0 : s == 2 ? 56 : 504; }
 
 __global__ void stage_twiddle_kernel(double2* __restrict__ out, const double2* __restrict__ tw,
                                      int L, int64_t m) {
   const int idx = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int s = idx < 8 ? 1 : idx < 72 ? 2 : 3, Ns = 1 << (3 * s);
+  const int s = idx < 56 ? 1 : idx < 504 ? 2 : 3, Ns = 1 << (3 * s);
   if (idx >= STAGE_TAB || Ns >= L) return;
   const int R = L / Ns < 8 ? L / Ns : 8;
-  out[idx] = tw[(int64_t)(idx - stage_off(s)) * (m / ((int64_t)Ns * R))];
+  const int r = (idx - stage_off(s)) / Ns + 1, k = (idx - stage_off(s)) & (Ns - 1);
+  if (r < R) out[idx] = tw[(int64_t)k * r * (m / ((int64_t)Ns * R))];
 }
 
 // The stages S .. of a row: v holds stage S's inputs for S = 0 (the elements
@@ -536,28 +536,31 @@ __device__ __forceinline__ void row_stages(double2 (&v)[8], double2* row,
   constexpr int L = 1 << LOG, TPR = L / 8, Ns = 1 << (3 * S);
   constexpr int R = L / Ns >= 8 ? 8 : L / Ns, B = 8 / R;
   const int k = q & (Ns - 1);
-  double2 w = make_double2(1.0, 0.0);
   if (S > 0) {
-    w = __ldg(st + stage_off(S) + k);
-    w.y *= sign;
 #pragma unroll
     for (int r = 0; r < 8; ++r) v[r] = row[padi(q + r * TPR)];
   }
+  // W_{Ns R}^{r (k + at)}
+  const auto tw = [&](int r, int at) {
+    return signed_tw(__ldg(st + stage_off(S) + (r - 1) * Ns + k + at), sign);
+  };
   if constexpr (R == 8) {
-    if (S > 0) twist8(v, w);
+    if (S > 0) {
+#pragma unroll
+      for (int r = 1; r < 8; ++r) v[r] = cmulf(v[r], tw(r, 0));
+    }
     dft8(v, sign);
-  } else if constexpr (R == 4) {  // butterflies q and q + L/8
-    const double2 u = mul_w8(w, sign);
+  } else if constexpr (R == 4) {  // butterflies q and q + Ns/2
+    const double2 w2 = tw(2, 0);
 #pragma unroll
     for (int b = 0; b < B; ++b) {
-      const double2 x = b ? u : w, x2 = cmulf(x, x);
-      v[b + 2] = cmulf(v[b + 2], x);
-      v[b + 4] = cmulf(v[b + 4], x2);
-      v[b + 6] = cmulf(v[b + 6], cmulf(x, x2));
+      v[b + 2] = cmulf(v[b + 2], tw(1, b * (Ns / 2)));
+      v[b + 4] = cmulf(v[b + 4], b ? mul_si(w2, sign) : w2);
+      v[b + 6] = cmulf(v[b + 6], tw(3, b * (Ns / 2)));
       dft4(v[b], v[b + 2], v[b + 4], v[b + 6], sign);
     }
-  } else {  // butterflies q + b L/8, b < 4
-    const double2 u = mul_w8(w, sign);
+  } else {  // butterflies q + b Ns/4, b < 4
+    const double2 w = tw(1, 0), u = tw(1, Ns / 4);
     v[4] = cmulf(v[4], w);
     v[5] = cmulf(v[5], u);
     v[6] = cmulf(v[6], mul_si(w, sign));
@@ -631,16 +634,16 @@ __global__ void __launch_bounds__(256, 4) fft_pass1(const double2* __restrict__ 
   row_rest<LOG, 0>(v, fsm + g * row_pitch(L, G), st, q, sign);
   if (n2 >= m2) return;
   // The outputs are column n2 at k1 = q + r L/8, their twiddles W_m^{n2 k1} =
-  // W^{n2 q} times the powers of W^{n2 L/8}: four table entries
-  // (W^a = W^{a - a mod 1024} W^{a mod 1024}) and products at most three deep.
-  const int64_t a0 = ((int64_t)n2 * q) & (m - 1), a1 = ((int64_t)n2 * TPR) & (m - 1);
-  double2 base = cmulf(__ldg(tw + (a0 & ~(int64_t)1023)), __ldg(tw + (a0 & 1023)));
-  double2 w = cmulf(__ldg(tw + (a1 & ~(int64_t)1023)), __ldg(tw + (a1 & 1023)));
-  base.y *= sign;
-  w.y *= sign;
-  twist8(v, w);
+  // W^{n2 q} W^{n2 r L/8}: two table entries, the second shared by the column.
+  const double2 base = signed_tw(__ldg(tw + (unsigned)(n2 * q)), sign);
+  const unsigned step = (unsigned)(n2 * TPR);  // m <= 2^22
+  double2* out = y + (int64_t)q * m2 + n2;
+  out[0] = cmulf(v[0], base);
 #pragma unroll
-  for (int r = 0; r < 8; ++r) y[(int64_t)(q + r * TPR) * m2 + n2] = cmulf(v[r], base);
+  for (int r = 1; r < 8; ++r) {
+    const double2 w = signed_tw(__ldg(tw + r * step), sign);
+    out[(unsigned)(r * TPR * m2)] = cmulf(cmulf(v[r], w), base);
+  }
 }
 
 // Pass 2: X[k1 + m1 k2] = sum_n2 Y[k1*m2 + n2] W_m2^{n2 k2}, G rows per CTA:
