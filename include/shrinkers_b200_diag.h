@@ -36,6 +36,12 @@ shrk_status shrk_measure_pipe_rates(double* fp32_ops_per_s, double* fp64_ops_per
  * (log-uniform).  The mixed-precision pair kernel removes the log-uniform
  * mean from its FP32 far-field partials; this probe re-measures it. */
 shrk_status shrk_measure_rcp_bias(double* uniform_mean, double* log_mean);
+/* The library's branch-free rounded reciprocals on device arrays of n values:
+ * d_rcp = 1 / a, d_quot = w / |a|, d_rcp32 = 1 / |(float)a|, each equal to the
+ * IEEE quotient for |a| in [2^-400, 2^400] (d_rcp [2^-900, 2^900], d_rcp32
+ * [2^-120, 2^120]) and w = 0 or |w| in [2^-400, 2^400].  Stream-ordered. */
+shrk_status shrk_diag_reciprocals(const double* d_a, const double* d_w, size_t n, double* d_rcp,
+                                  double* d_quot, float* d_rcp32, void* stream);
 /* Budget, in GPU clock cycles, of every bulk-copy wait of the exact pair
  * kernels launched after this call (shrk_stieltjes_all / _at_points with an
  * exact method, their _dev forms, shrk_stieltjes_at_points_noalloc); returns

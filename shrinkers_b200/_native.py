@@ -93,6 +93,7 @@ SIGNATURES = {
     "shrk_launch_count": (C.c_int64, []),
     "shrk_measure_pipe_rates": (_ST, [_D, _D]),
     "shrk_measure_rcp_bias": (_ST, [_D, _D]),
+    "shrk_diag_reciprocals": (_ST, [_P, _P, _SZ, _P, _P, _P, _P]),
     "shrk_diag_set_wait_limit": (C.c_longlong, [C.c_longlong]),
     "shrk_diag_dgemm": (_ST, [C.c_int, C.c_int, C.c_int64, C.c_int64, C.c_int64, C.c_double, _P,
                               C.c_int64, _P, C.c_int64, C.c_double, _P, C.c_int64, _P]),

@@ -1724,6 +1724,15 @@ shrk_status shrk_measure_rcp_bias(double* uniform_mean, double* log_mean) {
   return measure_rcp_bias(uniform_mean, log_mean);
 }
 
+shrk_status shrk_diag_reciprocals(const double* d_a, const double* d_w, size_t n, double* d_rcp,
+                                  double* d_quot, float* d_rcp32, void* stream) {
+  if (n > (size_t)INT32_MAX || (n > 0 && (!d_a || !d_w || !d_rcp || !d_quot || !d_rcp32)))
+    return einval("reciprocals: invalid arguments");
+  Guard g(stream);
+  SHRK_TRY(g.st);
+  return eval_reciprocals(d_a, d_w, (int64_t)n, d_rcp, d_quot, d_rcp32, (cudaStream_t)stream);
+}
+
 long long shrk_diag_set_wait_limit(long long cycles) { return set_wait_cycles(cycles); }
 
 shrk_status shrk_diag_dgemm(int ta, int tb, int64_t m, int64_t n, int64_t k, double alpha,

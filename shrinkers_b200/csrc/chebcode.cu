@@ -361,14 +361,14 @@ __device__ __forceinline__ void bary_rows_batch(double x, double mass, bool vali
       const double d = x - rt.t[j];
       mid = mid && row_mid(d);
       if (d == 0.0 && hit < 0) hit = j;
-      const double q = rt.lam[j] * copysign(rcp_rn_mid(fabs(d)), d);
+      const double q = rt.lam[j] * rcp_rn_signed(d);
       rt.q[lane * ROW_RS + j] = q;
       sum += q;
     }
     if (hit >= 0) {
       m = mass;
     } else if (mid && row_mid(sum)) {
-      m = mass * copysign(rcp_rn_mid(fabs(sum)), sum);
+      m = mass * rcp_rn_signed(sum);
     } else {
       sum = 0.0;
       for (int j = 0; j < n; ++j) {

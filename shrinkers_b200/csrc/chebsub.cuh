@@ -309,7 +309,7 @@ __device__ __forceinline__ void bary_rows_set(double x, const double (&mass)[NS]
     }
 #pragma unroll
     for (int j = 0; j < N; ++j) sum += q[j];
-    const double scale = copysign(rcp_rn_mid(fabs(sum)), sum);
+    const double scale = rcp_rn_signed(sum);
     // a hit's row is its mass times the hit node's unit vector
     plain = !on || hit >= 0 || (plain && row_mid(sum));
 #pragma unroll

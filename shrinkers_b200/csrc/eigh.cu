@@ -1213,7 +1213,7 @@ __device__ __forceinline__ void factor_row(double* r, double sub, double nd, dou
   const double piv = swp ? sub : diag;
   const double num = swp ? diag : sub;
   const double ap = fabs(piv);
-  const double rinv = ap > 0x1p-400 && ap < 0x1p400 ? rcp_rn_mid(piv) : 1.0 / piv;
+  const double rinv = ap > 0x1p-400 && ap < 0x1p400 ? rcp_rn_signed(piv) : 1.0 / piv;
   const double m = piv != 0.0 ? num * rinv : 0.0;
   r[II_U1 * 32] = swp ? nd : sup;
   r[II_U2 * 32] = swp ? ns : 0.0;

@@ -196,5 +196,7 @@ long long set_wait_cycles(long long cycles);
 long long wait_cycles();
 shrk_status measure_pipe_rates(double* fp32, double* fp64);
 shrk_status measure_rcp_bias(double* uniform_mean, double* log_mean);
+shrk_status eval_reciprocals(const double* d_a, const double* d_w, int64_t n, double* d_rcp,
+                             double* d_quot, float* d_rcp32, cudaStream_t s);
 
 }  // namespace shrk

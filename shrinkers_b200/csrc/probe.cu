@@ -1,6 +1,7 @@
 // Pipe-rate probes: measured FP32 and FP64 FMA lane-op rates of the current
-// device, the denominators of the exact kernels' roofline fractions; and the
-// mean error of the MUFU reciprocal that the mixed kernel corrects for.  Each
+// device, the denominators of the exact kernels' roofline fractions; the mean
+// error of the MUFU reciprocal that the mixed kernel corrects for; and the
+// rounded reciprocals of common.cuh evaluated on given values.  Each
 // thread runs independent dependency chains of FMAs whose operands stay in
 // registers, sized so that issue (not latency) limits the rate.
 #include "common.cuh"
@@ -78,7 +79,26 @@ __global__ void __launch_bounds__(BIAS_NT) rcp_bias_kernel(double* part) {
   if (threadIdx.x < 3) part[blockIdx.x * 3 + threadIdx.x] = red[threadIdx.x][0];
 }
 
+__global__ void reciprocals_kernel(const double* __restrict__ a, const double* __restrict__ w,
+                                   int64_t n, double* __restrict__ rcp, double* __restrict__ quot,
+                                   float* __restrict__ rcp32) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  rcp[i] = rcp_rn_signed(a[i]);
+  quot[i] = div_rn_mid(w[i], fabs(a[i]));
+  rcp32[i] = rcp_rn_mid(fabsf((float)a[i]));
+}
+
 }  // namespace
+
+shrk_status eval_reciprocals(const double* d_a, const double* d_w, int64_t n, double* d_rcp,
+                             double* d_quot, float* d_rcp32, cudaStream_t s) {
+  if (n == 0) return SHRK_OK;
+  reciprocals_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_a, d_w, n, d_rcp, d_quot,
+                                                                d_rcp32);
+  SHRK_CUDA(cudaGetLastError());
+  return SHRK_OK;
+}
 
 shrk_status measure_rcp_bias(double* uniform_mean, double* log_mean) {
   cudaStream_t s = library_stream();
