@@ -79,11 +79,10 @@ struct BuildArrays {
   int32_t* pre;  // pre-order index
   int* counter;  // next free BFS slot
   int* levels;   // level L = BFS slots [levels[2L], levels[2L+1])
-  int32_t* parent;  // parent slot (-1 at the root)
-  int32_t* arrive;  // the leaf starts' prefix count
+  int32_t* prefix;  // the leaf starts' exclusive prefix count
   int32_t* dep;     // depth
   int32_t* rturn;   // right turns on the path from the root
-  int32_t* leafpre; // [ns + 1]: leaf starts, then their exclusive prefix count
+  int32_t* leafpre; // [ns + 1]: leaf starts
 };
 
 __device__ __forceinline__ void tree_split_node(const double* __restrict__ sorted, BuildArrays b,
@@ -110,7 +109,6 @@ __device__ __forceinline__ void tree_split_node(const double* __restrict__ sorte
   b.bhi[slot + 1] = hi_idx;
   b.lc[i] = slot;
   b.rc[i] = slot + 1;
-  b.parent[slot] = b.parent[slot + 1] = i;
   b.dep[slot] = b.dep[slot + 1] = depth + 1;
   b.rturn[slot] = b.rturn[i];
   b.rturn[slot + 1] = b.rturn[i] + 1;
@@ -155,8 +153,7 @@ __device__ __forceinline__ void tree_split_node_warp(const double* __restrict__ 
     b.bhi[slot + 1] = hi_idx;
     b.lc[i] = slot;
     b.rc[i] = slot + 1;
-    if (b.parent) b.parent[slot] = b.parent[slot + 1] = i;  // absent in the one-CTA build
-    if (b.dep) {
+    if (b.dep) {  // absent in the one-CTA build
       b.dep[slot] = b.dep[slot + 1] = depth + 1;
       b.rturn[slot] = b.rturn[i];
       b.rturn[slot + 1] = b.rturn[i] + 1;
@@ -255,7 +252,7 @@ __global__ void tree_fill_kernel(const double* __restrict__ sorted, BuildArrays 
 // arrays.  A warp splits a node: its upper_bound of mid probes 32 evenly spaced
 // positions per step (the range shrinks 33-fold), then scans the last <= 32 --
 // the same index as tree_split_node's binary search, so the tree is identical.
-// The node arrays are in shared memory; parent, dep, rturn and arrive are not
+// The node arrays are in shared memory; dep, rturn, prefix and leafpre are not
 // needed (null).  Returns the number of levels.
 __device__ int topology_cta(const double* __restrict__ sorted, BuildArrays b, int64_t ns,
                             int64_t leaf_cap, FlatTree f, ChebConsts k, double theta_sq) {
@@ -266,11 +263,6 @@ __device__ int topology_cta(const double* __restrict__ sorted, BuildArrays b, in
     b.blo[0] = 0;
     b.bhi[0] = ns;
     b.pre[0] = 0;
-    if (b.parent) b.parent[0] = -1;
-    if (b.dep) {
-      b.dep[0] = 0;
-      b.rturn[0] = 0;
-    }
     *b.counter = 1;
     b.levels[0] = 0;
     b.levels[1] = 1;
@@ -301,15 +293,9 @@ __device__ int topology_cta(const double* __restrict__ sorted, BuildArrays b, in
   for (int L = 0; L < last; ++L) {
     const int begin = b.levels[2 * L], end = b.levels[2 * L + 1];
     for (int i = begin + tid; i < end; i += nt) {
-      if (b.arrive) b.arrive[i] = 0;
-      if (b.parent && L == 0) b.parent[i] = -1;
       if (b.lc[i] >= 0) {
         b.pre[b.lc[i]] = b.pre[i] + 1;
         b.pre[b.rc[i]] = b.pre[i] + 1 + b.size[b.lc[i]];
-        if (b.parent) {
-          b.parent[b.lc[i]] = i;
-          b.parent[b.rc[i]] = i;
-        }
       }
     }
     __syncthreads();
@@ -452,18 +438,16 @@ __global__ void __launch_bounds__(WEIGHT_NT) tree_p2m_kernel(const double* __res
 }
 
 // M2M of node i: rows (child c, child node ti), the left child first, in
-// node order, zero masses skipped (2 n <= 32 rows, one batch).  cg: read the
-// children's weights past L1 (they may come from another SM in this launch).
+// node order, zero masses skipped (2 n <= 32 rows, one batch).
 __device__ __forceinline__ void m2m_node(const BuildArrays& b, int i, int lane, const FlatTree& f,
-                                         double* wts, const ChebConsts& k, bool cg, RowTile& rt) {
+                                         double* wts, const ChebConsts& k, RowTile& rt) {
   const int idx = b.pre[i];
   const int n = k.n;
   row_tile_node(rt, f, idx, n, k, lane);
   double x = 0.0, mass = 0.0;
   if (lane < 2 * n) {
     const int kid = b.pre[lane < n ? b.lc[i] : b.rc[i]], ti = lane % n;
-    const double* mp = wts + (int64_t)kid * n + ti;
-    mass = cg ? __ldcg(mp) : *mp;
+    mass = wts[(int64_t)kid * n + ti];
     x = f.nodes[(int64_t)kid * n + ti];
   }
   double w = 0.0;
@@ -478,7 +462,7 @@ __global__ void __launch_bounds__(WEIGHT_NT) tree_m2m_kernel(BuildArrays b, int 
   const int i = begin + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= end || b.lc[i] < 0) return;  // whole warps leave together
-  m2m_node(b, i, lane, f, wts, k, false, tiles[threadIdx.x >> 5]);
+  m2m_node(b, i, lane, f, wts, k, tiles[threadIdx.x >> 5]);
 }
 
 __device__ __forceinline__ void mirror_f32(const FlatTree& f, int idx, int n, int lane,
@@ -498,10 +482,9 @@ __device__ __forceinline__ void mirror_f32(const FlatTree& f, int idx, int n, in
 // launch: the spectrum and every node array of the topology in shared memory
 // (a tree over ns sources has at most 2 ns - 1 nodes), the flat arrays, the
 // P2M of the leaves, then the M2M level by level from the deepest with a
-// barrier between levels, and the f32 mirror.  The same device functions as
-// the multi-launch builds, node by node, so the same tree and the same
-// weights bit for bit; what goes is a launch, the per-level round trips to
-// global memory and the climbing warps' fences and arrival counters.
+// barrier between levels, and the f32 mirror.  The same device functions as the
+// level-by-level build, node by node, so the same tree and the same weights bit
+// for bit, without its per-level round trips to global memory.
 constexpr int64_t TINY_NS = 2048;
 constexpr int TINY_NT = 1024;
 constexpr int TINY_TILES = 16;  // warps with a row tile (P2M / M2M)
@@ -535,7 +518,7 @@ __global__ void __launch_bounds__(TINY_NT, 1) tree_tiny_kernel(
   b.pre = b.size + cap;
   b.counter = b.pre + cap;
   b.levels = b.counter + 8;
-  b.parent = b.arrive = b.dep = b.rturn = b.leafpre = nullptr;
+  b.prefix = b.dep = b.rturn = b.leafpre = nullptr;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int64_t i = tid; i < ns; i += blockDim.x) s_sorted[i] = sorted_g[i];
   __syncthreads();
@@ -565,7 +548,7 @@ __global__ void __launch_bounds__(TINY_NT, 1) tree_tiny_kernel(
     const int begin = b.levels[2 * L], end = b.levels[2 * L + 1];
     if (warp < TINY_TILES)
       for (int i = begin + warp; i < end; i += TINY_TILES)
-        if (b.lc[i] >= 0) m2m_node(b, i, lane, fw, fw.w, k, !in_smem, tiles[warp]);
+        if (b.lc[i] >= 0) m2m_node(b, i, lane, fw, fw.w, k, tiles[warp]);
     __syncthreads();
   }
   if (in_smem) {
@@ -972,7 +955,6 @@ __global__ void tree_init_kernel(BuildArrays b, int64_t ns) {
   b.blo[0] = 0;
   b.bhi[0] = ns;
   b.pre[0] = 0;
-  b.parent[0] = -1;
   b.dep[0] = 0;
   b.rturn[0] = 0;
   b.counter[1] = 0;
@@ -1075,7 +1057,7 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
   void* p32 = nullptr;
   SHRK_TRY(scratch_get(25, sizeof(int64_t) * 2 * (size_t)cap, &p64));
   constexpr int NLEV = MAX_TREE_DEPTH + 2;  // levels 0..48 split, level 49 is empty
-  SHRK_TRY(scratch_get(26, sizeof(int32_t) * (8 * (size_t)cap + (size_t)ns + 2 + 8 + 2 * NLEV),
+  SHRK_TRY(scratch_get(26, sizeof(int32_t) * (7 * (size_t)cap + (size_t)ns + 2 + 8 + 2 * NLEV),
                        &p32));
   BuildArrays b;
   b.blo = (int64_t*)p64;
@@ -1086,9 +1068,8 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
   b.pre = b.size + cap;
   b.counter = (int*)(b.pre + cap);
   b.levels = b.counter + 8;
-  b.parent = b.levels + 2 * NLEV;
-  b.arrive = b.parent + cap;
-  b.dep = b.arrive + cap;
+  b.prefix = b.levels + 2 * NLEV;
+  b.dep = b.prefix + cap;
   b.rturn = b.dep + cap;
   b.leafpre = b.rturn + cap;
   constexpr int BS = 256;
@@ -1139,13 +1120,13 @@ shrk_status build_tree_gpu(const double* d_sorted, int64_t ns, const ChebParams&
     tree_leaf_flags_kernel<<<blocks_for(nn, BS), BS, 0, s>>>(b, nn);
     SHRK_CUDA(cudaGetLastError());
     size_t temp_bytes = 0;
-    SHRK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, b.leafpre, b.arrive,
+    SHRK_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp_bytes, b.leafpre, b.prefix,
                                             (int)(ns + 1), s));
     void* temp = nullptr;
     SHRK_TRY(scratch_get(28, std::max<size_t>(temp_bytes, 256), &temp));
-    SHRK_CUDA(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, b.leafpre, b.arrive,
+    SHRK_CUDA(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, b.leafpre, b.prefix,
                                             (int)(ns + 1), s));
-    tree_order_kernel<<<blocks_for(nn, BS), BS, 0, s>>>(b, nn, b.arrive);
+    tree_order_kernel<<<blocks_for(nn, BS), BS, 0, s>>>(b, nn, b.prefix);
     SHRK_CUDA(cudaGetLastError());
     add_launches(3);  // flags, the scan's two kernels, order
   }
@@ -1227,6 +1208,8 @@ shrk_status build_tree_sub(const double* d_sorted, int64_t ns, const ChebParams&
     SHRK_CUDA(cudaGetLastError());
     add_launches(1);
   }
+  // The tree's size sizes its arrays and the next grid, so the call waits for it
+  // here (a device-pointer call has waited before, for the sortedness check).
   int h[3];
   SHRK_CUDA(cudaMemcpyAsync(h, a.count, sizeof(h), cudaMemcpyDeviceToHost, s));
   SHRK_CUDA(cudaStreamSynchronize(s));
