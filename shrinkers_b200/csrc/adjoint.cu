@@ -574,7 +574,8 @@ shrk_status adjoint_f64(const double* d_ev, int64_t p, double eta, const double*
   const int tt = NT * R;
   const int n_tiles = (int)((p + tt - 1) / tt);
   const int ctas = sm_count() * 2;
-  // tiles of a phase: as many column slabs as 256 MB hold
+  // Tiles of a phase: as many column slabs as 256 MB hold (64 MB: 414 ms for 411
+  // at p = 1e6).
   const int64_t per = std::max<int64_t>(1, ((int64_t)256 << 20) / ((int64_t)sizeof(double) * p));
   const int phase = (int)std::min<int64_t>(n_tiles, per);
   const size_t row_n = (size_t)(ctas + phase) * tt, acc_n = phase < n_tiles ? (size_t)p : 0;

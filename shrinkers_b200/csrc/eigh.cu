@@ -1090,8 +1090,7 @@ struct EigSlot {
 // power of two to norm in (1/2, 1], so a minor grows at most threefold a row
 // and, with e^2 above eps^2, two rows lose at most 2^-104: rescaling the pair
 // by its exponent every eight rows keeps it in range.  Three FP64 operations,
-// two integer ones and a load a row (with a range test, a clamp and a select
-// on every row it was 43 instructions).
+// two integer ones and a load a row.
 __device__ __forceinline__ int sturm(const double2* __restrict__ te, int b0, int b1, double x) {
   double num = te[b0].x - x, den = 1.0;
   unsigned cnt = (unsigned)__double2hiint(num) >> 31;
@@ -1701,8 +1700,8 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
     mirror_lower_kernel<<<dim3(cdiv(p, 256), (unsigned)p), 256, 0, s>>>(A, p);
     SHRK_CUDA(cudaGetLastError());
   }
-  // 1. tridiagonalisation (cooperative: all CTAs resident): the last ~2 070
-  // columns by the resident kernel, those before them by tridiag1_kernel, which
+  // 1. tridiagonalisation (cooperative: all CTAs resident): the last 2 048
+  // rows and columns by the resident kernel, those before them by tridiag1_kernel, which
   // passes the trailing matrix through L2 once a column and leaves reflectors in
   // the upper triangle's rows.  SHRK_EIGH_TRIDIAG=2 runs the two-barrier form on
   // every column (reflectors in the lower triangle), SHRK_EIGH_TRI1_GLOBAL=1
@@ -1793,7 +1792,9 @@ shrk_status eigh_device(double* A, int64_t p, std::vector<double>& w_host, cudaS
   if (p > 1)
     SHRK_CUDA(cudaMemcpyAsync(he.data(), e, sizeof(double) * (p - 1), cudaMemcpyDeviceToHost, s));
   SHRK_CUDA(cudaStreamSynchronize(s));
-  SHRK_TRY(poll_device_error(s));  // a wait of the reduction gave up
+  // a wait of the reduction gave up (every matrix call, device-pointer ones too,
+  // runs in its thread's host context)
+  SHRK_TRY(poll_device_error(s));
   const double eps = 2.220446049250313e-16;
   double tnorm = 0.0;
   for (int64_t i = 0; i < p; ++i) {

@@ -1107,7 +1107,7 @@ shrk_status eval_grid(double2* A, double2* B, double2* Wa, double2* Wt, const Ta
 shrk_status run_grid_order(const double* d_q, int64_t nq, const double* d_src, int64_t ns,
                            double eta, const GridPlan& g, const Epilogue& epi, cudaStream_t s,
                            const double* dens_in = nullptr, double* dens_out = nullptr) {
-  // the first-source table and the run lists index sources with 32-bit ints
+  // the runs hold 32-bit source indices
   if (ns > (int64_t)INT32_MAX) {
     set_error("fft grid methods: at most 2^31 - 1 sources per call");
     return SHRK_EINVAL;

@@ -15,7 +15,7 @@
 // reduction across lanes adds one per four pairs).
 //
 // Measured (B200, eta = 1/sqrt(p)): p = 50 000 0.77 ms (sums of all ordered
-// pairs: 1.19), 1e6 304 ms (448), 0.82 of the FP64 pipe's operations; the
+// pairs: 1.19), 1e6 298 ms (448), 0.81 and 0.83 of the FP64 pipe; the
 // other issue slots go to the reciprocal seeds, the shuffles and the loads.
 #include "common.cuh"
 #include "epilogue.cuh"
@@ -288,7 +288,9 @@ shrk_status sym_sums(const double* d_ev, int64_t p, double eta, const Epilogue& 
   const int ctas = sm_count() * (R == 1 ? 3 : 2);
   const int tt = NT * R;
   const int n_tiles = (int)((p + tt - 1) / tt);
-  // tiles of a phase: as many column slabs as 256 MB hold
+  // Tiles of a phase: as many column slabs as 256 MB hold, scratch that the
+  // context keeps (64 MB, with a reduction more often: 3.01 ms for 2.98 at p =
+  // 100 003, 48.1 for 47.4 at 400 000, 306 for 298 at 1e6).
   const int64_t per = std::max<int64_t>(1, ((int64_t)256 << 20) / ((int64_t)sizeof(double2) * p));
   const int phase = (int)std::min<int64_t>(n_tiles, per);
   const size_t row_bytes = sizeof(double2) * (size_t)(ctas + phase) * tt;
