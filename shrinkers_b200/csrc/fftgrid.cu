@@ -451,7 +451,7 @@ __global__ void pack_density_kernel(const GridArgs a, const double* __restrict__
 // the stores and every twiddle staged in shared memory a pass over 2^20 points
 // took 36 (columns) and 21 us (rows), now 20 and 13 (16 + 16 MB each way
 // through L2); bound by the latency of a CTA's chain of load, four butterflies
-// with three exchanges, and store, 4 CTAs an SM overlapping.
+// with three exchanges, and store, 3 or 4 CTAs an SM overlapping.
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
@@ -613,8 +613,10 @@ __device__ __forceinline__ double2 spectral(double2 ck, double2 cn, double ke) {
 // G columns n2 per CTA (G*m1/8 threads), lanes side by side in the columns.
 // With ke the input is the spectral product of x, formed on the way in (a
 // kernel of its own took 8 us at 2^20).
+// Three CTAs an SM: in the 64 registers of four the table entries spill (both
+// transforms of 2^19 points 49.8 us, here 48.3; 2^22 336, here 316).
 template <int LOG>
-__global__ void __launch_bounds__(256, 4) fft_pass1(const double2* __restrict__ x,
+__global__ void __launch_bounds__(256, 3) fft_pass1(const double2* __restrict__ x,
                                                     double2* __restrict__ y, int m2, int64_t m,
                                                     const double2* __restrict__ tw,
                                                     const double2* __restrict__ st, double sign,
