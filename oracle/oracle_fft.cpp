@@ -34,6 +34,13 @@ static size_t next_pow2(size_t n) {  // mod.rs:529-535
   return p;
 }
 
+// Rust's saturating float -> usize cast (NaN -> 0, negative -> 0).
+static size_t sat_usize(double v) {
+  if (!(v > 0.0)) return 0;
+  if (v >= 18446744073709551616.0) return SIZE_MAX;
+  return (size_t)v;
+}
+
 // nufft.rs:106-126 grid_size_for_range.
 size_t nufft_grid_size(double raw_range, double eta) {
   double pad = std::max(PAD_ETA_MULT * eta, PAD_RANGE_FRAC * raw_range);
@@ -41,7 +48,7 @@ size_t nufft_grid_size(double raw_range, double eta) {
   size_t max_grid = std::max(std::max(MAX_GRID, MIN_GRID), (size_t)2);
   double target = RESOLUTION * range / eta;
   target = std::isfinite(target) ? std::min(target, (double)max_grid) : (double)max_grid;
-  return std::min(next_pow2(std::max((size_t)std::ceil(target), MIN_GRID)), max_grid);
+  return std::min(next_pow2(std::max(sat_usize(std::ceil(target)), MIN_GRID)), max_grid);
 }
 
 // fft5.rs:136-164 lagrange_weights<N>.
@@ -158,13 +165,6 @@ struct Opts {
   size_t m_override;  // 0 = the adaptive rule
   double pad_eta_mult, pad_range_frac;
 };
-
-// Rust's saturating float -> usize cast (NaN -> 0, negative -> 0).
-static size_t sat_usize(double v) {
-  if (!(v > 0.0)) return 0;
-  if (v >= 18446744073709551616.0) return SIZE_MAX;
-  return (size_t)v;
-}
 
 // fft5.rs:339-361: the fft5 grid rule dx <= eta/8 and m >= 8p, capped at 2^20.
 size_t fft5_grid_size(double lo_raw, double hi_raw, size_t p, double eta, double pad_eta_mult,

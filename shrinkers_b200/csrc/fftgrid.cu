@@ -1127,14 +1127,15 @@ shrk_status run_grid_order(const double* d_q, int64_t nq, const double* d_src, i
 
 }  // namespace
 
-// nufft.rs:106-126 grid_size_for_range.
+// nufft.rs:106-126 grid_size_for_range (a descending spectrum's range, and so the
+// target, may be negative: the smallest grid).
 size_t nufft_grid_size(double raw_range, double eta) {
   double pad = std::max(NUFFT_PAD_ETA_MULT * eta, NUFFT_PAD_RANGE_FRAC * raw_range);
   double range = raw_range + 2.0 * pad;
   size_t max_grid = std::max(std::max(NUFFT_MAX_GRID, NUFFT_MIN_GRID), (size_t)2);
   double target = NUFFT_RESOLUTION * range / eta;
   target = std::isfinite(target) ? std::min(target, (double)max_grid) : (double)max_grid;
-  return std::min(next_pow2(std::max((size_t)std::ceil(target), NUFFT_MIN_GRID)), max_grid);
+  return std::min(next_pow2(std::max(sat_usize(std::ceil(target)), NUFFT_MIN_GRID)), max_grid);
 }
 
 // fft5.rs:339-361: pad = max(pad_eta_mult eta, pad_range_frac raw_range),
