@@ -184,6 +184,10 @@ struct Runs {
 constexpr int SPLAT_CHUNK = 512;
 constexpr int SPLAT_NT = 256;
 constexpr int SPLAT_LONG = 32;  // longer pieces of a run are summed by a warp
+// Runs of more sources have their heads added by a warp in the pack (by a lane,
+// one after the other: 10^6 sources, half of them zeros as in a spectrum with a
+// null space, nufft 218 us, so 107; 4 10^6: 745 and 181).
+constexpr int HEADS_LONG = 8 * SPLAT_CHUNK;
 
 // One chunk of sources: each source's cell and weights once, by a thread each
 // (coalesced), into shared memory; the places where the cell changes cut the
@@ -310,6 +314,39 @@ __device__ __forceinline__ double odd_kernel(const GridArgs& a, int64_t c) {
   return x / (x * x + a.eta * a.eta);
 }
 
+// The long runs of a warp's window: for each, the warp adds its heads but the
+// first, a chunk a lane, all N sums together, and leaves the run as its tail and
+// one head to the lanes' own sums; the result is what those miss in the lane's
+// cell.  (Out of line: its registers are the pack's only where it runs.)
+template <int N>
+__device__ __noinline__ double add_heads(const double* __restrict__ head, int2* run, int lane,
+                                         double* tot) {
+  double extra = 0.0;
+  for (int e = 0; e < 32 + N; ++e) {
+    const int2 q = run[e];
+    if (q.y - q.x <= HEADS_LONG) continue;
+    double t[N] = {};
+    const int c0 = q.x / SPLAT_CHUNK, c1 = (q.y - 1) / SPLAT_CHUNK;
+#pragma unroll 2
+    for (int h = c0 + 2 + lane; h <= c1; h += 32) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) t[k] += __ldg(head + (int64_t)h * N + k);
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+      if (lane == 0) tot[k] = t[k];
+    }
+    if (lane == 0) run[e].y = (c0 + 1) * SPLAT_CHUNK + 1;
+    __syncwarp();
+    const int i = e - lane;
+    if (i >= 0 && i < N) extra += tot[N - 1 - i];
+    __syncwarp();
+  }
+  return extra;
+}
+
 // A cell's sources are one stretch [A, B) of the sorted sources.  The sparse
 // cells of a warp share theirs 32 sources at a time: a lane per source finds
 // its cell and weights into shared memory, then every lane adds its own cell's
@@ -323,7 +360,7 @@ __global__ void __launch_bounds__(256, 6) pack_kernel(const GridArgs a, const Ru
   constexpr int H = N / 2;
   constexpr int NP = N == 6 ? 8 : N;
   __shared__ double wsm[8][32 * NP];
-  __shared__ int off_sh[8][32];
+  __shared__ __align__(16) int off_sh[8][32];
   __shared__ int2 run_sh[8][32 + N];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, cw = c - lane;
@@ -337,6 +374,7 @@ __global__ void __launch_bounds__(256, 6) pack_kernel(const GridArgs a, const Ru
   double dens = 0.0;
   const bool edge = cw == 0 || cw + 32 >= m;
   if (edge || __any_sync(0xffffffffu, w0.y > w0.x || w1.y > w1.x)) {
+    const bool longs = __any_sync(0xffffffffu, max(w0.y - w0.x, w1.y - w1.x) > HEADS_LONG);
     run_sh[wib][lane] = w0;
     if (lane < N) run_sh[wib][32 + lane] = w1;
     __syncwarp();
@@ -380,6 +418,9 @@ __global__ void __launch_bounds__(256, 6) pack_kernel(const GridArgs a, const Ru
       }
       __syncwarp();
     }
+    double extra = 0.0;
+    if (longs)
+      extra = add_heads<N>(R.head, run_sh[wib], lane, reinterpret_cast<double*>(off_sh[wib]));
     if (c > 0 && c < m - 1) {
       if (any && !sparse) {
         double s[N];  // the run's sum, or its tail: N loads in flight (9 000 clk one by one)
@@ -398,6 +439,7 @@ __global__ void __launch_bounds__(256, 6) pack_kernel(const GridArgs a, const Ru
               s[i] += R.head[(int64_t)h * N + N - 1 - i];
           dens += s[i];
         }
+        dens += extra;
       }
     } else if (c < m) {
       // edge cell: every slot whose clamped index lands here, sources then slots
