@@ -1175,7 +1175,8 @@ __device__ __forceinline__ double start_entry(int slot, int i) {
   return (double)(h >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
-// One thread per cluster, a warp per CTA.  Workspace: the factorisation of
+// One thread per cluster, a warp per CTA (the warp together where a cluster's
+// vectors are orthogonalised).  Workspace: the factorisation of
 // T - lambda I (U's off-diagonals, reciprocal pivots, multipliers, row
 // swaps) and the right-hand side / solution x, rows relative to the block
 // start, stored per warp as [row][array][lane].  Each eigenvalue is factored
@@ -1235,14 +1236,56 @@ __device__ __forceinline__ void forward_row(double* r, double rn, double m, doub
   rhs = fma(-m, keep, other);
 }
 
+// Modified Gram-Schmidt of x (n rows II_RS apart) against q unit vectors (vector r
+// at z[r], its rows p apart), then to unit length; by the warp, a row a lane.  (The
+// vectors are not rescaled in between: x - (z . x) z does not depend on it.)  Two
+// L2 latencies a vector bound it.  A lane of its own waited out a load for every
+// row: rank 800 at p = 1 600 took 131 ms in this kernel, now 10.8; four clusters of
+// 250 at p = 1 000 24 s, now 2.8.
+__device__ void orthogonalise(double* x, int n, const double* z, int64_t p, int q, int lane) {
+  constexpr int U = 8;  // rows in flight a lane
+  __syncwarp();         // x and z as their lanes left them
+  double nrm2 = 0.0;
+  for (int r = 0; r < q; ++r) {
+    double xv[U], zv[U], dt = 0.0;
+    const auto load = [&](int i0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + 32 * u + lane;
+        xv[u] = i < n ? x[(int64_t)i * II_RS] : 0.0;
+        zv[u] = i < n ? z[r + i * p] : 0.0;
+      }
+    };
+    for (int i0 = 0; i0 < n; i0 += 32 * U) {
+      load(i0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) dt = fma(zv[u], xv[u], dt);
+    }
+    dt = warp_sum(dt);
+    nrm2 = 0.0;
+    for (int i0 = 0; i0 < n; i0 += 32 * U) {
+      if (n > 32 * U) load(i0);  // (else they are still there)
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + 32 * u + lane;
+        const double xi = fma(-dt, zv[u], xv[u]);
+        if (i < n) x[(int64_t)i * II_RS] = xi;
+        nrm2 = fma(xi, xi, nrm2);
+      }
+    }
+  }
+  const double inv = 1.0 / sqrt(warp_sum(nrm2));
+  for (int i = lane; i < n; i += 32) x[(int64_t)i * II_RS] *= inv;
+  __syncwarp();
+}
+
 __global__ void __launch_bounds__(32) inverse_iteration_kernel(
     const double* __restrict__ d, const double* __restrict__ e, const double* __restrict__ lam,
     const Cluster* __restrict__ cl, int ncl, int64_t p, double tnorm, double* __restrict__ ws,
     double* __restrict__ Zt) {
   const int lane = threadIdx.x;
   const int t = blockIdx.x * 32 + lane;
-  if (t >= ncl) return;
-  const Cluster c = cl[t];
+  const Cluster c = t < ncl ? cl[t] : Cluster{0, 0, 0, 0};
   double* const wl = ws + (int64_t)blockIdx.x * p * II_RS + lane;  // row 0 of this lane
 #define W(a, i) wl[(int64_t)(i) * II_RS + (a) * 32]
   extern __shared__ double ring[];  // [II_D][II_CH][4][32]
@@ -1255,151 +1298,149 @@ __global__ void __launch_bounds__(32) inverse_iteration_kernel(
   const double* db = d + c.b0;
   const double* eb = e + c.b0;
   constexpr int CH = II_CH;
-  for (int q = 0; q < c.ns; ++q) {
+  const int members = __reduce_max_sync(0xffffffffu, c.ns);  // of the warp's largest cluster
+  for (int q = 0; q < members; ++q) {
+    const bool on = q < c.ns;
     const int slot = c.s0 + q;
-    const double l = lam[slot];
-    // factor T - l I once with partial pivoting (and write the start
-    // vector); the three solves replay the elimination on their right-hand
-    // sides
-    {
-      double diag = db[0] - l;
-      double sup = n > 1 ? eb[0] : 0.0;
-      int i0 = 0;
-      for (; i0 + CH + 1 < n; i0 += CH) {  // full chunks: rows i0 + u + 2 < n
-        double subv[CH], ndv[CH], nsv[CH];
+    if (on) {
+      const double l = lam[slot];
+      // factor T - l I once with partial pivoting (and write the start
+      // vector); the three solves replay the elimination on their right-hand
+      // sides
+      {
+        double diag = db[0] - l;
+        double sup = n > 1 ? eb[0] : 0.0;
+        int i0 = 0;
+        for (; i0 + CH + 1 < n; i0 += CH) {  // full chunks: rows i0 + u + 2 < n
+          double subv[CH], ndv[CH], nsv[CH];
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-          subv[u] = eb[i0 + u];
-          ndv[u] = db[i0 + u + 1] - l;
-          nsv[u] = eb[i0 + u + 1];
-        }
-        double* r = &W(0, i0);
+          for (int u = 0; u < CH; ++u) {
+            subv[u] = eb[i0 + u];
+            ndv[u] = db[i0 + u + 1] - l;
+            nsv[u] = eb[i0 + u + 1];
+          }
+          double* r = &W(0, i0);
 #pragma unroll
-        for (int u = 0; u < CH; ++u) {
-          factor_row(r + u * II_RS, subv[u], ndv[u], nsv[u], small, rsmall, diag, sup);
-          r[u * II_RS + II_X * 32] = start_entry(slot, i0 + u);
+          for (int u = 0; u < CH; ++u) {
+            factor_row(r + u * II_RS, subv[u], ndv[u], nsv[u], small, rsmall, diag, sup);
+            r[u * II_RS + II_X * 32] = start_entry(slot, i0 + u);
+          }
         }
+        for (int i = i0; i + 1 < n; ++i) {
+          factor_row(&W(0, i), eb[i], db[i + 1] - l, i + 2 < n ? eb[i + 1] : 0.0, small, rsmall,
+                     diag, sup);
+          W(II_X, i) = start_entry(slot, i);
+        }
+        const double piv = diag;
+        W(II_RP, n - 1) = fabs(piv) < small ? (piv < 0.0 ? -rsmall : rsmall) : 1.0 / piv;
+        W(II_U1, n - 1) = 0.0;
+        W(II_U2, n - 1) = 0.0;
+        W(II_X, n - 1) = start_entry(slot, n - 1);
       }
-      for (int i = i0; i + 1 < n; ++i) {
-        factor_row(&W(0, i), eb[i], db[i + 1] - l, i + 2 < n ? eb[i + 1] : 0.0, small, rsmall,
-                   diag, sup);
-        W(II_X, i) = start_entry(slot, i);
-      }
-      const double piv = diag;
-      W(II_RP, n - 1) = fabs(piv) < small ? (piv < 0.0 ? -rsmall : rsmall) : 1.0 / piv;
-      W(II_U1, n - 1) = 0.0;
-      W(II_U2, n - 1) = 0.0;
-      W(II_X, n - 1) = start_entry(slot, n - 1);
     }
     double scale = 1.0;  // x in memory times scale is the current vector
     for (int iter = 0; iter < 3; ++iter) {
-      // the factorisation's row operations on the right-hand side
-      __threadfence();  // the workspace before the copies of it
-      double rhs = W(II_X, 0) * scale;
-      {
-        const int nch = (n - 1) / CH;  // full chunks: rows i0 + u + 1 < n
-        const auto fetch = [&](int k) {
-          if (k < nch) {
-            const double* r = &W(0, k * CH);
+      if (on) {
+        // the factorisation's row operations on the right-hand side
+        __threadfence();  // the workspace before the copies of it
+        double rhs = W(II_X, 0) * scale;
+        {
+          const int nch = (n - 1) / CH;  // full chunks: rows i0 + u + 1 < n
+          const auto fetch = [&](int k) {
+            if (k < nch) {
+              const double* r = &W(0, k * CH);
+#pragma unroll
+              for (int u = 0; u < CH; ++u) {
+                copy8(at(k, u, 0), r + (u + 1) * II_RS + II_X * 32);
+                copy8(at(k, u, 1), r + u * II_RS + II_MU * 32);
+                copy8(at(k, u, 2), r + u * II_RS + II_SW * 32);
+              }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+          };
+          for (int k = 0; k < II_D - 1; ++k) fetch(k);
+          for (int k = 0; k < nch; ++k) {
+            fetch(k + II_D - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(II_D - 1) : "memory");
+            double* r = &W(0, k * CH);
+            double rnv[CH], mv[CH], sv[CH];
 #pragma unroll
             for (int u = 0; u < CH; ++u) {
-              copy8(at(k, u, 0), r + (u + 1) * II_RS + II_X * 32);
-              copy8(at(k, u, 1), r + u * II_RS + II_MU * 32);
-              copy8(at(k, u, 2), r + u * II_RS + II_SW * 32);
+              rnv[u] = *at(k, u, 0) * scale;
+              mv[u] = *at(k, u, 1);
+              sv[u] = *at(k, u, 2);
             }
-          }
-          asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        for (int k = 0; k < II_D - 1; ++k) fetch(k);
-        for (int k = 0; k < nch; ++k) {
-          fetch(k + II_D - 1);
-          asm volatile("cp.async.wait_group %0;" ::"n"(II_D - 1) : "memory");
-          double* r = &W(0, k * CH);
-          double rnv[CH], mv[CH], sv[CH];
 #pragma unroll
-          for (int u = 0; u < CH; ++u) {
-            rnv[u] = *at(k, u, 0) * scale;
-            mv[u] = *at(k, u, 1);
-            sv[u] = *at(k, u, 2);
+            for (int u = 0; u < CH; ++u) forward_row(r + u * II_RS, rnv[u], mv[u], sv[u], rhs);
           }
+          for (int i = nch * CH; i + 1 < n; ++i) {
+            const double rn = W(II_X, i + 1) * scale;
+            forward_row(&W(0, i), rn, W(II_MU, i), W(II_SW, i), rhs);
+          }
+        }
+        W(II_X, n - 1) = rhs;
+        __threadfence();
+        // back substitution (the last row's U entries are zero), chunks of
+        // rows from the last
+        double nrm2 = 0.0, x1 = 0.0, x2 = 0.0;
+        {
+          const int nch = n / CH;
+          const auto fetch = [&](int k) {
+            if (k < nch) {
+              const double* r = &W(0, n - 1 - k * CH);
 #pragma unroll
-          for (int u = 0; u < CH; ++u) forward_row(r + u * II_RS, rnv[u], mv[u], sv[u], rhs);
-        }
-        for (int i = nch * CH; i + 1 < n; ++i) {
-          const double rn = W(II_X, i + 1) * scale;
-          forward_row(&W(0, i), rn, W(II_MU, i), W(II_SW, i), rhs);
-        }
-      }
-      W(II_X, n - 1) = rhs;
-      __threadfence();
-      // back substitution (the last row's U entries are zero), chunks of
-      // rows from the last
-      double nrm2 = 0.0, x1 = 0.0, x2 = 0.0;
-      {
-        const int nch = n / CH;
-        const auto fetch = [&](int k) {
-          if (k < nch) {
-            const double* r = &W(0, n - 1 - k * CH);
+              for (int u = 0; u < CH; ++u) {
+                copy8(at(k, u, 0), r - u * II_RS + II_RP * 32);
+                copy8(at(k, u, 1), r - u * II_RS + II_U1 * 32);
+                copy8(at(k, u, 2), r - u * II_RS + II_U2 * 32);
+                copy8(at(k, u, 3), r - u * II_RS + II_X * 32);
+              }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+          };
+          for (int k = 0; k < II_D - 1; ++k) fetch(k);
+          for (int k = 0; k < nch; ++k) {
+            fetch(k + II_D - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(II_D - 1) : "memory");
+            double* r = &W(0, n - 1 - k * CH);
 #pragma unroll
             for (int u = 0; u < CH; ++u) {
-              copy8(at(k, u, 0), r - u * II_RS + II_RP * 32);
-              copy8(at(k, u, 1), r - u * II_RS + II_U1 * 32);
-              copy8(at(k, u, 2), r - u * II_RS + II_U2 * 32);
-              copy8(at(k, u, 3), r - u * II_RS + II_X * 32);
+              // the pivot multiplied in first: one FMA from x1 to xi
+              const double r0 = *at(k, u, 0);
+              const double xi = fma(-(*at(k, u, 1) * r0), x1,
+                                    fma(-(*at(k, u, 2) * r0), x2, *at(k, u, 3) * r0));
+              r[-u * II_RS + II_X * 32] = xi;
+              nrm2 = fma(xi, xi, nrm2);
+              x2 = x1;
+              x1 = xi;
             }
           }
-          asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        for (int k = 0; k < II_D - 1; ++k) fetch(k);
-        for (int k = 0; k < nch; ++k) {
-          fetch(k + II_D - 1);
-          asm volatile("cp.async.wait_group %0;" ::"n"(II_D - 1) : "memory");
-          double* r = &W(0, n - 1 - k * CH);
-#pragma unroll
-          for (int u = 0; u < CH; ++u) {
-            // the pivot multiplied in first: one FMA from x1 to xi
-            const double r0 = *at(k, u, 0);
-            const double xi = fma(-(*at(k, u, 1) * r0), x1,
-                                  fma(-(*at(k, u, 2) * r0), x2, *at(k, u, 3) * r0));
-            r[-u * II_RS + II_X * 32] = xi;
+          const int i0 = n - 1 - nch * CH;
+          for (int i = i0; i >= 0; --i) {
+            const double r0 = W(II_RP, i);
+            const double xi =
+                fma(-(W(II_U1, i) * r0), x1, fma(-(W(II_U2, i) * r0), x2, W(II_X, i) * r0));
+            W(II_X, i) = xi;
             nrm2 = fma(xi, xi, nrm2);
             x2 = x1;
             x1 = xi;
           }
         }
-        const int i0 = n - 1 - nch * CH;
-        for (int i = i0; i >= 0; --i) {
-          const double r0 = W(II_RP, i);
-          const double xi =
-              fma(-(W(II_U1, i) * r0), x1, fma(-(W(II_U2, i) * r0), x2, W(II_X, i) * r0));
-          W(II_X, i) = xi;
-          nrm2 = fma(xi, xi, nrm2);
-          x2 = x1;
-          x1 = xi;
-        }
+        scale = 1.0 / sqrt(nrm2);
       }
-      scale = 1.0 / sqrt(nrm2);
-      if (q > 0) {
-        // modified Gram-Schmidt against the cluster's earlier vectors (on the
-        // normalised vector; rare: numerically equal eigenvalues only)
-        for (int i = 0; i < n; ++i) W(II_X, i) *= scale;
-        scale = 1.0;
-        for (int r = 0; r < q; ++r) {
-          const double* zr = Zt + (c.s0 + r);
-          double dt = 0.0;
-          for (int i = 0; i < n; ++i) dt += zr[(int64_t)(c.b0 + i) * p] * W(II_X, i);
-          nrm2 = 0.0;
-          for (int i = 0; i < n; ++i) {
-            const double xi = W(II_X, i) - dt * zr[(int64_t)(c.b0 + i) * p];
-            W(II_X, i) = xi;
-            nrm2 += xi * xi;
-          }
-          const double inv = 1.0 / sqrt(nrm2);
-          for (int i = 0; i < n; ++i) W(II_X, i) *= inv;
-        }
+      // The cluster's earlier vectors (numerically equal eigenvalues only).
+      unsigned todo = __ballot_sync(0xffffffffu, on && q > 0);
+      for (; todo; todo &= todo - 1) {
+        const int k = __ffs(todo) - 1;
+        const int s0 = __shfl_sync(0xffffffffu, c.s0, k), b0 = __shfl_sync(0xffffffffu, c.b0, k);
+        orthogonalise(&W(II_X, 0) - lane + k, __shfl_sync(0xffffffffu, n, k),
+                      Zt + s0 + (int64_t)b0 * p, p, q, lane);
+        if (lane == k) scale = 1.0;
       }
     }
-    for (int i = 0; i < n; ++i) Zt[slot + (int64_t)(c.b0 + i) * p] = W(II_X, i) * scale;
+    if (on)
+      for (int i = 0; i < n; ++i) Zt[slot + (int64_t)(c.b0 + i) * p] = W(II_X, i) * scale;
+    __syncwarp();  // the vector before the warp reads it
   }
 #undef W
 }
