@@ -45,7 +45,7 @@ struct __align__(16) PairStage {
 // and no source further than PAIR_SPREAD eta from the middle one.
 struct __align__(16) PairStageNear : PairStage {
   double2 sc[PAIR_CH / 2], hw[PAIR_CH / 2];
-  unsigned char tight[PAIR_CH / 64];
+  alignas(4) unsigned char tight[PAIR_CH / 64];
   double2 range[PAIR_NT / 32];  // (min, max) of each warp's targets
 };
 template <bool PAIRED>
@@ -289,13 +289,18 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
           }
         };
         if constexpr (PAIRED) {
-          if (!MIXED) {  // no bounds: the targets themselves
+          // The flags of the block's whole groups; with none set it is summed as one
+          // (in pieces of 64 values out of order took 21.2 ms at 200 000 FP64 queries
+          // and as many sources, so 18.9; mixed 21.2 and 19.9).
+          uint32_t flags = *reinterpret_cast<const uint32_t*>(&st.tight[sub >> 6]);
+          if (!MIXED && slen < SUB) flags &= (1u << (8 * (slen >> 6))) - 1u;
+          if (!MIXED && flags) {  // no bounds: the targets themselves
             bool in = eta >= 1e-60 && eta <= 1e60;
 #pragma unroll
             for (int r = 0; r < R; ++r) in = in && fabs(x[r] - st.sbuf[b][sub]) <= 1e60;
             pairs = __all_sync(0xffffffffu, in);
           }
-          if (pairs) {
+          if (pairs && flags) {
             double rn[R], vn[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) rn[r] = vn[r] = 0.0;
