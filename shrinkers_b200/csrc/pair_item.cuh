@@ -312,7 +312,8 @@ __device__ __forceinline__ bool pair_item(const PairItem& a, PairStageOf<PAIRED>
                 double X2[R];
 #pragma unroll
                 for (int r = 0; r < R; ++r) X2[r] = 2.0 * (x[r] - cg);
-#pragma unroll 2
+                // (two a step: mixed sums of 200 000 10.6 ms, four 10.1)
+#pragma unroll 4
                 for (int i = i0; i < i0 + 32; ++i) {
                   const double2 sc = st.sc[i], hw = st.hw[i];
 #pragma unroll
