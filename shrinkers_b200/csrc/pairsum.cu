@@ -56,9 +56,9 @@ constexpr int R_SMALL_MIXED = 2;  // the packed far field takes target pairs
 
 // MIXED sums over more sources take their near field pair by pair: it is then
 // a few per cent of the pairs, and the paired form costs the far field's loop
-// about 1 % in registers.  Full tiles, eta = 1/sqrt(p): 65 536 sources 1.11 ms
-// paired, 1.14 not; 262 144: 16.7 and 17.1; 400 000: 35.6 and 35.8; 10^6:
-// 214.1 and 212.3.
+// about 1 % in registers.  Full tiles, eta = 1/sqrt(p): 65 536 sources 1.10 ms
+// paired, 1.13 not; 262 144: 16.6 and 17.1; 400 000: 35.4 and 35.8; 524 288: 61.9
+// and 61.2; 10^6: 213.6 and 211.9.
 constexpr int64_t PAIRED_MAX = 1 << 19;
 
 double g_near_k = SHRK_NEAR_K;
